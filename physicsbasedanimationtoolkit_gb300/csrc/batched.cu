@@ -74,8 +74,8 @@ __device__ __forceinline__ void sweep_tile(SweepParams const& p, int begin, int 
         int i       = 0;
         float xi[3] = {0.f, 0.f, 0.f};
         int k = 0, k1 = 0, n0 = 0, n1 = 0, base = 0;
-        uint2 q0 = make_uint2(0u, 0u), q1 = q0;
-        float4 st0 = make_float4(0.f, 0.f, 0.f, 0.f), st1 = st0;
+        uint32_t q0 = 0u, q1 = 0u;
+        float2 mt0 = make_float2(0.f, 0.f), mt1 = mt0;
         if (valid)
         {
             i    = __ldg(p.solve + s);
@@ -86,22 +86,22 @@ __device__ __forceinline__ void sweep_tile(SweepParams const& p, int begin, int 
             k    = __ldg(p.incPtr + s) + lane;
             if (k < k1)
             {
-                q0  = __ldg(p.incPack + k);
-                st0 = __ldg(p.stiff + k);
+                q0  = __ldg(p.incSlots + k);
+                mt0 = __ldg(p.incMat + k);
             }
             if (k + L < k1)
             {
-                q1  = __ldg(p.incPack + k + L);
-                st1 = __ldg(p.stiff + k + L);
+                q1  = __ldg(p.incSlots + k + L);
+                mt1 = __ldg(p.incMat + k + L);
             }
             load3(Mem<true>::ld((CHEB ? p.hprev : p.x) + i), xi);
             for (int j = n0 + lane; j < n1; j += L)
             {
-                uint32_t const a  = __ldg(p.nbr + j);
+                uint2 const a     = __ldg(p.nbr + j);
                 float4 const* src = p.x;
-                if (CHEB && !(a >> 31))
+                if (CHEB && !(a.x >> 31))
                     src = p.hprev;
-                slab[base + j - n0] = Mem<true>::ld(src + (a & kIndexMask));
+                stage_neighbour(b, slab + base + j - n0, Mem<true>::ld(src + (a.x & kIndexMask)), xi, __uint_as_float(a.y));
             }
         }
         __syncwarp();
@@ -109,27 +109,18 @@ __device__ __forceinline__ void sweep_tile(SweepParams const& p, int begin, int 
         {
             for (; k < k1; k += L)
             {
-                uint2 q2   = make_uint2(0u, 0u);
-                float4 st2 = make_float4(0.f, 0.f, 0.f, 0.f);
+                uint32_t q2 = 0u;
+                float2 mt2  = make_float2(0.f, 0.f);
                 if (k + 2 * L < k1)
                 {
-                    q2  = __ldg(p.incPack + k + 2 * L);
-                    st2 = __ldg(p.stiff + k + 2 * L);
+                    q2  = __ldg(p.incSlots + k + 2 * L);
+                    mt2 = __ldg(p.incMat + k + 2 * L);
                 }
-                float d[3][3];
-#pragma unroll
-                for (int m = 0; m < 3; ++m)
-                {
-                    float4 const xa = slab[base + int((q0.x >> (8 * m)) & 0xFFu)];
-                    d[m][0] = xa.x - xi[0];
-                    d[m][1] = xa.y - xi[1];
-                    d[m][2] = xa.z - xi[2];
-                }
-                accumulate_incidence(b, d, st0.x, st0.y, st0.z, __uint_as_float(q0.y), st0.w);
+                staged_incidence(b, slab + base, q0, mt0);
                 q0  = q1;
-                st0 = st1;
+                mt0 = mt1;
                 q1  = q2;
-                st1 = st2;
+                mt1 = mt2;
             }
         }
         finish_vertex<L, CHEB, false, false, true>(p, b, valid, lane, i, s, xi);
@@ -248,7 +239,7 @@ cudaError_t launch_batched_step(BatchedStepParams const& p, int lanes, int block
     if (p.nItems <= 0)
         return cudaSuccess;
     if (grid < 1 || block < 32 || block > 256 || block % lanes != 0 || smem > kStagedMaxBytes || !p.items ||
-        !p.control || !p.done || !p.flags || !p.sweep.stiff || !p.sweep.incPack || !p.sweep.nbrPtr || (chebyshev && (!p.H0 || !p.H1 || !p.omega)))
+        !p.control || !p.done || !p.flags || !p.sweep.incMat || !p.sweep.incSlots || !p.sweep.nbrPtr || (chebyshev && (!p.H0 || !p.H1 || !p.omega)))
         return cudaErrorInvalidValue;
     return chebyshev ? launch_c<true>(p, lanes, block, grid, smem, s) : launch_c<false>(p, lanes, block, grid, smem, s);
 }

@@ -256,19 +256,20 @@ class VbdSystem
     DeviceArray<TetRecord> tets;
     DeviceArray<int32_t> solve, incPtr, flags;
     DeviceArray<uint32_t> inc;
-    // Staged sweep: per free vertex its distinct neighbours, per incidence (tet, neighbour slots),
-    // per tet its material words.  stagedOk is false when some vertex has more than 256
+    // Distinct neighbours of every free vertex (solve order), and the rest-state constants of the
+    // solves (SweepParams): incMat and incSlots per incidence, nbr (index, K) per neighbour, diag per
+    // entry; formed on the device from the tets' geometry and Lame coefficients (FP64), at creation and
+    // by pbgb_vbd_set_material.  stagedOk is false when some vertex has more than 256
     // neighbours (slots are bytes); `staged` is the user's choice.
     bool stagedOk = false, staged = true;
     std::vector<int32_t> hostNbrPtr;
+    DeviceArray<TetGeometry> tetGeometry;
+    DeviceArray<double> dMu, dLambda;
     DeviceArray<int32_t> nbrPtr;
-    DeviceArray<uint32_t> nbr;
-    DeviceArray<uint2> incPack;
-    // Per-incidence stiffness of the sweeps (TetStiffness resolved for the incidence's own corner):
-    // incStiff[k] = (b0, b1, b2, kappa_o) and incPack[k].y = sigma.  Host copies of the incidence
-    // words and neighbour slots let pbgb_vbd_set_material rebuild them.
-    DeviceArray<float4> incStiff;
-    std::vector<uint32_t> hostInc, hostSlots;
+    DeviceArray<uint2> nbr;
+    DeviceArray<float2> incMat;
+    DeviceArray<uint32_t> incSlots;
+    DeviceArray<float> diag;
     DeviceArray<double> red, gradBuf, objPartials;
 
     // Sweep timing: with `profiling` on, the captured step records an event pair around the colour
@@ -290,8 +291,8 @@ class VbdSystem
     DeviceArray<float4> cTlo, cThi, cVlo, cVhi, xpred;
     DeviceArray<uint8_t> cActive;
 
-    // Host copies of the tet records and quadrature weights (pbgb_vbd_set_material rewrites the
-    // material words).
+    // Host copies of the tet records' vertices (the material words live on the device only) and
+    // quadrature weights.
     std::vector<TetRecord> hostRecords;
     std::vector<double> hostWg;
     // Host copies for the descent-path traces: lumped masses, Lame coefficients and the
@@ -460,12 +461,18 @@ class VbdSystem
         return total;
     }
 
-    // Staged-sweep fields of a SweepParams, and the shared memory of colour c's launch (0: gather).
-    void stagedFields(SweepParams& w) const
+    // Mesh tables of a SweepParams, and the shared memory of colour c's staged launch (0: gather).
+    void meshTables(SweepParams& w) const
     {
-        w.nbrPtr  = nbrPtr.get();
-        w.nbr     = nbr.get();
-        w.incPack = incPack.get();
+        w.tets     = tets.get();
+        w.solve    = solve.get();
+        w.incPtr   = incPtr.get();
+        w.inc      = inc.get();
+        w.incMat   = incMat.get();
+        w.incSlots = incSlots.get();
+        w.diag     = diag.get();
+        w.nbrPtr   = nbrPtr.get();
+        w.nbr      = nbr.get();
     }
     size_t stagedBytes(int32_t c, int L) const
     {
@@ -655,7 +662,7 @@ class VbdSystem
                 }
                 TetRecord& r   = hrec[t0 + e];
                 r.v            = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                r.mat          = make_float4(float(w * mu), float(w * la), float(1.0 + mu / la), 0.f);
+                r.mat          = make_float4(0.f, 0.f, 0.f, 0.f); // uploadMaterial
             }
             v0 += d.n_vertices;
             t0 += d.n_tets;
@@ -717,10 +724,11 @@ class VbdSystem
         }
         meanDegree = nFree > 0 ? double(degSum) / nFree : 0.0;
 
-        // Neighbour lists of the staged sweep, in first-use order over the vertex's incidences and
+        // Neighbour lists, in first-use order over the vertex's incidences and
         // corners ((local + 1 + m) & 3, the order the sweep visits them).
-        std::vector<uint32_t> hNbr;
-        hostSlots.assign(hInc.size(), 0u);
+        std::vector<uint2> hNbr;
+        hNbr.reserve(hInc.size());
+        std::vector<uint32_t> hSlots(hInc.size(), 0u);
         hostNbrPtr.assign(size_t(nFree) + 1, 0);
         stagedOk = true;
         {
@@ -747,21 +755,16 @@ class VbdSystem
                             list.push_back(a);
                         slots |= uint32_t(idx) << (8 * m);
                     }
-                    hostSlots[k] = slots; // meaningful only while the list has at most 256 entries
+                    hSlots[k] = slots; // meaningful only while the list has at most 256 entries
                 }
                 if (list.size() > 256)
                     stagedOk = false;
-                if (stagedOk)
-                {
-                    hNbr.insert(hNbr.end(), list.begin(), list.end());
-                    hostNbrPtr[s + 1] = int32_t(hNbr.size());
-                }
+                for (uint32_t a : list)
+                    hNbr.push_back(make_uint2(a, 0u));
+                hostNbrPtr[s + 1] = int32_t(hNbr.size());
             }
         }
-        hostInc = hInc;
-        std::vector<float4> hStiff;
-        std::vector<uint2> hPack;
-        incidenceRecords(hStiff, hPack);
+        hostRecords = std::move(hrec);
 
         // Device allocation and upload.
         check(cudaGetDevice(&device), "cudaGetDevice");
@@ -818,7 +821,7 @@ class VbdSystem
         v.upload(hv.data(), nV, stream);
         aext.upload(ha.data(), nV, stream);
         m.upload(hm.data(), nV, stream);
-        tets.upload(hrec.data(), nT, stream);
+        tets.upload(hostRecords.data(), nT, stream);
         X.upload(hX.data(), nV, stream);
         std::vector<float4> hOrigin;
         if (useOrigins)
@@ -830,24 +833,30 @@ class VbdSystem
             origin.upload(hOrigin.data(), size_t(nV), stream);
         }
         solve.upload(hsolve.data(), nFree, stream);
-        incStiff.allocate(hStiff.size());
-        incStiff.upload(hStiff.data(), hStiff.size(), stream);
-        incPack.allocate(hPack.size());
-        incPack.upload(hPack.data(), hPack.size(), stream);
+        nbrPtr.allocate(hostNbrPtr.size());
+        nbrPtr.upload(hostNbrPtr.data(), hostNbrPtr.size(), stream);
+        nbr.allocate(hNbr.size());
+        nbr.upload(hNbr.data(), hNbr.size(), stream);
+        incMat.allocate(hInc.size());
+        incSlots.allocate(hInc.size());
+        incSlots.upload(hSlots.data(), hInc.size(), stream);
+        diag.allocate(size_t(nFree));
+        std::vector<TetGeometry> hGeometry(static_cast<size_t>(nT));
+        for (int32_t e = 0; e < nT; ++e)
+            hGeometry[e] = tet_geometry(hostGP.data() + 12 * size_t(e), hostWg[e]);
+        tetGeometry.allocate(size_t(nT));
+        tetGeometry.upload(hGeometry.data(), size_t(nT), stream);
+        dMu.allocate(size_t(nT));
+        dLambda.allocate(size_t(nT));
         incPtr.upload(hIncPtr.data(), hIncPtr.size(), stream);
         inc.upload(hInc.data(), hInc.size(), stream);
+        uploadMaterial();
         if (stagedOk)
         {
-            nbrPtr.allocate(hostNbrPtr.size());
-            nbr.allocate(hNbr.size());
-            nbrPtr.upload(hostNbrPtr.data(), hostNbrPtr.size(), stream);
-            nbr.upload(hNbr.data(), hNbr.size(), stream);
             check(prepare_staged_sweeps(), "cudaFuncSetAttribute");
             if (nMeshes > 1)
                 check(prepare_batched_step(), "cudaFuncSetAttribute");
         }
-        else
-            hostNbrPtr.clear();
         if (nV > 0)
         {
             check(cudaMemcpyAsync(xt.get(), x.get(), sizeof(float4) * nV, cudaMemcpyDeviceToDevice, stream), "copy");
@@ -964,36 +973,29 @@ class VbdSystem
         }
         // The host staging vectors die at the end of this scope: wait for the uploads.
         check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-        hostRecords = std::move(hrec);
     }
 
-    // Per-incidence stiffness of all solved incidences (solve order) from the host copies of the
-    // shape-function gradients, quadrature weights and Lame coefficients: stiff[k] = (b0, b1, b2,
-    // kappa_o) of incidence k's own corner o, pack[k] = (neighbour slots, sigma as bits).
-    void incidenceRecords(std::vector<float4>& stiffOut, std::vector<uint2>& packOut) const
+    // The tets' material words and the rest-state constants of the solves for the Lame coefficients in
+    // hostMu, hostLambda, formed on the device.
+    void uploadMaterial()
     {
-        std::vector<double> words(8 * size_t(nT));
-        for (int32_t e = 0; e < nT; ++e)
-        {
-            double w[8];
-            tet_stiffness_words(hostGP.data() + 12 * size_t(e), hostWg[e], hostMu[e], hostLambda[e], w);
-            std::copy(w, w + 8, words.begin() + 8 * size_t(e));
-        }
-        stiffOut.resize(hostInc.size());
-        packOut.resize(hostInc.size());
-        for (size_t k = 0; k < hostInc.size(); ++k)
-        {
-            uint32_t const q   = hostInc[k];
-            double const* w    = words.data() + 8 * size_t(q >> 2);
-            double const bw[6] = {w[0], w[1], w[2], w[3], w[4], w[5]};
-            double b0, b1, b2, kappa;
-            corner_stiffness(bw, w[7], int(q & 3u), b0, b1, b2, kappa);
-            stiffOut[k]        = make_float4(float(b0), float(b1), float(b2), float(kappa));
-            float const sigma  = float(w[6]);
-            uint32_t sbits     = 0;
-            std::memcpy(&sbits, &sigma, sizeof(sbits));
-            packOut[k] = make_uint2(hostSlots[k], sbits);
-        }
+        dMu.upload(hostMu.data(), size_t(nT), stream);
+        dLambda.upload(hostLambda.data(), size_t(nT), stream);
+        StiffnessParams p{};
+        p.geometry = tetGeometry.get();
+        p.mu       = dMu.get();
+        p.lambda   = dLambda.get();
+        p.tets     = tets.get();
+        p.solve    = solve.get();
+        p.incPtr   = incPtr.get();
+        p.inc      = inc.get();
+        p.nbrPtr   = nbrPtr.get();
+        p.incMat   = incMat.get();
+        p.nbr      = nbr.get();
+        p.diag     = diag.get();
+        p.nT       = nT;
+        p.nFree    = nFree;
+        check(launch_stiffness(p, stream), "stiffness");
     }
 
     // Per-tet Lame coefficients (system order); the records keep (wg mu, wg lambda, 1 + mu/lambda).
@@ -1003,21 +1005,9 @@ class VbdSystem
         for (int32_t e = 0; e < nT; ++e)
             if (!(mu[e] > 0.0) || !(lambda[e] > 0.0) || !std::isfinite(mu[e]) || !std::isfinite(lambda[e]))
                 throw std::invalid_argument("pbgb_vbd_set_material: expected finite mu > 0 and lambda > 0");
-        for (int32_t e = 0; e < nT; ++e)
-        {
-            double const w     = hostWg[e];
-            hostRecords[e].mat = make_float4(float(w * mu[e]), float(w * lambda[e]), float(1.0 + mu[e] / lambda[e]), 0.f);
-            hostMu[e]          = mu[e];
-            hostLambda[e]      = lambda[e];
-        }
-        tets.upload(hostRecords.data(), size_t(nT), stream);
-        std::vector<float4> hStiff;
-        std::vector<uint2> hPack;
-        incidenceRecords(hStiff, hPack);
-        incStiff.upload(hStiff.data(), hStiff.size(), stream);
-        incPack.upload(hPack.data(), hPack.size(), stream);
-        // The uploads read the host arrays asynchronously.
-        check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+        std::copy(mu, mu + nT, hostMu.begin());
+        std::copy(lambda, lambda + nT, hostLambda.begin());
+        uploadMaterial();
     }
 
     void adjointReserve(int32_t slots, int32_t iterations)
@@ -1132,13 +1122,7 @@ class VbdSystem
         w.x        = x.get();
         w.xt       = xt.get();
         w.xtilde   = xtilde.get();
-        w.tets     = tets.get();
-        w.stiff    = incStiff.get();
-        w.incPack  = incPack.get();
-        w.solve    = solve.get();
-        w.incPtr   = incPtr.get();
-        w.inc      = inc.get();
-        stagedFields(w);
+        meshTables(w);
         w.h        = h;
         w.h2       = h * h;
         w.kD       = kD;
@@ -1438,13 +1422,7 @@ class VbdSystem
         w.x        = x.get();
         w.xt       = xt.get();
         w.xtilde   = xtilde.get();
-        w.stiff    = incStiff.get();
-        w.incPack  = incPack.get();
-        w.tets     = tets.get();
-        w.solve    = solve.get();
-        w.incPtr   = incPtr.get();
-        w.inc      = inc.get();
-        stagedFields(w);
+        meshTables(w);
         w.h        = h;
         w.h2       = h * h;
         w.kD       = kD;
@@ -1505,13 +1483,7 @@ class VbdSystem
         w.x        = x.get();
         w.xt       = xt.get();
         w.xtilde   = xtilde.get();
-        w.tets     = tets.get();
-        w.stiff    = incStiff.get();
-        w.incPack  = incPack.get();
-        w.solve    = solve.get();
-        w.incPtr   = incPtr.get();
-        w.inc      = inc.get();
-        stagedFields(w);
+        meshTables(w);
         w.h        = h;
         w.h2       = h2;
         w.kD       = kD;
@@ -3179,7 +3151,7 @@ PBGB_API int pbgb_debug_vertex_block(
         double const* G4 = GPs + 12 * size_t(q);
         if (il[q] < 0 || il[q] > 3)
             return fail(nullptr, kInvalid, "local index out of range");
-        // Same own-corner-relative form and per-tet record as the device sweep (in FP64).
+        // Same own-corner-relative form and rest-state constants as the device sweep (in FP64).
         double d[3][3];
         for (int m = 0; m < 3; ++m)
         {
@@ -3187,12 +3159,14 @@ PBGB_API int pbgb_debug_vertex_block(
             for (int r = 0; r < 3; ++r)
                 d[m][r] = xq[3 * a + r] - xq[3 * il[q] + r];
         }
-        double w[8];
-        pbgb::tet_stiffness_words(G4, wg[q], mu[q], lambda[q], w);
-        double const bw[6] = {w[0], w[1], w[2], w[3], w[4], w[5]};
-        double b0, b1, b2, kappa;
-        pbgb::corner_stiffness(bw, w[7], il[q], b0, b1, b2, kappa);
-        pbgb::accumulate_incidence(b, d, b0, b1, b2, w[6], kappa);
+        double bm[3], kappa, sigma;
+        pbgb::corner_stiffness(pbgb::tet_geometry(G4, wg[q]), mu[q], lambda[q], il[q], bm, kappa, sigma);
+        for (int m = 0; m < 3; ++m)
+        {
+            pbgb::accumulate_neighbour(b, d[m], bm[m]);
+            b.s -= bm[m];
+        }
+        pbgb::accumulate_incidence(b, d, sigma, kappa);
     }
     pbgb::newton_update(b, xt, xtilde, m, h, h2, kD, detHZero, x, g, H);
     return kOk;

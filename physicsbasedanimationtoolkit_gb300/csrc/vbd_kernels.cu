@@ -14,9 +14,9 @@ namespace {
 // Integrator::SolveVertex, sim/vbd/Integrator.cpp:98-136).  L lanes cooperate on one vertex: lane
 // l takes incidences l, l+L, ...; the 10 accumulated floats are then reduced with xor shuffles
 // and lane 0 applies damping, inertia and the 3x3 Newton step, writing x in place.  Vertices of a
-// colour share no tet, so the in-place write races with no reader of this launch.  Each incidence
-// reads its 20 bytes of rest-state stiffness (b0, b1, b2, kappa, sigma; TetStiffness resolved for
-// the vertex's corner) and the three other corners' current positions: no rest position is read.
+// colour share no tet, so the in-place write races with no reader of this launch.  The vertex's
+// neighbours give its mu term (8 bytes each: index, K), then each incidence its volume term from
+// (kappa, sigma) and the three other corners' current positions: no rest position is read.
 //
 // CHEB: the Chebyshev update of the reference (applied to all vertices after each full sweep,
 // sim/vbd/ChebyshevIntegrator.cpp:15-32) is fused in.  Only vertex i's own values enter its
@@ -39,16 +39,17 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) sweep_kernel(SweepParams
     zero(b);
     int i       = 0;
     float xi[3] = {0.f, 0.f, 0.f};
-    int k = 0, k1 = 0;
+    int k = 0, k1 = 0, n = 0, n1 = 0;
     uint32_t q0 = 0u, q1 = 0u;
     uint4 t     = make_uint4(0u, 0u, 0u, 0u);
-    float4 st   = make_float4(0.f, 0.f, 0.f, 0.f);
-    float sg    = 0.f;
+    float2 mt   = make_float2(0.f, 0.f);
     // Prologue on data no earlier launch writes (mesh tables): with programmatic dependent launch
     // it overlaps the previous colour's tail.
     if (valid)
     {
         i  = __ldg(p.solve + s);
+        n  = __ldg(p.nbrPtr + s) + lane;
+        n1 = __ldg(p.nbrPtr + s + 1);
         k1 = __ldg(p.incPtr + s + 1);
         k  = __ldg(p.incPtr + s) + lane;
         // Software pipeline: the records of incidence k+L and the incidence word of k+2L are in
@@ -58,8 +59,7 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) sweep_kernel(SweepParams
         if (k < k1)
         {
             t  = __ldg(&p.tets[q0 >> 2].v);
-            st = __ldg(p.stiff + k);
-            sg = __uint_as_float(__ldg(&p.incPack[k].y));
+            mt = __ldg(p.incMat + k);
         }
     }
     // Positions are written by the previous launches: wait for them (no-op without PDL), then let
@@ -69,17 +69,22 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) sweep_kernel(SweepParams
     if (valid)
     {
         load3(CHEB ? p.hprev[i] : p.x[i], xi);
+        for (; n < n1; n += L)
+        {
+            uint2 const a     = __ldg(p.nbr + n);
+            float4 const xa   = __ldg((CHEB && !(a.x >> 31) ? p.hprev : p.x) + (a.x & kIndexMask));
+            float const d[3]  = {xa.x - xi[0], xa.y - xi[1], xa.z - xi[2]};
+            accumulate_neighbour(b, d, __uint_as_float(a.y));
+        }
         for (; k < k1; k += L)
         {
             int const il = int(q0 & 3u);
             uint4 tn     = make_uint4(0u, 0u, 0u, 0u);
-            float4 stn   = make_float4(0.f, 0.f, 0.f, 0.f);
-            float sgn    = 0.f;
+            float2 mtn   = make_float2(0.f, 0.f);
             if (k + L < k1)
             {
                 tn  = __ldg(&p.tets[q1 >> 2].v);
-                stn = __ldg(p.stiff + k + L);
-                sgn = __uint_as_float(__ldg(&p.incPack[k + L].y));
+                mtn = __ldg(p.incMat + k + L);
             }
             uint32_t const q2 = k + 2 * L < k1 ? __ldg(p.inc + k + 2 * L) : 0u;
             uint32_t const own = corner(t, il) >> 30;
@@ -97,12 +102,11 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) sweep_kernel(SweepParams
                 d[m][1] = xa.y - xi[1];
                 d[m][2] = xa.z - xi[2];
             }
-            accumulate_incidence(b, d, st.x, st.y, st.z, sg, st.w);
+            accumulate_incidence(b, d, mt.y, mt.x);
             q0 = q1;
             q1 = q2;
             t  = tn;
-            st = stn;
-            sg = sgn;
+            mt = mtn;
         }
     }
     finish_vertex<L, CHEB, REC, CONTACT>(p, b, valid, lane, i, s, xi);
@@ -110,10 +114,14 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) sweep_kernel(SweepParams
 
 // The same sweep with each vertex's neighbours staged in shared memory.  A vertex's ~23 incident
 // tets reference only ~14 distinct neighbours, so instead of gathering three corners' positions
-// per incidence, the vertex's lanes load each neighbour's current position once into its slice of
-// the block's slab (a float4 per neighbour) after griddepcontrol.wait, and the incidence loop reads
-// them back through the three slot bytes of its packed incidence word.  The slab slice of solve entry s starts at nbrPtr[s] - nbrPtr[first entry of the block].
-// The lanes of a vertex share a warp, so __syncwarp orders the staging.
+// per incidence, the vertex's lanes load each neighbour's current position once, add its mu term and
+// put the edge vector to it into the vertex's slice of the block's slab (a float4 per neighbour), and
+// the incidence loop reads the edge vectors back through its three slot bytes.  The slab slice of solve
+// entry s starts at nbrPtr[s] - nbrPtr[first entry of the block].  The lanes of a vertex share a
+// warp, so __syncwarp orders the staging.  What a solve reads of the rest state (8 B per neighbour, 12 B
+// per incidence) streams from L2 for every update and bounds a large mesh: with the mu terms kept per
+// incidence (24 B each, 4 B per neighbour) the 270,641-vertex beam took 2.76 ms per 50-iteration step,
+// now 2.36 ms.
 template <int L, bool CHEB, bool REC = false, bool CONTACT = false>
 __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) staged_sweep_kernel(SweepParams p)
 {
@@ -131,16 +139,16 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) staged_sweep_kernel(Swee
     int i       = 0;
     float xi[3] = {0.f, 0.f, 0.f};
     int k = 0, k1 = 0, n0 = 0, n1 = 0, base = 0;
-    uint2 q0 = make_uint2(0u, 0u), q1 = q0;
-    float4 st0 = make_float4(0.f, 0.f, 0.f, 0.f), st1 = st0;
+    uint32_t q0 = 0u, q1 = 0u;
+    float2 mt0 = make_float2(0.f, 0.f), mt1 = mt0;
     // The mesh tables are not written by any launch of the step: the vertex's first neighbour
-    // indices and first two incidence records are loaded before griddepcontrol.wait, so that
+    // records and first two incidence records are loaded before griddepcontrol.wait, so that
     // only the position loads remain on the path after it.
     int constexpr kPreNbr = 4;
-    uint32_t pre[kPreNbr];
+    uint2 pre[kPreNbr];
 #pragma unroll
     for (int m = 0; m < kPreNbr; ++m)
-        pre[m] = 0u;
+        pre[m] = make_uint2(0u, 0u);
     if (valid)
     {
         i    = __ldg(p.solve + s);
@@ -155,13 +163,13 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) staged_sweep_kernel(Swee
                 pre[m] = __ldg(p.nbr + n0 + lane + m * L);
         if (k < k1)
         {
-            q0  = __ldg(p.incPack + k);
-            st0 = __ldg(p.stiff + k);
+            q0  = __ldg(p.incSlots + k);
+            mt0 = __ldg(p.incMat + k);
         }
         if (k + L < k1)
         {
-            q1  = __ldg(p.incPack + k + L);
-            st1 = __ldg(p.stiff + k + L);
+            q1  = __ldg(p.incSlots + k + L);
+            mt1 = __ldg(p.incMat + k + L);
         }
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -176,18 +184,18 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) staged_sweep_kernel(Swee
             if (j < n1)
             {
                 float4 const* src = p.x;
-                if (CHEB && !(pre[m] >> 31))
+                if (CHEB && !(pre[m].x >> 31))
                     src = p.hprev;
-                slab[base + j - n0] = __ldg(src + (pre[m] & kIndexMask));
+                stage_neighbour(b, slab + base + j - n0, __ldg(src + (pre[m].x & kIndexMask)), xi, __uint_as_float(pre[m].y));
             }
         }
         for (int j = n0 + lane + kPreNbr * L; j < n1; j += L)
         {
-            uint32_t const a  = __ldg(p.nbr + j);
+            uint2 const a     = __ldg(p.nbr + j);
             float4 const* src = p.x;
-            if (CHEB && !(a >> 31))
+            if (CHEB && !(a.x >> 31))
                 src = p.hprev;
-            slab[base + j - n0] = __ldg(src + (a & kIndexMask));
+            stage_neighbour(b, slab + base + j - n0, __ldg(src + (a.x & kIndexMask)), xi, __uint_as_float(a.y));
         }
     }
     __syncwarp();
@@ -196,27 +204,18 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) staged_sweep_kernel(Swee
         // Two incidences' records in flight ahead of the one being accumulated.
         for (; k < k1; k += L)
         {
-            uint2 q2   = make_uint2(0u, 0u);
-            float4 st2 = make_float4(0.f, 0.f, 0.f, 0.f);
+            uint32_t q2 = 0u;
+            float2 mt2  = make_float2(0.f, 0.f);
             if (k + 2 * L < k1)
             {
-                q2  = __ldg(p.incPack + k + 2 * L);
-                st2 = __ldg(p.stiff + k + 2 * L);
+                q2  = __ldg(p.incSlots + k + 2 * L);
+                mt2 = __ldg(p.incMat + k + 2 * L);
             }
-            float d[3][3];
-#pragma unroll
-            for (int m = 0; m < 3; ++m)
-            {
-                float4 const xa = slab[base + int((q0.x >> (8 * m)) & 0xFFu)];
-                d[m][0] = xa.x - xi[0];
-                d[m][1] = xa.y - xi[1];
-                d[m][2] = xa.z - xi[2];
-            }
-            accumulate_incidence(b, d, st0.x, st0.y, st0.z, __uint_as_float(q0.y), st0.w);
+            staged_incidence(b, slab + base, q0, mt0);
             q0  = q1;
-            st0 = st1;
+            mt0 = mt1;
             q1  = q2;
-            st1 = st2;
+            mt1 = mt2;
         }
     }
     finish_vertex<L, CHEB, REC, CONTACT>(p, b, valid, lane, i, s, xi);
@@ -361,6 +360,62 @@ __global__ void unpack3_kernel(float4 const* __restrict__ in4, float* __restrict
     }
 }
 
+// Material words of every tet.
+__global__ void tet_material_kernel(StiffnessParams p)
+{
+    int const e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= p.nT)
+        return;
+    double const mu = p.mu[e], la = p.lambda[e], w = p.geometry[e].wg;
+    p.tets[e].mat = make_float4(float(w * mu), float(w * la), float(1.0 + mu / la), 0.f);
+}
+
+// Rest-state constants of one solve entry per warp: lanes take the entry's incidences for
+// (kappa, sigma), then its neighbours, each lane adding the b of every incidence that holds its
+// neighbour (in incidence order).  pbgb_vbd_set_material with this kernel takes 0.09 ms for 24,000
+// tets and 0.49 ms for 197,000 (most of it the host's checks and the upload of 16 B per tet); with the
+// records formed on the host and uploaded (24 B per incidence) it took 0.88 and 8.2 ms.
+__global__ void __launch_bounds__(256) stiffness_kernel(StiffnessParams p)
+{
+    int const s    = int((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    int const lane = int(threadIdx.x & 31);
+    if (s >= p.nFree)
+        return;
+    int const k0 = p.incPtr[s], k1 = p.incPtr[s + 1], n0 = p.nbrPtr[s], n1 = p.nbrPtr[s + 1];
+    for (int k = k0 + lane; k < k1; k += 32)
+    {
+        uint32_t const q = p.inc[k];
+        double b[3], kappa, sigma;
+        corner_stiffness(p.geometry[q >> 2], p.mu[q >> 2], p.lambda[q >> 2], int(q & 3u), b, kappa, sigma);
+        p.incMat[k] = make_float2(float(kappa), float(sigma));
+    }
+    double sum = 0.0;
+    for (int j = n0 + lane; j < n1; j += 32)
+    {
+        uint32_t const v = p.nbr[j].x & kIndexMask;
+        double K         = 0.0;
+        for (int k = k0; k < k1; ++k)
+        {
+            uint32_t const q = p.inc[k];
+            uint4 const t    = p.tets[q >> 2].v;
+#pragma unroll
+            for (int m = 0; m < 3; ++m)
+                if ((corner(t, int((q + 1 + m) & 3u)) & kIndexMask) == v)
+                {
+                    double b[3], kappa, sigma;
+                    corner_stiffness(p.geometry[q >> 2], p.mu[q >> 2], p.lambda[q >> 2], int(q & 3u), b, kappa, sigma);
+                    K += b[m];
+                }
+        }
+        p.nbr[j].y = __float_as_uint(float(K));
+        sum += K;
+    }
+    for (int off = 16; off > 0; off >>= 1)
+        sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    if (lane == 0)
+        p.diag[s] = float(-sum);
+}
+
 // Contact records of vertex i (SweepParams::crec): the area-scaled penalty of every listed
 // triangle (the vertex area over the summed areas of its listed triangles, times muC and the
 // triangle's area) and the corners' read rule for the colour sweep.
@@ -451,7 +506,7 @@ cudaError_t launch_sweep(SweepParams const& p, int lanes, int block, bool chebys
     int64_t const n = int64_t(p.end - p.begin) * lanes;
     if (n <= 0)
         return cudaSuccess;
-    if (!p.stiff || !p.incPack || stagedBytes > kStagedMaxBytes || (stagedBytes > 0 && (!p.nbrPtr || !p.nbr)))
+    if (!p.incMat || !p.diag || !p.nbrPtr || !p.nbr || stagedBytes > kStagedMaxBytes || (stagedBytes > 0 && !p.incSlots))
         return cudaErrorInvalidValue;
     // Contact terms exist only in the two-buffer sweep (a contact partner of the same colour is
     // read as it was before the pass): a one-buffer launch with contact lists is a caller error.
@@ -470,7 +525,7 @@ cudaError_t launch_sweep_record(SweepParams const& p, int lanes, int block, bool
     int64_t const n = int64_t(p.end - p.begin) * lanes;
     if (n <= 0)
         return cudaSuccess;
-    if (!p.tape || !p.stiff || !p.incPack || p.fc || stagedBytes > kStagedMaxBytes || (stagedBytes > 0 && (!p.nbrPtr || !p.nbr)))
+    if (!p.tape || p.fc || !p.incMat || !p.diag || !p.nbrPtr || !p.nbr || stagedBytes > kStagedMaxBytes || (stagedBytes > 0 && !p.incSlots))
         return cudaErrorInvalidValue;
     int const g = blocks_for(n, block);
     return chebyshev ? launch_sweep_t<true, true>(p, lanes, g, block, pdl, s, stagedBytes)
@@ -524,6 +579,15 @@ cudaError_t prepare_staged_sweeps()
     if (e == cudaSuccess)
         e = allow_staged_smem<true, false, true>();
     return e;
+}
+
+cudaError_t launch_stiffness(StiffnessParams const& p, cudaStream_t s)
+{
+    if (p.nT > 0)
+        tet_material_kernel<<<blocks_for(p.nT, 256), 256, 0, s>>>(p);
+    if (p.nFree > 0)
+        stiffness_kernel<<<blocks_for(int64_t(p.nFree) * 32, 256), 256, 0, s>>>(p);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_begin_substep(SubstepParams const& p, cudaStream_t s)

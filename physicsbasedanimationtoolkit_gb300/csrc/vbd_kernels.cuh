@@ -72,18 +72,17 @@ struct SweepParams
     float muC;
     float muF;
     float epsv;
-    // Per-incidence stiffness (solve order, TetStiffness resolved for the incidence's own corner):
-    // stiff[k] = (b0, b1, b2, kappa_o); incPack[k] = (neighbour slots, sigma as bits): the three
-    // other corners' positions in the vertex's neighbour list in bytes 0-2 of .x (corner order
-    // (local + 1 + m) & 3; staged sweep only).  Every incidence reads these instead of rest
-    // positions.
-    float4 const* __restrict__ stiff;
-    uint2 const* __restrict__ incPack;
-    // Neighbour staging (staged sweep only): for solve-list entry s, its distinct neighbours
-    // nbr[nbrPtr[s] .. nbrPtr[s+1]) (vertex index in bits 0-29, bit 31 set when the neighbour has a
-    // lower colour, so that the two-buffer sweep reads it from x rather than hprev).
+    // Rest-state constants of the solves (vbd_math.cuh), solve order.  Incidence k: incMat[k] =
+    // (kappa, sigma), incSlots[k] = the three other corners' positions in the vertex's neighbour list
+    // in bytes 0-2 (corner order (local + 1 + m) & 3; staged sweep only).  Solve entry s: diag[s] = the
+    // constant s of its block and its distinct neighbours nbr[nbrPtr[s] .. nbrPtr[s+1]), each (vertex
+    // index in bits 0-29, bit 31 set when the neighbour has a lower colour, so that the two-buffer
+    // sweep reads it from x rather than hprev; K as bits).
+    float2 const* __restrict__ incMat;
+    uint32_t const* __restrict__ incSlots;
+    float const* __restrict__ diag;
     int32_t const* __restrict__ nbrPtr;
-    uint32_t const* __restrict__ nbr;
+    uint2 const* __restrict__ nbr;
     // Applied Newton increments (one-buffer sweeps only, nullptr: not written): step[i] = x_new -
     // x_old for every solved vertex, the residual Anderson acceleration mixes (exact to FP32
     // relative precision, unlike the difference of two rounded positions).
@@ -133,6 +132,25 @@ struct EnergyParams
     double restEnergy;
 };
 
+// Per-tet material words and the rest-state constants of the solves from FP64 inputs (see
+// launch_stiffness).
+struct StiffnessParams
+{
+    TetGeometry const* __restrict__ geometry;
+    double const* __restrict__ mu;
+    double const* __restrict__ lambda;
+    TetRecord* __restrict__ tets; // mat written
+    int32_t const* __restrict__ solve;
+    int32_t const* __restrict__ incPtr;
+    uint32_t const* __restrict__ inc;
+    int32_t const* __restrict__ nbrPtr;
+    float2* __restrict__ incMat;
+    uint2* __restrict__ nbr; // .y written
+    float* __restrict__ diag;
+    int32_t nT;
+    int32_t nFree;
+};
+
 // Launchers (defined in vbd_kernels.cu).  Each returns the launch status.
 // pdl: launch with programmatic stream serialization, so that the kernel's mesh-table prologue
 // overlaps the tail of the previous launch on the stream (the kernel waits before reading
@@ -155,6 +173,9 @@ size_t constexpr kStagedMaxBytes = 200 * 1024;
 // Bytes of one staged neighbour: its current position (float4).
 size_t constexpr kStagedSlotBytes = sizeof(float4);
 cudaError_t prepare_staged_sweeps();
+// Writes the tets' material words (wg mu, wg lambda, 1 + mu/lambda) and incMat, nbr's K and diag of
+// every solve entry; sums in FP64, each result rounded once.
+cudaError_t launch_stiffness(StiffnessParams const& p, cudaStream_t s);
 cudaError_t launch_begin_substep(SubstepParams const& p, cudaStream_t s);
 cudaError_t launch_end_substep(SubstepParams const& p, cudaStream_t s);
 // Blocks of the objective's reduction grid (p.partials holds this many doubles).
