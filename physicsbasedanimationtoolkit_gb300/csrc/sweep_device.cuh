@@ -187,7 +187,7 @@ __device__ __forceinline__ void finish_vertex(SweepParams const& p, VertexBlock<
         g[2] += cg[2];
     }
     float dx[3];
-    bool const moved = inertia_solve(H, g, xl, xt4.w, p.h2, p.detHZero, xi, static_cast<float*>(nullptr),
+    bool const moved = inertia_solve(H, g, xl, xt4.w / p.h2, p.detHZero, xi, static_cast<float*>(nullptr),
                                      static_cast<float*>(nullptr), dx);
     if (p.step)
         p.step[i] = make_float4(dx[0], dx[1], dx[2], 0.f);

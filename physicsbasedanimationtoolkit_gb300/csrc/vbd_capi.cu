@@ -8,6 +8,7 @@
 // pass), and several meshes concatenated into one system for the batched form.
 #include "adjoint.cuh"
 #include "batched.cuh"
+#include "cluster_step.cuh"
 #include "anderson.cuh"
 #include "nesterov.cuh"
 #include "trust_region.cuh"
@@ -351,6 +352,23 @@ class VbdSystem
     DeviceArray<int32_t> batchCounters; // [0] ticket, [1] abort, then one completion counter per mesh
     DeviceArray<float> batchOmega;
 
+    // Cluster step (cluster_step.cuh): the parts of every mesh and their tables, made at creation
+    // (clusterBlocks = 0: the system has none), and the launch for the current lanes.
+    int32_t clusterBlocks = 0, clusterLocal = 0, clusterOwned = 0, clusterColor = 0, clusterTiles = 0, clusterStage = 0;
+    std::vector<int2> hostPartRange; // solve entries of every (part, colour)
+    DeviceArray<int32_t> partPtr, partOwned, partTile;
+    DeviceArray<uint32_t> partVertex;
+    DeviceArray<int2> partColor, clusterTile;
+    DeviceArray<unsigned char> tileData;
+    DeviceArray<int4> tileAt;
+    struct ClusterLaunch
+    {
+        int32_t lanes = 0, warps = 0, slabPerWarp = 0, stages = 0, resident = 0, residentRecord = 0;
+    } clusterLaunch;
+    bool stepInCluster      = false; // the last step ran (or is being captured) as a cluster launch
+    int32_t omegaIterations = -1; // iterations stepOmega holds the Chebyshev weights of
+    DeviceArray<float> stepOmega;
+
     // Graph cache for Step(dt, iterations, substeps)
     cudaGraphExec_t graph = nullptr;
     float gDt = -1.f;
@@ -482,16 +500,494 @@ class VbdSystem
         return bytes <= kStagedMaxBytes ? bytes : 0;
     }
 
+    // Lanes per vertex of plain and Chebyshev iterations on every path (the cluster step, the persistent
+    // batch, launches per colour, recorded and traced steps), which then give the same positions bit
+    // for bit.
     int lanesToUse() const
     {
         if (lanes > 0)
             return lanes;
-        // Default: enough lanes that a colour fills the GPU, few enough that the incidence loop
-        // keeps each lane busy.
+        return clusterBlocks > 0 ? clusterDefaultLanes() : launchLanes();
+    }
+
+    // The same for kernels launched per colour only (the reversed sweeps, the other accelerations,
+    // contact).  Default: enough lanes that a colour fills the GPU, few enough that the
+    // incidence loop keeps each lane busy.
+    int launchLanes() const
+    {
+        if (lanes > 0)
+            return lanes;
         int const perColor = nColors > 0 ? nFree / nColors : nFree;
-        if (perColor < 4096)
-            return 32;
-        return 4;
+        return perColor < 4096 ? 32 : 4;
+    }
+
+    // Lanes per vertex of the cluster step by default, from the solve entries n of the part's largest
+    // colour: with n L <= 320 each warp has one group of vertices at a time and the block up to 10 warps
+    // of work; fewer lanes make each vertex's chain longer, more a second round.  Measured (us per
+    // 20-iteration step): n = 10: 16 lanes 170, 8 lanes 179, 32 lanes 195; n = 25: 8 lanes 200, 4 lanes
+    // 206, 16 lanes 208; n = 69: 4 lanes 322, 2 lanes 343, 8 lanes 458; n = 148: 2 lanes 530, 4 lanes
+    // 656, 1 lane 769.
+    int clusterDefaultLanes() const
+    {
+        int L = 16;
+        while (L > 2 && clusterColor * L > 320)
+            L /= 2;
+        return L;
+    }
+
+    // Splits mesh vertices into `parts` spatially compact parts with equal numbers of solved vertices
+    // (recursive bisection at the median along the longest axis); vertices that are never solved go
+    // where the cuts put them.  part is indexed by vertex - v0.
+    static void bisect(std::vector<float4> const& X, std::vector<int32_t>& solved, std::vector<int32_t>& fixed, int32_t parts, int32_t first, int32_t* part)
+    {
+        if (parts == 1 || (solved.empty() && fixed.empty()))
+        {
+            for (auto const* list : {&solved, &fixed})
+                for (int32_t v : *list)
+                    part[v] = first;
+            return;
+        }
+        auto const& span = solved.empty() ? fixed : solved;
+        float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+        for (int32_t v : span)
+            for (int k = 0; k < 3; ++k)
+            {
+                lo[k] = std::min(lo[k], (&X[size_t(v)].x)[k]);
+                hi[k] = std::max(hi[k], (&X[size_t(v)].x)[k]);
+            }
+        int axis = 0;
+        for (int k = 1; k < 3; ++k)
+            if (hi[k] - lo[k] > hi[axis] - lo[axis])
+                axis = k;
+        // Along the axis, then the other two, so that the vertices of a grid plane split compactly.
+        auto before = [&](int32_t a, int32_t b) {
+            for (int k = 0; k < 3; ++k)
+            {
+                float const u = (&X[size_t(a)].x)[(axis + k) % 3], w = (&X[size_t(b)].x)[(axis + k) % 3];
+                if (u != w)
+                    return u < w;
+            }
+            return a < b;
+        };
+        int32_t const half = parts / 2;
+        std::vector<int32_t> s2, f2;
+        if (solved.empty())
+        {
+            auto const mid = fixed.begin() + int64_t(fixed.size()) * half / parts;
+            std::nth_element(fixed.begin(), mid, fixed.end(), before);
+            f2.assign(mid, fixed.end());
+            fixed.erase(mid, fixed.end());
+        }
+        else
+        {
+            auto const mid = solved.begin() + int64_t(solved.size()) * half / parts;
+            std::nth_element(solved.begin(), mid, solved.end(), before);
+            int32_t const pivot = *mid;
+            s2.assign(mid, solved.end());
+            solved.erase(mid, solved.end());
+            auto const cut = std::partition(fixed.begin(), fixed.end(), [&](int32_t v) { return before(v, pivot); });
+            f2.assign(cut, fixed.end());
+            fixed.erase(cut, fixed.end());
+        }
+        bisect(X, solved, fixed, half, first, part);
+        bisect(X, s2, f2, parts - half, first + half, part);
+    }
+
+    // Blocks per mesh of the cluster step and every vertex's part (rank in its mesh's cluster); 0 when
+    // the cluster step does not apply: contact, a part's positions
+    // that do not fit a block's shared memory even with 16 blocks, or a mesh so large that the whole GPU
+    // per colour is faster than one cluster per step.
+    //
+    // Blocks: as many as leave 8 solves per part and colour, while all the batch's blocks find an SM of
+    // their own (a 1331-vertex cube, us per 20-iteration step: 4 blocks 236, 8 blocks 191, 16 blocks 170;
+    // 24 cubes of 6^3 to 12^3 hexes: 2 blocks each 319, 4 blocks 220, 8 blocks 273; 200 cubes of 2^3 to
+    // 8^3: 1 block 290, 2 blocks 476).
+    // Limits: one mesh of 8,820 free vertices takes 322 us in a cluster and 321 us in colour launches,
+    // 11,638 take 377 and 362 us; batches of larger meshes keep every SM busy with the persistent
+    // kernel's tickets (64 cubes of 6^3 to 32^3: 2.8 ms, in clusters 4.0 ms), smaller ones wait there
+    // (10 cubes of 8^3 to 28^3, Chebyshev: 0.81 ms, in clusters 0.37 ms).
+    static int32_t constexpr kClusterSingleFree = 9000, kClusterBatchFree = 24000, kClusterBatchTotal = 400000;
+    int32_t chooseParts(std::vector<float4> const& X, std::vector<int32_t> const& color, std::vector<TetRecord> const& records,
+                        std::vector<int32_t> const& vPtr, std::vector<uint32_t> const& vInc, bool hasContact, std::vector<int32_t>& part) const
+    {
+        if (hasContact || nFree <= 0)
+            return 0;
+        int64_t largest = 0;
+        std::vector<int64_t> free(size_t(nMeshes), 0);
+        for (int32_t b = 0; b < nMeshes; ++b)
+        {
+            for (int32_t v = meshV0[b]; v < meshV0[b + 1]; ++v)
+                free[b] += color[v] >= 0 ? 1 : 0;
+            largest = std::max(largest, free[b]);
+        }
+        if (nMeshes == 1 ? nFree > kClusterSingleFree : (largest > kClusterBatchFree || nFree > kClusterBatchTotal))
+            return 0;
+        int sms = 0;
+        check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
+        int32_t P = 1;
+        while (P < kClusterMaxBlocks && int64_t(nMeshes) * P * 2 <= sms && largest >= int64_t(nColors) * P * 2 * 8)
+            P *= 2;
+        for (; P <= kClusterMaxBlocks; P *= 2)
+        {
+            part.assign(size_t(nV), 0);
+            for (int32_t b = 0; b < nMeshes; ++b)
+            {
+                std::vector<int32_t> solved, fixed;
+                for (int32_t v = meshV0[b]; v < meshV0[b + 1]; ++v)
+                    (color[v] >= 0 ? solved : fixed).push_back(v);
+                bisect(X, solved, fixed, P, 0, part.data());
+            }
+            // Local vertices of every part: its own and the neighbours of its solved ones.
+            int64_t local = 0, owned = 0;
+            std::vector<int64_t> stamp(size_t(nV), -1);
+            for (int32_t b = 0; b < nMeshes; ++b)
+                for (int32_t q = 0; q < P; ++q)
+                {
+                    int64_t const id = int64_t(b) * P + q;
+                    int64_t nOwn = 0, nHalo = 0;
+                    for (int32_t v = meshV0[b]; v < meshV0[b + 1]; ++v)
+                    {
+                        if (part[v] != q)
+                            continue;
+                        ++nOwn;
+                        if (color[v] < 0)
+                            continue;
+                        for (int32_t k = vPtr[v]; k < vPtr[v + 1]; ++k)
+                        {
+                            uint4 const t        = records[vInc[k] >> 2].v;
+                            uint32_t const c4[4] = {t.x, t.y, t.z, t.w};
+                            for (uint32_t w : c4)
+                            {
+                                uint32_t const j = w & kIndexMask;
+                                if (part[j] != q && stamp[j] != id)
+                                {
+                                    stamp[j] = id;
+                                    ++nHalo;
+                                }
+                            }
+                        }
+                    }
+                    local = std::max(local, nOwn + nHalo);
+                    owned = std::max(owned, nOwn);
+                }
+            // Slabs and a few tiles take about 90 KB more.
+            int64_t const float4s = acceleration == PBGB_ACCEL_CHEBYSHEV ? 2 * (local + owned) : local + owned;
+            if (local <= kClusterMaxLocal && float4s * int64_t(sizeof(float4)) <= 130 * 1024)
+                return P;
+        }
+        return 0;
+    }
+
+    // The cluster step's tables from the parts (solve order already grouped by part inside a colour).
+    // False when a tile is too large for its entries' 16-bit fields.
+    bool buildCluster(std::vector<int32_t> const& part, std::vector<int32_t> const& color, std::vector<int32_t> const& solveList,
+                      std::vector<int32_t> const& incPtrH, std::vector<uint32_t> const& slotsH, std::vector<uint2> const& nbrH)
+    {
+        int32_t const P = clusterBlocks, parts = nMeshes * P;
+        // Larger meshes first: their clusters start first.
+        std::vector<int32_t> order(static_cast<size_t>(nMeshes)), base(static_cast<size_t>(nMeshes));
+        for (int32_t b = 0; b < nMeshes; ++b)
+            order[b] = b;
+        std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
+            return meshV0[a + 1] - meshV0[a] > meshV0[b + 1] - meshV0[b];
+        });
+        for (int32_t k = 0; k < nMeshes; ++k)
+            base[order[k]] = k * P;
+        std::vector<int32_t> entryOf(size_t(nV), -1);
+        for (int32_t s = 0; s < nFree; ++s)
+            entryOf[solveList[s]] = s;
+        std::vector<std::vector<uint32_t>> local(static_cast<size_t>(parts));
+        std::vector<int32_t> owned(size_t(parts), 0), ownSlot(size_t(nV), 0);
+        for (int32_t b = 0; b < nMeshes; ++b)
+            for (int32_t v = meshV0[b]; v < meshV0[b + 1]; ++v)
+            {
+                auto& list = local[size_t(base[b] + part[v])];
+                ownSlot[v] = int32_t(list.size());
+                list.push_back(uint32_t(v) | (color[v] < 0 ? 0x80000000u : 0u));
+            }
+        std::vector<uint32_t> nbrSlot(nbrH.size());
+        std::vector<int2> hColor(size_t(parts) * size_t(nColors), make_int2(0, 0));
+        std::vector<std::pair<int32_t, uint32_t>> sends;
+        std::vector<int32_t> stamp(size_t(nV), -1), slot(size_t(nV), 0);
+        clusterLocal = clusterOwned = 0;
+        for (int32_t q = 0; q < parts; ++q)
+        {
+            auto& list       = local[size_t(q)];
+            size_t const own = list.size();
+            owned[q]         = int32_t(own);
+            for (size_t k = 0; k < own; ++k)
+            {
+                int32_t const v = int32_t(list[k] & kIndexMask), s = entryOf[v];
+                if (s < 0)
+                    continue;
+                for (int32_t j = hostNbrPtr[s]; j < hostNbrPtr[s + 1]; ++j)
+                {
+                    int32_t const w = int32_t(nbrH[j].x & kIndexMask);
+                    int32_t at      = ownSlot[w];
+                    if (part[w] != part[v])
+                    {
+                        if (stamp[w] != q)
+                        {
+                            stamp[w] = q;
+                            slot[w]  = int32_t(list.size());
+                            list.push_back(uint32_t(w) | (color[w] < 0 ? 0x80000000u : 0u));
+                            if (entryOf[w] >= 0)
+                            {
+                                sends.emplace_back(entryOf[w], uint32_t(part[v]) << 16 | uint32_t(slot[w]));
+                                ++hColor[size_t(q) * size_t(nColors) + size_t(color[w])].y;
+                            }
+                        }
+                        at = slot[w];
+                    }
+                    nbrSlot[j] = uint32_t(at) | (nbrH[j].x & 0x80000000u);
+                }
+            }
+            clusterLocal = std::max(clusterLocal, int32_t(list.size()));
+            clusterOwned = std::max(clusterOwned, int32_t(own));
+        }
+        std::stable_sort(sends.begin(), sends.end(), [](auto const& a, auto const& b) { return a.first < b.first; });
+        std::vector<uint32_t> hSend(sends.size());
+        std::vector<int32_t> sendPtr(size_t(nFree) + 1, 0);
+        for (size_t k = 0; k < sends.size(); ++k)
+        {
+            hSend[k] = sends[k].second;
+            sendPtr[sends[k].first + 1]++;
+        }
+        for (int32_t s = 0; s < nFree; ++s)
+            sendPtr[s + 1] += sendPtr[s];
+        // Solve entries of every (part, colour): inside a (mesh, colour) range the parts follow one
+        // another.
+        hostPartRange.assign(size_t(parts) * size_t(nColors), make_int2(0, 0));
+        clusterColor = 0;
+        for (int32_t b = 0; b < nMeshes; ++b)
+            for (int32_t c = 0; c < nColors; ++c)
+            {
+                int32_t s         = meshSolve[b][2 * c];
+                int32_t const end = meshSolve[b][2 * c + 1];
+                for (int32_t q = 0; q < P; ++q)
+                {
+                    int32_t const begin = s;
+                    while (s < end && part[solveList[s]] == q)
+                        ++s;
+                    size_t const pc   = size_t(base[b] + q) * size_t(nColors) + size_t(c);
+                    hostPartRange[pc] = make_int2(begin, s);
+                    hColor[pc].x      = s - begin;
+                    clusterColor      = std::max(clusterColor, s - begin);
+                }
+            }
+        // Tiles: sizes and offsets, then their contents (the material's constants come from
+        // uploadMaterial).
+        std::vector<int32_t> hPartTile(size_t(parts) + 1, 0);
+        std::vector<int2> hTile;
+        std::vector<int32_t> tileFirst;
+        size_t bytes = 0;
+        clusterTiles = clusterStage = 0;
+        auto even    = [](int64_t n) { return (n + 1) & ~int64_t(1); };
+        for (int32_t q = 0; q < parts; ++q)
+        {
+            for (int32_t c = 0; c < nColors; ++c)
+            {
+                int2 const r = hostPartRange[size_t(q) * size_t(nColors) + size_t(c)];
+                for (int32_t f = r.x; f < r.y; f += kClusterTileVertices)
+                {
+                    int32_t const e    = std::min(f + kClusterTileVertices, r.y);
+                    int64_t const nNbr = hostNbrPtr[e] - hostNbrPtr[f], nInc = incPtrH[e] - incPtrH[f];
+                    size_t const size = kClusterTileVertices * sizeof(ClusterEntry) + size_t(even(nNbr)) * sizeof(uint2) +
+                                        size_t(even(nInc)) * sizeof(float2) +
+                                        (size_t(nInc + sendPtr[e] - sendPtr[f]) * sizeof(uint32_t) + 15) / 16 * 16;
+                    if (size > kClusterMaxTile || nInc > 0xFFFF)
+                        return false;
+                    hTile.push_back(make_int2(int32_t(bytes / 16), int32_t(size)));
+                    tileFirst.push_back(f);
+                    clusterStage = std::max(clusterStage, int32_t((size + 127) / 128 * 128));
+                    bytes += size;
+                }
+            }
+            hPartTile[q + 1] = int32_t(hTile.size());
+            clusterTiles     = std::max(clusterTiles, hPartTile[q + 1] - hPartTile[q]);
+        }
+        if (bytes / 8 > size_t(INT32_MAX))
+            return false;
+        std::vector<unsigned char> hData(bytes, 0);
+        std::vector<int4> hAt(static_cast<size_t>(nFree));
+        for (size_t k = 0; k < hTile.size(); ++k)
+        {
+            int32_t const f = tileFirst[k];
+            size_t const at = size_t(hTile[k].x) * 16;
+            // The tile's last entry: up to the next tile of its (part, colour), or that range's end.
+            int32_t e = f + 1;
+            while (e < nFree && e - f < kClusterTileVertices && part[solveList[e]] == part[solveList[f]] &&
+                   color[solveList[e]] == color[solveList[f]] && meshOf(solveList[e]) == meshOf(solveList[f]))
+                ++e;
+            int32_t const nNbr = hostNbrPtr[e] - hostNbrPtr[f], nInc = incPtrH[e] - incPtrH[f];
+            size_t const nbrs  = kClusterTileVertices * sizeof(ClusterEntry);
+            size_t const mats = nbrs + size_t(even(nNbr)) * sizeof(uint2), slots = mats + size_t(even(nInc)) * sizeof(float2);
+            size_t const copies = slots + size_t(nInc) * sizeof(uint32_t);
+            for (int32_t s = f; s < f + kClusterTileVertices; ++s)
+            {
+                ClusterEntry en{};
+                en.vertex = -1;
+                if (s < e)
+                {
+                    size_t const n0 = nbrs / 8 + size_t(hostNbrPtr[s] - hostNbrPtr[f]), i0 = size_t(incPtrH[s] - incPtrH[f]);
+                    en.vertex = solveList[s];
+                    en.solve  = s;
+                    en.nbr    = uint32_t(n0) | uint32_t(hostNbrPtr[s + 1] - hostNbrPtr[s]) << 16;
+                    en.inc    = uint32_t(mats / 8 + i0) | uint32_t(incPtrH[s + 1] - incPtrH[s]) << 16;
+                    en.slot   = uint32_t(ownSlot[solveList[s]]) | uint32_t(sendPtr[s + 1] - sendPtr[s]) << 16;
+                    en.words  = uint32_t(slots / 4 + i0) | uint32_t(copies / 4 + size_t(sendPtr[s] - sendPtr[f])) << 16;
+                    hAt[s] = make_int4(int32_t(at / 16 + 2 * size_t(s - f)), int32_t(at / 8 + n0), int32_t((at + mats) / 8 + i0), 0);
+                }
+                std::memcpy(hData.data() + at + size_t(s - f) * sizeof(en), &en, sizeof(en));
+            }
+            for (int32_t j = hostNbrPtr[f]; j < hostNbrPtr[e]; ++j)
+                std::memcpy(hData.data() + at + nbrs + size_t(j - hostNbrPtr[f]) * sizeof(uint2), &nbrSlot[j], sizeof(uint32_t));
+            std::memcpy(hData.data() + at + slots, slotsH.data() + incPtrH[f], size_t(nInc) * sizeof(uint32_t));
+            std::memcpy(hData.data() + at + copies, hSend.data() + sendPtr[f], size_t(sendPtr[e] - sendPtr[f]) * sizeof(uint32_t));
+        }
+        std::vector<int32_t> hPtr(size_t(parts) + 1, 0);
+        std::vector<uint32_t> hVertex;
+        for (int32_t q = 0; q < parts; ++q)
+        {
+            hVertex.insert(hVertex.end(), local[size_t(q)].begin(), local[size_t(q)].end());
+            hPtr[q + 1] = int32_t(hVertex.size());
+        }
+        auto put = [&](auto& array, auto const& host) {
+            array.allocate(host.size());
+            array.upload(host.data(), host.size(), stream);
+        };
+        put(partPtr, hPtr);
+        put(partOwned, owned);
+        put(partVertex, hVertex);
+        put(partColor, hColor);
+        put(partTile, hPartTile);
+        put(clusterTile, hTile);
+        put(tileData, hData);
+        put(tileAt, hAt);
+        check(cudaStreamSynchronize(stream), "cudaStreamSynchronize"); // the uploads read local arrays
+        return true;
+    }
+
+    int32_t meshOf(int32_t v) const
+    {
+        return int32_t(std::upper_bound(meshV0.begin(), meshV0.end(), v) - meshV0.begin()) - 1;
+    }
+
+    // The size fields of the cluster step's launch.
+    ClusterStepParams clusterShape(ClusterLaunch const& c) const
+    {
+        ClusterStepParams p{};
+        p.nColors       = nColors;
+        p.localCapacity = clusterLocal;
+        p.ownedCapacity = clusterOwned;
+        p.slabPerWarp   = c.slabPerWarp;
+        p.stages        = c.stages;
+        p.stageBytes    = clusterStage;
+        return p;
+    }
+
+    // Makes the cluster step's launch for the current lanes (outside any stream capture).  False: the
+    // system takes the other paths.
+    bool prepareClusterLaunch(bool record)
+    {
+        if (clusterBlocks < 1 || !stagedOk || !staged || !persistent || profiling || (nMeshes > 1 && batchPoison >= 0))
+            return false;
+        bool const cheb = acceleration == PBGB_ACCEL_CHEBYSHEV;
+        int const L     = lanesToUse();
+        if (clusterLaunch.lanes != L)
+        {
+            ClusterLaunch c;
+            c.lanes            = L;
+            c.warps            = std::clamp<int32_t>((clusterColor * L + 31) / 32, 4, kClusterMaxWarps);
+            for (int2 const r : hostPartRange)
+                for (int32_t s = r.x; s < r.y; s += 32 / L)
+                    c.slabPerWarp = std::max(c.slabPerWarp, hostNbrPtr[std::min(s + 32 / L, r.y)] - hostNbrPtr[s]);
+            // As many ring slots as fit, all of a part's tiles when they do; the solving warps' tiles must
+            // fit the ring (cluster_step.cu), so fewer warps where they do not.
+            for (; c.warps >= 1; --c.warps)
+            {
+                c.stages          = 0;
+                size_t const rest = cluster_step_smem(clusterShape(c), c.warps, cheb);
+                if (rest < kClusterMaxBytes)
+                    c.stages = int32_t(std::min<size_t>({size_t(kClusterMaxStages), size_t(clusterTiles),
+                                                         (kClusterMaxBytes - rest) / (size_t(clusterStage) + 2 * sizeof(uint64_t))}));
+                if (c.stages >= std::min(2, clusterTiles) && c.stages * L >= c.warps)
+                    break;
+            }
+            if (c.warps >= 1)
+            {
+                size_t const smem = cluster_step_smem(clusterShape(c), c.warps, cheb);
+                c.resident        = cluster_step_resident(L, c.warps, clusterBlocks, smem, cheb, false);
+                c.residentRecord  = cluster_step_resident(L, c.warps, clusterBlocks, smem, cheb, true);
+            }
+            clusterLaunch = c;
+        }
+        return (record ? clusterLaunch.residentRecord : clusterLaunch.resident) > 0;
+    }
+
+    // Whether a step is colour sweeps alone (fused Chebyshev included): also the trust region's curved
+    // path, and Nesterov acceleration that starts after the last iteration.
+    bool plainForm(int32_t iterations) const
+    {
+        return acceleration == PBGB_ACCEL_NONE || acceleration == PBGB_ACCEL_CHEBYSHEV ||
+               (acceleration == PBGB_ACCEL_NESTEROV && nesterovStart >= iterations - 1) ||
+               (acceleration == PBGB_ACCEL_TRUST_REGION && trCurved);
+    }
+
+    // The same, with the Chebyshev weights of at least `iterations` on the device.
+    bool prepareCluster(int32_t iterations, bool record)
+    {
+        if (!plainForm(iterations) || !prepareClusterLaunch(record))
+            return false;
+        if (acceleration == PBGB_ACCEL_CHEBYSHEV && omegaIterations < iterations)
+        {
+            check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+            std::vector<float> om(size_t(std::max(iterations, 1)), 1.f);
+            double omega = 0.0;
+            for (int32_t k = 0; k < iterations; ++k)
+            {
+                omega         = chebyshev_omega<double>(k, rho * rho, omega, chebFormula);
+                om[size_t(k)] = float(omega);
+            }
+            invalidate(); // captured graphs hold the array's address
+            stepOmega.allocate(om.size());
+            check(cudaMemcpy(stepOmega.get(), om.data(), sizeof(float) * om.size(), cudaMemcpyHostToDevice), "H2D");
+            omegaIterations = iterations;
+        }
+        return true;
+    }
+
+    // One launch for the whole step; slot0 >= 0: recorded into the tape's slots from slot0.
+    void enqueueClusterStep(float dt, int32_t iterations, int32_t substeps, int32_t slot0)
+    {
+        float const h   = dt / float(substeps);
+        bool const cheb = acceleration == PBGB_ACCEL_CHEBYSHEV, record = slot0 >= 0;
+        ClusterStepParams p = clusterShape(clusterLaunch);
+        p.sweep.h        = h;
+        p.sweep.h2       = h * h;
+        p.sweep.kD       = kD;
+        p.sweep.detHZero = detHZero;
+        p.sub            = substepParams(h);
+        p.omega          = stepOmega.get();
+        p.partPtr        = partPtr.get();
+        p.partOwned      = partOwned.get();
+        p.partVertex     = partVertex.get();
+        p.partColor      = partColor.get();
+        p.partTile       = partTile.get();
+        p.tiles          = clusterTile.get();
+        p.tileData       = tileData.get();
+        p.iterations     = iterations;
+        p.substeps       = substeps;
+        if (record)
+        {
+            p.tapeX          = slotX(slot0, 0);
+            p.tapeRaw        = cheb ? slotRaw(slot0, 0) : nullptr;
+            p.tapeH          = slotTape(slot0, 0);
+            p.tapeS          = slotStart(slot0, 0);
+            p.tapeIterations = tapeIters;
+            p.nFree          = nFree;
+        }
+        check(launch_cluster_step(p, clusterLaunch.lanes, clusterLaunch.warps, clusterBlocks, nMeshes, cheb, record, stream), "cluster_step");
     }
 
     void build(pbgb_vbd_desc const* descs, int32_t nMeshes)
@@ -682,17 +1178,22 @@ class VbdSystem
                     vInc[cur[a[q]]++] = (uint32_t(e) << 2) | uint32_t(q);
             }
         }
-        // Colour-major solve list: colour c = union of every mesh's partition c; inside a colour,
-        // stable order by decreasing degree so that lanes of a warp see similar trip counts.
-        // Inside a colour the meshes follow one another, each mesh's entries in stable order of
-        // decreasing degree, so that a (mesh, colour) pair is one range of the list.
-        std::vector<int32_t> hsolve;
-        hsolve.reserve(nFree);
-        colorPtr.assign(size_t(nColors) + 1, 0);
         this->nMeshes = nMeshes;
         meshV0.assign(size_t(nMeshes) + 1, 0);
         for (int32_t b = 0; b < nMeshes; ++b)
             meshV0[b + 1] = meshV0[b] + descs[b].n_vertices;
+        check(cudaGetDevice(&device), "cudaGetDevice");
+        std::vector<int32_t> part;
+        clusterBlocks = chooseParts(hX, color, hrec, vPtr, vInc, d0.n_collision_triangles > 0, part);
+        if (clusterBlocks == 0)
+            part.assign(size_t(nV), 0);
+        // Colour-major solve list: colour c = union of every mesh's partition c.  Inside a colour the
+        // meshes follow one another, so that a (mesh, colour) pair is one range of the list; inside it
+        // the parts of the cluster step follow one another, each in stable order of decreasing degree,
+        // so that lanes of a warp see similar trip counts.
+        std::vector<int32_t> hsolve;
+        hsolve.reserve(nFree);
+        colorPtr.assign(size_t(nColors) + 1, 0);
         meshSolve.assign(size_t(nMeshes), std::vector<int32_t>(2 * size_t(nColors), 0));
         for (int32_t c = 0; c < nColors; ++c)
         {
@@ -705,7 +1206,7 @@ class VbdSystem
                     for (int32_t k = d.Pptr[c]; k < d.Pptr[c + 1]; ++k)
                         hsolve.push_back(d.Padj[k] + meshV0[b]);
                 std::stable_sort(hsolve.begin() + start, hsolve.end(), [&](int32_t a, int32_t q) {
-                    return deg[a] > deg[q];
+                    return part[a] != part[q] ? part[a] < part[q] : deg[a] > deg[q];
                 });
                 meshSolve[b][2 * c + 1] = int32_t(hsolve.size());
             }
@@ -733,6 +1234,7 @@ class VbdSystem
         stagedOk = true;
         {
             std::vector<uint32_t> list;
+            std::vector<int32_t> seen(size_t(nV), -1), where(size_t(nV), 0); // last entry that lists v, its slot there
             for (int32_t s = 0; s < nFree; ++s)
             {
                 list.clear();
@@ -747,13 +1249,14 @@ class VbdSystem
                     for (int m = 0; m < 3; ++m)
                     {
                         uint32_t const ca = c4[(il + 1 + m) & 3];
-                        uint32_t const a  = (ca & kIndexMask) | ((ca >> 30) < own ? 0x80000000u : 0u);
-                        size_t idx        = 0;
-                        while (idx < list.size() && list[idx] != a)
-                            ++idx;
-                        if (idx == list.size())
-                            list.push_back(a);
-                        slots |= uint32_t(idx) << (8 * m);
+                        uint32_t const v  = ca & kIndexMask;
+                        if (seen[v] != s)
+                        {
+                            seen[v]  = s;
+                            where[v] = int32_t(list.size());
+                            list.push_back(v | ((ca >> 30) < own ? 0x80000000u : 0u));
+                        }
+                        slots |= uint32_t(where[v]) << (8 * m);
                     }
                     hSlots[k] = slots; // meaningful only while the list has at most 256 entries
                 }
@@ -767,7 +1270,6 @@ class VbdSystem
         hostRecords = std::move(hrec);
 
         // Device allocation and upload.
-        check(cudaGetDevice(&device), "cudaGetDevice");
         check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
         x.allocate(nV);
         xt.allocate(nV);
@@ -850,6 +1352,8 @@ class VbdSystem
         dLambda.allocate(size_t(nT));
         incPtr.upload(hIncPtr.data(), hIncPtr.size(), stream);
         inc.upload(hInc.data(), hInc.size(), stream);
+        if (!stagedOk || clusterBlocks == 0 || !buildCluster(part, color, hsolve, hIncPtr, hSlots, hNbr))
+            clusterBlocks = 0;
         uploadMaterial();
         if (stagedOk)
         {
@@ -992,6 +1496,8 @@ class VbdSystem
         p.nbrPtr   = nbrPtr.get();
         p.incMat   = incMat.get();
         p.nbr      = nbr.get();
+        p.tileData = clusterBlocks > 0 ? tileData.get() : nullptr;
+        p.tileAt   = tileAt.get();
         p.diag     = diag.get();
         p.nT       = nT;
         p.nFree    = nFree;
@@ -1083,6 +1589,7 @@ class VbdSystem
         checkDifferentiable();
         if (iterations != tapeIters || slot0 < 0 || int64_t(slot0) + substeps > tapeSlots)
             throw std::invalid_argument("pbgb_vbd_step_record: slots or iteration count differ from pbgb_vbd_adjoint_reserve");
+        bool const cluster = prepareCluster(iterations, true);
         if (recGraphs.size() < size_t(tapeSlots))
             recGraphs.resize(size_t(tapeSlots));
         SlotGraph& g = recGraphs[slot0];
@@ -1092,7 +1599,12 @@ class VbdSystem
             if (g.exec)
                 cudaGraphExecDestroy(g.exec);
             g.exec     = nullptr;
-            g.exec     = capture([&] { enqueueRecord(dt, iterations, substeps, slot0); });
+            g.exec     = capture([&] {
+                if (cluster)
+                    enqueueClusterStep(dt, iterations, substeps, slot0);
+                else
+                    enqueueRecord(dt, iterations, substeps, slot0);
+            });
             g.dt       = dt;
             g.iters    = iterations;
             g.sub      = substeps;
@@ -1226,7 +1738,7 @@ class VbdSystem
 
     void enqueueAdjoint(int32_t slot0, int32_t substeps, float* xbar, float* vbar, float* pbar, double* dlogmu, double* dloglambda)
     {
-        int const L     = lanesToUse();
+        int const L     = launchLanes();
         bool const cheb = acceleration == PBGB_ACCEL_CHEBYSHEV;
         // Chebyshev weights of the iterations, as the forward formed them.
         std::vector<float> om(size_t(std::max(tapeIters, 1)), 1.f);
@@ -1461,6 +1973,11 @@ class VbdSystem
 
     void enqueueStep(float dt, int32_t iterations, int32_t substeps, StepHooks const* hooks = nullptr)
     {
+        if (!hooks && stepInCluster)
+        {
+            enqueueClusterStep(dt, iterations, substeps, -1);
+            return;
+        }
         if (!hooks && persistentActive() && plan.iters == iterations && plan.sub == substeps && plan.grid > 0 &&
             plan.lanes == lanesToUse() && plan.block == std::min(block, 256) && plan.tile == batchTile)
         {
@@ -1504,7 +2021,7 @@ class VbdSystem
             w.muF    = muF;
             w.epsv   = epsv;
         }
-        int const L = lanesToUse();
+        int const L = plainOnly || plainForm(iterations) ? lanesToUse() : launchLanes();
         if (profiling)
             ensureEvents(size_t(iterations) * size_t(substeps));
         float4* H[2] = {h0.get(), h1.get()};
@@ -1890,8 +2407,10 @@ class VbdSystem
     // Anderson and Broyden share the window buffers and kernels.
     bool windowed() const { return acceleration == PBGB_ACCEL_ANDERSON || acceleration == PBGB_ACCEL_BROYDEN; }
 
-    int64_t launchesPerStep(int32_t iterations, int32_t substeps) const
+    int64_t launchesPerStep(int32_t iterations, int32_t substeps)
     {
+        if (plainForm(iterations) && prepareClusterLaunch(false))
+            return 1;
         if (persistentActive() && plan.iters == iterations && plan.sub == substeps && plan.grid > 0)
             return plan.nItems > 0 ? 1 : 0;
         int64_t perIter = 0;
@@ -1939,7 +2458,11 @@ class VbdSystem
     void step(float dt, int32_t iterations, int32_t substeps)
     {
         reserveTrustLog(iterations, substeps);
-        if (persistentActive())
+        bool const cluster = prepareCluster(iterations, false);
+        if (cluster != stepInCluster)
+            graphValid = false;
+        stepInCluster = cluster;
+        if (!cluster && persistentActive())
         {
             int32_t const before = plan.nItems, beforeGrid = plan.grid;
             bool const same = plan.iters == iterations && plan.sub == substeps && plan.lanes == lanesToUse() &&
@@ -2098,6 +2621,9 @@ class VbdSystem
                 for (int32_t B : blockSet)
                 {
                     lanes = L;
+                    // The cluster step sizes its own blocks.
+                    if (plainForm(iterations) && prepareClusterLaunch(false) && B != 256)
+                        continue;
                     block = B;
                     invalidate();
                     step(dt, iterations, substeps); // capture + warm-up
@@ -2160,7 +2686,7 @@ class VbdSystem
         if (f[1] != 0)
         {
             check(cudaMemset(flags.get(), 0, sizeof(f)), "cudaMemset");
-            lastError = "a bounded device wait of the persistent batched step gave up; the step's positions are not valid";
+            lastError = "a bounded device wait of the persistent step gave up; the step's positions are not valid";
             return kTimeout;
         }
         if (f[0] != 0)

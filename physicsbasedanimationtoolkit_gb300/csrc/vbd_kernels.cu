@@ -1,5 +1,6 @@
 // CUDA kernels of the VBD step (sm_103a).  See vbd_kernels.cuh for the data layout.
 #include "vbd_kernels.cuh"
+#include "cluster_step.cuh"
 #include "energy.cuh"
 #include "sweep_device.cuh"
 
@@ -388,6 +389,8 @@ __global__ void __launch_bounds__(256) stiffness_kernel(StiffnessParams p)
         double b[3], kappa, sigma;
         corner_stiffness(p.geometry[q >> 2], p.mu[q >> 2], p.lambda[q >> 2], int(q & 3u), b, kappa, sigma);
         p.incMat[k] = make_float2(float(kappa), float(sigma));
+        if (p.tileData)
+            reinterpret_cast<float2*>(p.tileData)[p.tileAt[s].z + k - k0] = p.incMat[k];
     }
     double sum = 0.0;
     for (int j = n0 + lane; j < n1; j += 32)
@@ -408,12 +411,18 @@ __global__ void __launch_bounds__(256) stiffness_kernel(StiffnessParams p)
                 }
         }
         p.nbr[j].y = __float_as_uint(float(K));
+        if (p.tileData)
+            reinterpret_cast<uint2*>(p.tileData)[p.tileAt[s].y + j - n0].y = p.nbr[j].y;
         sum += K;
     }
     for (int off = 16; off > 0; off >>= 1)
         sum += __shfl_xor_sync(0xffffffffu, sum, off);
     if (lane == 0)
+    {
         p.diag[s] = float(-sum);
+        if (p.tileData)
+            reinterpret_cast<ClusterEntry*>(p.tileData + 16 * size_t(p.tileAt[s].x))->diag = float(-sum);
+    }
 }
 
 // Contact records of vertex i (SweepParams::crec): the area-scaled penalty of every listed

@@ -146,6 +146,10 @@ struct StiffnessParams
     int32_t const* __restrict__ nbrPtr;
     float2* __restrict__ incMat;
     uint2* __restrict__ nbr; // .y written
+    // The cluster step's tiles (nullptr: none), which hold the same constants: per solve entry, the
+    // offsets of its entry (16-byte units), first neighbour and first incidence (8-byte units).
+    unsigned char* __restrict__ tileData;
+    int4 const* __restrict__ tileAt;
     float* __restrict__ diag;
     int32_t nT;
     int32_t nFree;

@@ -220,23 +220,36 @@ PBGB_HD void elastic_system(VertexBlock<T> const& b, T const* xt, T const* x, T 
     }
 }
 
+// a - b, rounded by itself (never contracted with the operation that made b).
+template <class T>
+PBGB_HD T subtract_rounded(T a, T b)
+{
+#if defined(__CUDA_ARCH__)
+    if constexpr (sizeof(T) == sizeof(float))
+        return __fsub_rn(a, b);
+    else
+        return __dsub_rn(a, b);
+#else
+    return a - b;
+#endif
+}
+
 // Inertia (sim/vbd/Kernels.h:310-322) and the 3x3 Newton step with the near-singular skip
 // (:329-339).  Updates x in place; returns false when the step was skipped.  dxOut (optional): the
 // applied increment -H^-1 g (zero when skipped).
+//   K: m / h^2 of the vertex.
 template <class T>
 PBGB_HD bool inertia_solve(
     T* H,
     T* g,
     T const* xtilde,
-    T m,
-    T h2,
+    T K,
     T detHZero,
     T* x,
     T* gout  = nullptr,
     T* Hout  = nullptr,
     T* dxOut = nullptr)
 {
-    T const K = m / h2;
     H[0] += K;
     H[3] += K;
     H[5] += K;
@@ -270,9 +283,11 @@ PBGB_HD bool inertia_solve(
     T const d0  = inv * (a00 * g[0] + a01 * g[1] + a02 * g[2]);
     T const d1  = inv * (a01 * g[0] + a11 * g[1] + a12 * g[2]);
     T const d2  = inv * (a02 * g[0] + a12 * g[1] + a22 * g[2]);
-    x[0] -= d0;
-    x[1] -= d1;
-    x[2] -= d2;
+    // Rounded as written: fused into the product where d is not stored, a caller's step would differ
+    // by a bit from another's.
+    x[0] = subtract_rounded(x[0], d0);
+    x[1] = subtract_rounded(x[1], d1);
+    x[2] = subtract_rounded(x[2], d2);
     if (dxOut)
     {
         dxOut[0] = -d0;
@@ -299,7 +314,7 @@ PBGB_HD bool newton_update(
 {
     T H[6], g[3];
     elastic_system(b, xt, x, h, kD, H, g);
-    return inertia_solve(H, g, xtilde, m, h2, detHZero, x, gout, Hout);
+    return inertia_solve(H, g, xtilde, m / h2, detHZero, x, gout, Hout);
 }
 
 // Vertex-triangle contact (sim/vbd/Kernels.h:215-302 of the reference): penalty 1/2 muC d^2 on the

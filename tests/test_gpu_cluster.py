@@ -1,0 +1,88 @@
+"""The cluster step (one launch per step, a mesh's parts in the blocks of a thread-block cluster) against
+launches per colour: the per-vertex arithmetic, its order and the lanes are the same, so positions and
+velocities must be equal bit for bit, whatever the number of blocks, the ring of tiles or the rounds of a
+colour; and a recorded rollout must tape the same iterates."""
+
+import numpy as np
+import pytest
+
+from physicsbasedanimationtoolkit_gb300 import _capi, meshgen, pbat
+
+pytestmark = pytest.mark.gpu
+
+
+def data_of(nx, ny, nz, rho=None, kD=0.0, strategy=4, seed=0):
+    X, T = meshgen.hex_grid(nx, ny, nz, hi=(nx / nz, ny / nz, 1.0))
+    dbc = meshgen.face_vertices(X, 0, 0.0)
+    X = meshgen.jitter(X, 0.02 / nz, seed)
+    mu, lam = meshgen.lame(np.full(T.shape[0], 1e6), np.full(T.shape[0], 0.45))
+    v = np.random.default_rng(seed).uniform(-0.5, 0.5, X.shape)
+    d = (pbat.sim.vbd.Data().with_volume_mesh(X.T, T.T).with_material(np.full(T.shape[0], 1000.0), mu, lam)
+         .with_dirichlet_vertices(dbc).with_velocity(v.T).with_initialization_strategy(strategy))
+    if rho is not None:
+        d = d.with_chebyshev_acceleration(rho)
+    if kD:
+        d = d.with_rayleigh_damping(kD)
+    return d.construct()
+
+
+def set_persistent(I, on):
+    _capi.check(_capi.lib().pbgb_vbd_set_persistent(I.handle, int(on)), I.handle)
+
+
+# Sizes: one hex (4 free vertices), 1 to 16 blocks, parts of uneven size, parts whose tiles do not all
+# fit the ring (20^3), and the smallest mesh past the limit.  Lanes 1 and 32 give several rounds of
+# groups per colour and tiles shared by many warps.
+@pytest.mark.parametrize("shape,lanes", [((1, 1, 1), 0), ((3, 2, 2), 32), ((5, 4, 4), 0), ((7, 5, 4), 8), ((9, 9, 9), 4),
+                                         ((31, 7, 6), 0), ((13, 11, 10), 32), ((16, 16, 16), 1), ((20, 20, 20), 0),
+                                         ((20, 20, 20), 2), ((20, 20, 22), 0)])
+@pytest.mark.parametrize("mode", ["plain", "chebyshev_damped_substeps"])
+def test_cluster_step_equals_colour_launches(shape, lanes, mode):
+    kw, sub = ({}, 1) if mode == "plain" else (dict(rho=0.85, kD=1e-3, strategy=3), 2)
+    d = data_of(*shape, **kw)
+    A, B = pbat.gpu.vbd.Integrator(d), pbat.gpu.vbd.Integrator(d)
+    for I in (A, B):
+        I.lanes_per_vertex = lanes
+    set_persistent(B, False)
+    for _ in range(3):
+        A.step(1 / 60, 6, sub)
+        B.step(1 / 60, 6, sub)
+    assert A.launches_per_step(6, sub) == (1 if A.n_free <= 9000 else B.launches_per_step(6, sub))
+    assert B.launches_per_step(6, sub) > 1
+    np.testing.assert_array_equal(A.x, B.x)
+    np.testing.assert_array_equal(A.v, B.v)
+
+
+@pytest.mark.parametrize("n_meshes,nmin,nmax", [(1, 3, 3), (3, 1, 12), (9, 2, 9), (40, 2, 5)])
+def test_cluster_batch_equals_colour_launches(n_meshes, nmin, nmax):
+    datas = [data_of(n, n, n, rho=0.8, seed=n) for n in np.linspace(nmin, nmax, n_meshes).astype(int)]
+    A, B = pbat.gpu.vbd.BatchedIntegrator(datas), pbat.gpu.vbd.BatchedIntegrator(datas)
+    B.persistent = False
+    for _ in range(2):
+        A.step(1 / 60, 5, 2)
+        B.step(1 / 60, 5, 2)
+    assert A.launches_per_step(5, 2) == 1
+    np.testing.assert_array_equal(A.x, B.x)
+    np.testing.assert_array_equal(A.v, B.v)
+
+
+@pytest.mark.parametrize("rho", [None, 0.85])
+@pytest.mark.parametrize("shape", [(2, 2, 2), (12, 5, 4)])
+def test_recorded_cluster_rollout_equals_colour_launches(shape, rho):
+    torch = pytest.importorskip("torch")
+    d = data_of(*shape, rho=rho, strategy=2)
+    out = []
+    for on in (True, False):
+        I = pbat.gpu.vbd.Integrator(d)
+        set_persistent(I, on)
+        x0 = torch.tensor(np.ascontiguousarray(d.X.T), dtype=torch.float32, device="cuda", requires_grad=True)
+        v0 = torch.tensor(np.ascontiguousarray(d.v.T), dtype=torch.float32, device="cuda", requires_grad=True)
+        mu, lam = torch.tensor(d.lame[0]), torch.tensor(d.lame[1])
+        x, v = pbat.gpu.vbd.rollout(I, mu, lam, x0, v0, dt=1 / 60, iterations=6, steps=3, substeps=2, checkpoint_every=2)
+        ((x ** 2).sum() + (v ** 2).sum()).backward()
+        out.append((x.detach().cpu().numpy(), v.detach().cpu().numpy(), x0.grad.cpu().numpy(), v0.grad.cpu().numpy()))
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+    # The same tape; the reversed sweeps add to neighbours' adjoints with FP32 atomics in any order.
+    for a, b in zip(out[0][2:], out[1][2:]):
+        assert np.linalg.norm(a - b) <= 1e-4 * np.linalg.norm(b)
