@@ -687,6 +687,11 @@ __device__ __forceinline__ float point_tet_sqdist(float3 p, float3 a, float3 b, 
 // then right, so the right child is visited first), leaves pruned by their box, exact ties (eps 0)
 // kept in a list of 8 in visit order; the reference's callback writes every listed simplex in turn,
 // so the last one stays.  Squared distances order the candidates as distances do.
+//
+// Bound by its chain of dependent node reads, one query per thread: the order of the visits is the
+// reference's, not the nearest first, so without a bound most of the tree's right side is read before
+// the nearest leaf is.  21,904 queries on 43,218 triangles: a whole build and query from host arrays
+// took 3.75 ms with this kernel at 1.5 ms; with the descent's bound 2.64 ms.
 template <int K>
 __global__ void nearest_simplex_kernel(BvhView V, int32_t nq, float4 const* __restrict__ X, float4 const* __restrict__ P, int32_t const* __restrict__ S, int32_t* __restrict__ nn, int32_t* __restrict__ flags)
 {
@@ -700,6 +705,25 @@ __global__ void nearest_simplex_kernel(BvhView V, int32_t nq, float4 const* __re
     }
     float3 const x          = f3(X[q]);
     int32_t const leafBegin = V.n - 1;
+    auto distance           = [&](int32_t i) {
+        int32_t const* const c = S + size_t(i) * K;
+        return K == 3 ? point_triangle_sqdist(x, f3(P[c[0]]), f3(P[c[1]]), f3(P[c[2]]))
+                      : point_tet_sqdist(x, f3(P[c[0]]), f3(P[c[1]]), f3(P[c[2]]), f3(P[c[K - 1]]));
+    };
+    // A bound on the nearest distance: the leaf reached by descending into the nearer child.  With it
+    // the scan below passes over subtrees whose box lies beyond it by more than the rounding of the two
+    // distances (some 1e-7 of the coordinates): none of their leaves can be nearest or tie, and no
+    // decision about one that can depends on them.
+    int32_t node = 0;
+    while (node < leafBegin)
+    {
+        int32_t const l = node_link(node_lo(V, node)), r = node_link(node_hi(V, node));
+        float const dl = point_box_sqdist(x, node_lo(V, l), node_hi(V, l)), dr = point_box_sqdist(x, node_lo(V, r), node_hi(V, r));
+        node           = dr <= dl ? r : l;
+    }
+    float const reach  = sqrtf(distance(node_link(node_lo(V, node))));
+    float const margin = reach + 2e-6f * (fabsf(x.x) + fabsf(x.y) + fabsf(x.z) + reach);
+    float const bound  = margin * margin;
     int32_t stack[kBvhStack];
     int top      = 0;
     stack[top++] = 0;
@@ -708,12 +732,13 @@ __global__ void nearest_simplex_kernel(BvhView V, int32_t nq, float4 const* __re
     float dmin = FLT_MAX;
     while (top > 0)
     {
-        int32_t const node = stack[--top];
-        float4 const nl    = node_lo(V, node);
-        float4 const nh    = node_hi(V, node);
-        if (point_box_sqdist(x, nl, nh) > dmin)
+        int32_t const at = stack[--top];
+        float4 const nl  = node_lo(V, at);
+        float4 const nh  = node_hi(V, at);
+        float const box  = point_box_sqdist(x, nl, nh);
+        if (box > dmin || box > bound)
             continue;
-        if (node < leafBegin)
+        if (at < leafBegin)
         {
             if (top + 2 > kBvhStack)
             {
@@ -725,15 +750,13 @@ __global__ void nearest_simplex_kernel(BvhView V, int32_t nq, float4 const* __re
             stack[top++] = node_link(nh);
             continue;
         }
-        int32_t const i      = node_link(nl);
-        int32_t const* const c = S + size_t(i) * K;
-        float const d = K == 3 ? point_triangle_sqdist(x, f3(P[c[0]]), f3(P[c[1]]), f3(P[c[2]]))
-                               : point_tet_sqdist(x, f3(P[c[0]]), f3(P[c[1]]), f3(P[c[2]]), f3(P[c[K - 1]]));
+        int32_t const i = node_link(nl);
+        float const d   = distance(i);
         if (d < dmin)
         {
-            count     = 0;
+            count         = 0;
             list[count++] = i;
-            dmin      = d;
+            dmin          = d;
         }
         else if (d <= dmin && count < kMaxContacts)
             list[count++] = i;

@@ -274,3 +274,41 @@ def test_point_tetrahedron_nearest_neighbours_are_nearest():
         d = np.array([_np_point_tet(P[q].astype(np.float64), *X64[T[j]]) for j in range(T.shape[0])])
         assert 0 <= t < T.shape[0]
         assert d[t] <= d.min() + 1e-5
+
+
+@pytest.mark.parametrize("n,scale,offset", [(1, 1.0, 0.0), (2, 0.5, 3.0), (9, 1.0, 0.0), (16, 4.0, -64.0), (33, 0.25, 128.0)])
+@pytest.mark.parametrize("height", [0.0, 0.5, 1024.0])
+def test_nearest_triangle_among_exact_ties(n, scale, offset, height):
+    """Queries over the vertices, edge middles and face interiors of a flat sheet whose coordinates are
+    dyadic, so that every squared distance is rounded once and ties are many: the pick is the last of the first 8
+    nearest triangles in decreasing leaf order, whatever the query passes over on its way."""
+    i, j = (a.ravel() for a in np.meshgrid(np.arange(n + 1), np.arange(n + 1), indexing="ij"))
+    P = np.stack([i * scale + offset, j * scale + offset, 0.0 * i], 1).astype(np.float32)
+    a, b = (c.ravel() for c in np.meshgrid(np.arange(n), np.arange(n), indexing="ij"))
+    v = a * (n + 1) + b
+    F = np.concatenate([np.stack([v, v + n + 1, v + n + 2], 1), np.stack([v, v + n + 2, v + 1], 1)])
+    Q = np.concatenate([P, P + [scale / 2, 0, 0], P + [scale / 2, scale / 2, 0], P + [scale / 2, scale / 4, 0],
+                        P - [4 * scale, 0, 0]]).astype(np.float32)
+    Q[:, 2] = height
+    bvh = pbat.gpu.geometry.Bvh(F.shape[0])
+    boxes = pbat.gpu.geometry.Aabb()
+    boxes.construct(P.T, F.T)
+    bvh.build(boxes, P.min(0) - 1, P.max(0) + 1)
+    nn = bvh.point_triangle_nearest_neighbours(boxes, Q.T, P.T, F.T)
+    # Squared distances to the nearest point of a right triangle of the sheet, exact in FP64 and then
+    # rounded to FP32 with the height's square (which hides small differences far above the sheet).
+    A = P[F].astype(np.float64)
+    q = Q[:, None, :2].astype(np.float64)
+    lo, hi = A[:, :, :2].min(1), A[:, :, :2].max(1)
+    c = np.clip(q, lo, hi)
+    u = (c - lo) / (hi - lo)
+    lower = np.arange(F.shape[0]) < n * n  # the triangle below the diagonal: u >= v
+    wrong = np.where(lower, u[..., 1] - u[..., 0], u[..., 0] - u[..., 1])
+    # A clipped point on the far side of the diagonal is nearest to the diagonal's projection.
+    t = np.clip(((q - lo) / (hi - lo)).sum(-1) / 2, 0, 1)
+    near = np.where((wrong > 0)[..., None], lo + t[..., None] * (hi - lo), c)
+    d = (((q - near) ** 2).sum(-1) + height**2).astype(np.float32)
+    order = bvh.ordering[::-1]
+    for k in range(Q.shape[0]):
+        ties = order[d[k, order] == d[k].min()][:8]
+        assert nn[k] == ties[-1], (k, Q[k], ties, nn[k])
