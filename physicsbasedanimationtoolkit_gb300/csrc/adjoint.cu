@@ -118,9 +118,9 @@ __global__ void __launch_bounds__(256) adjoint_sweep_kernel(AdjointSweepParams p
                 own[1] += c[m][1];
                 own[2] += c[m][2];
             }
-            // One corner of each tet per colour: this lane is the only writer of tet e here.
-            p.dlogmu[a.e] -= double(dmu);
-            p.dloglambda[a.e] -= double(dla);
+            // Added in L2 without a value returned: nothing here waits for the FP64 sums.
+            atomicAdd(p.dlogmu + a.e, -double(dmu));
+            atomicAdd(p.dloglambda + a.e, -double(dla));
             k += L;
             has = k < k1;
             if (has)
