@@ -511,14 +511,23 @@ class VbdSystem
     }
 
     // The same for kernels launched per colour only (the reversed sweeps, the other accelerations,
-    // contact).  Default: enough lanes that a colour fills the GPU, few enough that the
-    // incidence loop keeps each lane busy.
+    // contact, meshes past the cluster step).  One mesh, by the solves n of a colour: below 1,000 a
+    // vertex's chain is what counts (32 lanes), then blocks that leave room for the next colour's while
+    // the GPU fills (8), at last work per vertex (4).  With blocks of 128 (the default for one mesh), us
+    // per 20-iteration step alone / in turn with two others: n = 1,455: 32 lanes 347 / 141, 8 lanes 317 /
+    // 132; n = 4,356: 32 lanes 473 / 313, 8 lanes 378 / 183, 4 lanes 389 / 223; n = 8,400: 8 lanes 462 /
+    // 222, 4 lanes 464 / 298; n = 18,260: 8 lanes 580 / 506, 4 lanes 791 / 400; n = 33,600 (Chebyshev):
+    // 8 lanes 1,400 / 1,234, 4 lanes 1,135 / 919, with blocks of 256 1,145 / 967.  A batch's persistent
+    // kernel takes 4 lanes and blocks of 256 (40 cubes of 12^3 to 30^3, Chebyshev: 1.09 ms, blocks of 128
+    // 1.92 ms; 8 lanes 11.2 ms).
     int launchLanes() const
     {
         if (lanes > 0)
             return lanes;
         int const perColor = nColors > 0 ? nFree / nColors : nFree;
-        return perColor < 4096 ? 32 : 4;
+        if (nMeshes > 1)
+            return perColor < 4096 ? 32 : 4;
+        return perColor < 1000 ? 32 : (perColor < 12000 ? 8 : 4);
     }
 
     // Lanes per vertex of the cluster step by default, from the solve entries n of the part's largest
@@ -1179,6 +1188,7 @@ class VbdSystem
             }
         }
         this->nMeshes = nMeshes;
+        block         = nMeshes == 1 ? 128 : 256; // launchLanes
         meshV0.assign(size_t(nMeshes) + 1, 0);
         for (int32_t b = 0; b < nMeshes; ++b)
             meshV0[b + 1] = meshV0[b] + descs[b].n_vertices;
