@@ -52,10 +52,14 @@ __device__ bool wait_for(BatchedStepParams const& p, int32_t const* counter, int
     return false;
 }
 
+// Bound by memory: DRAM for batches larger than L2 (20 B per pair of incidences, 8 B per neighbour, the
+// positions that leave L2 between two colours of a mesh).  64 cubes of 6^3 to 32^3, 20 iterations: 3.05
+// ms with 24 B per incidence, 2.75 ms with 12 B, 2.37 ms with pairs and 2 lanes.
+//
 // Colour sweep of solve entries [begin, end) by the whole block: sub-tiles of blockDim / L vertices,
 // each staged and solved like staged_sweep_kernel (the same arithmetic in the same order), with the
-// block's positions read through L2.  The incidence loop keeps two incidences' records in flight
-// (this one's and the next two's loads overlap its arithmetic): the batch's incidence records
+// block's positions read through L2.  The pair loop keeps two pairs' records in flight
+// (this one's and the next two's loads overlap its arithmetic): the batch's records
 // stream from DRAM, and one record ahead per lane left too few bytes in flight per SM.  (Loading
 // the records evict-first, ld.global.cs, doubled the DRAM reads of a 256-mesh step: a record's
 // sector left L2 before the neighbouring lanes had read their parts of it.)
@@ -75,24 +79,24 @@ __device__ __forceinline__ void sweep_tile(SweepParams const& p, int begin, int 
         float xi[3] = {0.f, 0.f, 0.f};
         int k = 0, k1 = 0, n0 = 0, n1 = 0, base = 0;
         uint32_t q0 = 0u, q1 = 0u;
-        float2 mt0 = make_float2(0.f, 0.f), mt1 = mt0;
+        float4 mt0 = make_float4(0.f, 0.f, 0.f, 0.f), mt1 = mt0;
         if (valid)
         {
             i    = __ldg(p.solve + s);
             n0   = __ldg(p.nbrPtr + s);
             n1   = __ldg(p.nbrPtr + s + 1);
             base = n0 - nb0;
-            k1   = __ldg(p.incPtr + s + 1);
-            k    = __ldg(p.incPtr + s) + lane;
+            k1   = __ldg(p.pairPtr + s + 1);
+            k    = __ldg(p.pairPtr + s) + lane;
             if (k < k1)
             {
-                q0  = __ldg(p.incSlots + k);
-                mt0 = __ldg(p.incMat + k);
+                q0  = __ldg(p.pairSlots + k);
+                mt0 = __ldg(p.pairMat + k);
             }
             if (k + L < k1)
             {
-                q1  = __ldg(p.incSlots + k + L);
-                mt1 = __ldg(p.incMat + k + L);
+                q1  = __ldg(p.pairSlots + k + L);
+                mt1 = __ldg(p.pairMat + k + L);
             }
             load3(Mem<true>::ld((CHEB ? p.hprev : p.x) + i), xi);
             for (int j = n0 + lane; j < n1; j += L)
@@ -110,13 +114,13 @@ __device__ __forceinline__ void sweep_tile(SweepParams const& p, int begin, int 
             for (; k < k1; k += L)
             {
                 uint32_t q2 = 0u;
-                float2 mt2  = make_float2(0.f, 0.f);
+                float4 mt2  = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (k + 2 * L < k1)
                 {
-                    q2  = __ldg(p.incSlots + k + 2 * L);
-                    mt2 = __ldg(p.incMat + k + 2 * L);
+                    q2  = __ldg(p.pairSlots + k + 2 * L);
+                    mt2 = __ldg(p.pairMat + k + 2 * L);
                 }
-                staged_incidence(b, slab + base, q0, mt0);
+                staged_pair(b, slab + base, q0, mt0);
                 q0  = q1;
                 mt0 = mt1;
                 q1  = q2;
@@ -239,7 +243,7 @@ cudaError_t launch_batched_step(BatchedStepParams const& p, int lanes, int block
     if (p.nItems <= 0)
         return cudaSuccess;
     if (grid < 1 || block < 32 || block > 256 || block % lanes != 0 || smem > kStagedMaxBytes || !p.items ||
-        !p.control || !p.done || !p.flags || !p.sweep.incMat || !p.sweep.incSlots || !p.sweep.nbrPtr || (chebyshev && (!p.H0 || !p.H1 || !p.omega)))
+        !p.control || !p.done || !p.flags || !p.sweep.pairMat || !p.sweep.pairSlots || !p.sweep.nbrPtr || (chebyshev && (!p.H0 || !p.H1 || !p.omega)))
         return cudaErrorInvalidValue;
     return chebyshev ? launch_c<true>(p, lanes, block, grid, smem, s) : launch_c<false>(p, lanes, block, grid, smem, s);
 }

@@ -93,10 +93,9 @@ __device__ __forceinline__ void barrier_wait(uint64_t* bar, uint32_t parity, int
 template <int L, bool CHEB, bool REC, bool CLUSTER>
 __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_kernel(ClusterStepParams p)
 {
-    // Neighbours and incidences a lane has in flight at once: a block holds few warps, so a lane's own
-    // independent loads hide the latency of shared memory and of the arithmetic.
-    constexpr int kNbrs = L >= 32 ? 1 : (L >= 16 ? 1 : (L >= 8 ? 2 : 4));
-    constexpr int kIncs = L >= 32 ? 1 : (L >= 8 ? 2 : 2);
+    // Neighbours a lane has in flight at once: a block holds few warps, so a lane's own independent
+    // loads hide the latency of shared memory.
+    constexpr int kNbrs = L >= 16 ? 1 : (L >= 8 ? 2 : 4);
     extern __shared__ __align__(128) unsigned char shared[];
     __shared__ int32_t sGaveUp;
     int32_t volatile* const gaveUp = &sGaveUp;
@@ -313,31 +312,11 @@ __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_k
                     __syncwarp();
                     if (valid)
                     {
-                        float2 const* const mat     = reinterpret_cast<float2 const*>(base) + (e0.w & 0xFFFF);
+                        float4 const* const mat     = reinterpret_cast<float4 const*>(base) + (e0.w & 0xFFFF);
                         uint32_t const* const slots = reinterpret_cast<uint32_t const*>(base) + (e1.y & 0xFFFF);
-                        int const nInc              = int(uint32_t(e0.w) >> 16);
-                        for (int j = lane; j < nInc; j += kIncs * L)
-                        {
-                            float2 m[kIncs];
-                            float d[kIncs][3][3];
-#pragma unroll
-                            for (int u = 0; u < kIncs; ++u)
-                            {
-                                // Past the end: the turn's first incidence with zero constants, which
-                                // adds zeros.
-                                int const ju     = j + u * L < nInc ? j + u * L : j;
-                                uint32_t const q = slots[ju];
-                                m[u]             = mat[ju];
-                                if (u > 0 && j + u * L >= nInc)
-                                    m[u] = make_float2(0.f, 0.f);
-#pragma unroll
-                                for (int c3 = 0; c3 < 3; ++c3)
-                                    load3(slice[(q >> (8 * c3)) & 0xFFu], d[u][c3]);
-                            }
-#pragma unroll
-                            for (int u = 0; u < kIncs; ++u)
-                                accumulate_incidence(b, d[u], m[u].y, m[u].x);
-                        }
+                        int const nPair             = int(uint32_t(e0.w) >> 16);
+                        for (int j = lane; j < nPair; j += L)
+                            staged_pair(b, slice, slots[j], mat[j]);
                     }
                     reduce_lanes<L>(b);
                     if (valid && lane == 0)

@@ -21,13 +21,13 @@
 // of the next iteration are sent only after the block has passed this iteration's wait.
 //
 // What bounds it: with a few solves per part and colour, the chain of one vertex solve (about 300
-// instructions of one warp, 0.8 us) times the colours; with many, shared memory (three 16-byte reads per
+// instructions of one warp, 0.8 us) times the colours; with many, shared memory (with three 16-byte reads per
 // incidence: L1 at 68 % with 272 vertices per block and colour, issue at 44 %).  A first version with a
 // cluster barrier per colour and tables read from global memory took 1.6 us per colour where this one
 // takes 1.1: the barrier's acquire empties L1, so that every table read after it went to L2.
 // 20 iterations without acceleration, colour launches -> one cluster: 27 vertices 113 -> 62 us, 1331
-// vertices 285 -> 170 us, 4913 vertices 290 -> 244 us; 48 meshes of 27 to 512 vertices 795 (persistent
-// tickets) -> 195 us.
+// vertices 285 -> 169 us, 4913 vertices 290 -> 220 us (244 with three edge vectors read per incidence
+// instead of four per pair); 48 meshes of 27 to 512 vertices 795 (persistent tickets) -> 187 us.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -39,14 +39,14 @@ namespace pbgb {
 
 // One solved vertex of a tile.  A tile is kClusterTileVertices entries (unused ones have vertex -1),
 // then, each array from a 16-byte boundary, the neighbours (slot, bit 31: lower colour; K as bits), the
-// incidences (kappa, sigma), the incidences' slot words and the copies of the vertices' positions in
-// other blocks (rank << 16 | slot there).  Offsets count from the tile's start.
+// pairs of incidences (kappa, sigma of each), the pairs' slot words and the copies of the vertices'
+// positions in other blocks (rank << 16 | slot there).  Offsets count from the tile's start.
 struct __align__(16) ClusterEntry
 {
     int32_t vertex;
     int32_t solve; // solve-list entry (the tape's order)
     uint32_t nbr;  // offset in 8-byte units | count << 16
-    uint32_t inc;  // offset in 8-byte units | count << 16
+    uint32_t pair; // offset in 16-byte units | count << 16
     uint32_t slot; // slot among the part's local vertices | copies << 16
     uint32_t words; // slot words, copies: offsets in 4-byte units, the second << 16
     float diag;     // SweepParams::diag

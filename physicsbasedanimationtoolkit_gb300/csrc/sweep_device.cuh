@@ -56,15 +56,15 @@ __device__ __forceinline__ void stage_neighbour(VertexBlock<float>& b, float4* s
     accumulate_neighbour(b, d, K);
 }
 
-// One incidence of a staged solve: the edge vectors of its other corners are slab slots q (bytes 0-2)
-// of the vertex's slice.
-__device__ __forceinline__ void staged_incidence(VertexBlock<float>& b, float4 const* slice, uint32_t q, float2 const& mat)
+// One pair of incidences of a staged solve: A, B, C, D are slab slots q (bytes 0-3) of the vertex's
+// slice.
+__device__ __forceinline__ void staged_pair(VertexBlock<float>& b, float4 const* slice, uint32_t q, float4 const& mat)
 {
-    float d[3][3];
+    float d[4][3];
 #pragma unroll
-    for (int m = 0; m < 3; ++m)
+    for (int m = 0; m < 4; ++m)
         load3(slice[(q >> (8 * m)) & 0xFFu], d[m]);
-    accumulate_incidence(b, d, mat.y, mat.x);
+    accumulate_pair(b, d[0], d[1], d[2], d[3], mat.x, mat.y, mat.z, mat.w);
 }
 
 // Contact terms of one vertex-triangle pair (gpu/impl/vbd/Kernels.cuh:80-114,203-223): the

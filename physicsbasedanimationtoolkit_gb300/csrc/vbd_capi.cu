@@ -26,6 +26,8 @@
 #include <cstdio>
 #include <cstring>
 #include <functional>
+#include <future>
+#include <thread>
 #include <exception>
 #include <memory>
 #include <mutex>
@@ -216,6 +218,164 @@ inline void validate_descs(pbgb_vbd_desc const* descs, int32_t nMeshes)
         bad("system too large for 32-bit indexing");
 }
 
+// One incidence of a solved vertex: its word (tet << 2 | local) and the slots of the other corners in the
+// vertex's neighbour list, in the order (local + 1 + m) & 3.
+struct LinkTriangle
+{
+    uint32_t inc;
+    int32_t slot[3];
+};
+
+// Pairs of incidences of every solve entry (SweepParams).
+struct PairTables
+{
+    std::vector<int32_t> ptr;
+    std::vector<uint2> inc;
+    std::vector<uint32_t> slots;
+    std::vector<uint8_t> sign;
+
+    void reserve(size_t n)
+    {
+        inc.reserve(n);
+        slots.reserve(n);
+        sign.reserve(n);
+    }
+    void add(LinkTriangle const& t, int A, int B, int C, bool flip, LinkTriangle const* u, int D, bool flipU)
+    {
+        inc.push_back(make_uint2(t.inc, u ? u->inc : t.inc));
+        slots.push_back(uint32_t(A & 0xFF) | uint32_t(B & 0xFF) << 8 | uint32_t(C & 0xFF) << 16 | uint32_t(D & 0xFF) << 24);
+        sign.push_back(uint8_t((flip ? 1 : 0) | (flipU ? 2 : 0) | (u ? 0 : 4)));
+    }
+    // Every incidence by itself.
+    void split(std::vector<int32_t> const& incPtr, std::vector<uint32_t> const& words)
+    {
+        ptr = incPtr;
+        inc.clear();
+        for (uint32_t q : words)
+            inc.push_back(make_uint2(q, q));
+        slots.assign(words.size(), 0u);
+        sign.assign(words.size(), uint8_t(4));
+    }
+};
+
+// Pairs the incidences of one vertex that share a face with it, i.e. the triangles of its link that share
+// an edge: greedily, a triangle with the fewest free neighbours among an unpaired one's first, then one
+// round of exchanges along paths of three.  What stays single is a pair with no second.
+class PairMatcher
+{
+  public:
+    void pair(std::vector<LinkTriangle> const& link, size_t nNbr, PairTables& out)
+    {
+        size_t const n = link.size();
+        next_.resize(3 * n);
+        mate_.assign(n, -1);
+        if (nNbr > 256)
+            std::fill(next_.begin(), next_.end(), -1);
+        else
+        {
+            // Edge (a, b) of a triangle -> the triangle: neighbours run along it the other way.
+            if (edge_.size() < nNbr * nNbr)
+                edge_.assign(nNbr * nNbr, Edge{-1, -1});
+            ++stamp_;
+            for (size_t t = 0; t < n; ++t)
+            {
+                int32_t const c[3] = {cyclic(link[t], 0), cyclic(link[t], 1), cyclic(link[t], 2)};
+                for (int m = 0; m < 3; ++m)
+                    edge_[size_t(c[m]) * nNbr + size_t(c[(m + 1) % 3])] = Edge{stamp_, int32_t(t)};
+            }
+            for (size_t t = 0; t < n; ++t)
+            {
+                int32_t const c[3] = {cyclic(link[t], 0), cyclic(link[t], 1), cyclic(link[t], 2)};
+                for (int m = 0; m < 3; ++m)
+                {
+                    Edge const e     = edge_[size_t(c[(m + 1) % 3]) * nNbr + size_t(c[m])];
+                    next_[3 * t + m] = e.stamp == stamp_ && !has(link[size_t(e.triangle)], c[(m + 2) % 3]) ? e.triangle : -1;
+                }
+            }
+        }
+        for (size_t t = 0; t < n; ++t)
+            if (mate_[t] < 0)
+            {
+                int32_t best = -1, bestFree = 4;
+                for (int m = 0; m < 3; ++m)
+                {
+                    int32_t const u = next_[3 * t + m];
+                    if (u < 0 || mate_[u] >= 0)
+                        continue;
+                    int32_t const f = freeNeighbours(u);
+                    if (f < bestFree)
+                        best = u, bestFree = f;
+                }
+                if (best >= 0)
+                    join(int32_t(t), best);
+            }
+        for (size_t t = 0; t < n; ++t)
+            for (int m = 0; m < 3 && mate_[t] < 0; ++m)
+            {
+                int32_t const u = next_[3 * t + m];
+                if (u < 0)
+                    continue;
+                int32_t const w = mate_[u];
+                for (int k = 0; k < 3 && w >= 0 && mate_[t] < 0; ++k)
+                {
+                    int32_t const x = next_[3 * size_t(w) + k];
+                    if (x >= 0 && x != int32_t(t) && mate_[x] < 0)
+                    {
+                        join(int32_t(t), u);
+                        join(w, x);
+                    }
+                }
+            }
+        for (size_t t = 0; t < n; ++t)
+        {
+            LinkTriangle const& a = link[t];
+            if (mate_[t] < 0)
+                out.add(a, a.slot[0], a.slot[1], a.slot[2], false, nullptr, a.slot[2], false);
+            else if (mate_[t] > int32_t(t))
+            {
+                LinkTriangle const& b = link[size_t(mate_[t])];
+                // A, C: the shared corners; B, D: the others.  The parity of (A, B, C) and (A, C, D)
+                // against the triangles' own orders gives the signs of kappa.
+                int ia = 0, ib = 0; // index of the corner not shared
+                while (has(b, a.slot[ia]))
+                    ++ia;
+                while (has(a, b.slot[ib]))
+                    ++ib;
+                int const B = a.slot[ia], C = a.slot[(ia + 1) % 3], A = a.slot[(ia + 2) % 3]; // (A, B, C) is cyclic in a
+                int const D = b.slot[ib];
+                // (A, C, D) against b's order: cyclic when C follows A there.
+                int const j   = b.slot[0] == A ? 0 : (b.slot[1] == A ? 1 : 2);
+                bool const odd = b.slot[(j + 1) % 3] != C;
+                out.add(a, A, B, C, false, &b, D, odd);
+            }
+        }
+    }
+
+  private:
+    struct Edge
+    {
+        int32_t stamp, triangle;
+    };
+    // Corner m of the triangle in an order that is the same way round for all tets of one orientation.
+    static int32_t cyclic(LinkTriangle const& t, int m) { return t.inc & 1u ? t.slot[(5 - m) % 3] : t.slot[m % 3]; }
+    static bool has(LinkTriangle const& t, int32_t s) { return t.slot[0] == s || t.slot[1] == s || t.slot[2] == s; }
+    int32_t freeNeighbours(int32_t t) const
+    {
+        int32_t f = 0;
+        for (int m = 0; m < 3; ++m)
+            f += next_[3 * size_t(t) + m] >= 0 && mate_[next_[3 * size_t(t) + m]] < 0 ? 1 : 0;
+        return f;
+    }
+    void join(int32_t a, int32_t b)
+    {
+        mate_[a] = b;
+        mate_[b] = a;
+    }
+    std::vector<int32_t> next_, mate_;
+    std::vector<Edge> edge_;
+    int32_t stamp_ = 0;
+};
+
 class VbdSystem
 {
   public:
@@ -258,8 +418,9 @@ class VbdSystem
     DeviceArray<int32_t> solve, incPtr, flags;
     DeviceArray<uint32_t> inc;
     // Distinct neighbours of every free vertex (solve order), and the rest-state constants of the
-    // solves (SweepParams): incMat and incSlots per incidence, nbr (index, K) per neighbour, diag per
-    // entry; formed on the device from the tets' geometry and Lame coefficients (FP64), at creation and
+    // solves (SweepParams): pairMat, pairSlots, pairInc (and pairSign for the set-up) per pair of
+    // incidences, nbr (index, K) per neighbour, diag per entry; the constants are formed on the device
+    // from the tets' geometry and Lame coefficients (FP64), at creation and
     // by pbgb_vbd_set_material.  stagedOk is false when some vertex has more than 256
     // neighbours (slots are bytes); `staged` is the user's choice.
     bool stagedOk = false, staged = true;
@@ -268,8 +429,11 @@ class VbdSystem
     DeviceArray<double> dMu, dLambda;
     DeviceArray<int32_t> nbrPtr;
     DeviceArray<uint2> nbr;
-    DeviceArray<float2> incMat;
-    DeviceArray<uint32_t> incSlots;
+    DeviceArray<int32_t> pairPtr;
+    DeviceArray<float4> pairMat;
+    DeviceArray<uint32_t> pairSlots;
+    DeviceArray<uint2> pairInc;
+    DeviceArray<uint8_t> pairSign;
     DeviceArray<float> diag;
     DeviceArray<double> red, gradBuf, objPartials;
 
@@ -484,11 +648,11 @@ class VbdSystem
     {
         w.tets     = tets.get();
         w.solve    = solve.get();
-        w.incPtr   = incPtr.get();
-        w.inc      = inc.get();
-        w.incMat   = incMat.get();
-        w.incSlots = incSlots.get();
-        w.diag     = diag.get();
+        w.pairPtr   = pairPtr.get();
+        w.pairMat   = pairMat.get();
+        w.pairSlots = stagedOk ? pairSlots.get() : nullptr;
+        w.pairInc   = pairInc.get();
+        w.diag      = diag.get();
         w.nbrPtr   = nbrPtr.get();
         w.nbr      = nbr.get();
     }
@@ -514,34 +678,36 @@ class VbdSystem
     // contact, meshes past the cluster step).  One mesh, by the solves n of a colour: below 1,000 a
     // vertex's chain is what counts (32 lanes), then blocks that leave room for the next colour's while
     // the GPU fills (8), at last work per vertex (4).  With blocks of 128 (the default for one mesh), us
-    // per 20-iteration step alone / in turn with two others: n = 1,455: 32 lanes 347 / 141, 8 lanes 317 /
-    // 132; n = 4,356: 32 lanes 473 / 313, 8 lanes 378 / 183, 4 lanes 389 / 223; n = 8,400: 8 lanes 462 /
-    // 222, 4 lanes 464 / 298; n = 18,260: 8 lanes 580 / 506, 4 lanes 791 / 400; n = 33,600 (Chebyshev):
-    // 8 lanes 1,400 / 1,234, 4 lanes 1,135 / 919, with blocks of 256 1,145 / 967.  A batch's persistent
-    // kernel takes 4 lanes and blocks of 256 (40 cubes of 12^3 to 30^3, Chebyshev: 1.09 ms, blocks of 128
-    // 1.92 ms; 8 lanes 11.2 ms).
+    // per 20-iteration step alone / in turn with two others: n = 578: 32 lanes 281, 8 lanes 285, 4 lanes
+    // 327 (alone); n = 2,369: 32 lanes 450 / 179, 8 lanes 300 / 137, 4 lanes 329 / 137; n = 8,400: 8 lanes
+    // 472 / 205, 4 lanes 421 / 255; n = 18,260: 8 lanes 641 / 456, 4 lanes 681 / 308; n = 33,600
+    // (Chebyshev): 8 lanes 1,296 / 1,149, 4 lanes 944 / 744, 2 lanes 1,212 / 732; blocks of 256 with 4
+    // lanes were 1 to 25 % slower.  Contact steps: 4 lanes at any size (9 cubes of 11^3, 30 iterations:
+    // 1,041 / 393, 8 lanes 1,075 / 425, 32 lanes 1,361 / 505; 4 cubes of 6^3, 20 iterations: 691 / 246, 32
+    // lanes 712 / 250).  A batch's persistent kernel takes blocks of 256 and 4 lanes, or 2 when its colours
+    // are large enough that only throughput counts (40 cubes of 12^3 to 30^3, Chebyshev, n = 59,000:
+    // 4 lanes 1.02 ms, 2 lanes 1.17 ms, blocks of 128 1.41 ms; 64 cubes of 6^3 to 32^3, n = 87,000: 2 lanes
+    // 2.32 ms, 4 lanes 2.58 ms, blocks of 128 4.2 ms).
     int launchLanes() const
     {
         if (lanes > 0)
             return lanes;
         int const perColor = nColors > 0 ? nFree / nColors : nFree;
         if (nMeshes > 1)
-            return perColor < 4096 ? 32 : 4;
+            return perColor < 4096 ? 32 : (perColor < 70000 ? 4 : 2);
+        if (contact)
+            return 4;
         return perColor < 1000 ? 32 : (perColor < 12000 ? 8 : 4);
     }
 
     // Lanes per vertex of the cluster step by default, from the solve entries n of the part's largest
-    // colour: with n L <= 320 each warp has one group of vertices at a time and the block up to 10 warps
-    // of work; fewer lanes make each vertex's chain longer, more a second round.  Measured (us per
-    // 20-iteration step): n = 10: 16 lanes 170, 8 lanes 179, 32 lanes 195; n = 25: 8 lanes 200, 4 lanes
-    // 206, 16 lanes 208; n = 69: 4 lanes 322, 2 lanes 343, 8 lanes 458; n = 148: 2 lanes 530, 4 lanes
-    // 656, 1 lane 769.
+    // colour: each warp has one group of vertices at a time and the block up to 12 warps of work; fewer
+    // lanes make each vertex's chain longer, more a second round.  Measured (us per 20-iteration step):
+    // n = 10: 16 lanes 169, 8 lanes 179, 32 lanes 203; n = 25: 8 lanes 193, 4 lanes 195, 16 lanes 198; n
+    // = 40: 4 lanes 220, 8 lanes 226, 16 lanes 335; n = 81: 4 lanes 287, 2 lanes 312, 8 lanes 433.
     int clusterDefaultLanes() const
     {
-        int L = 16;
-        while (L > 2 && clusterColor * L > 320)
-            L /= 2;
-        return L;
+        return clusterColor <= 20 ? 16 : (clusterColor <= 36 ? 8 : (clusterColor <= 96 ? 4 : 2));
     }
 
     // Splits mesh vertices into `parts` spatially compact parts with equal numbers of solved vertices
@@ -690,7 +856,7 @@ class VbdSystem
     // The cluster step's tables from the parts (solve order already grouped by part inside a colour).
     // False when a tile is too large for its entries' 16-bit fields.
     bool buildCluster(std::vector<int32_t> const& part, std::vector<int32_t> const& color, std::vector<int32_t> const& solveList,
-                      std::vector<int32_t> const& incPtrH, std::vector<uint32_t> const& slotsH, std::vector<uint2> const& nbrH)
+                      PairTables const& pairs, std::vector<uint2> const& nbrH)
     {
         int32_t const P = clusterBlocks, parts = nMeshes * P;
         // Larger meshes first: their clusters start first.
@@ -800,11 +966,11 @@ class VbdSystem
                 for (int32_t f = r.x; f < r.y; f += kClusterTileVertices)
                 {
                     int32_t const e    = std::min(f + kClusterTileVertices, r.y);
-                    int64_t const nNbr = hostNbrPtr[e] - hostNbrPtr[f], nInc = incPtrH[e] - incPtrH[f];
+                    int64_t const nNbr = hostNbrPtr[e] - hostNbrPtr[f], nPair = pairs.ptr[e] - pairs.ptr[f];
                     size_t const size = kClusterTileVertices * sizeof(ClusterEntry) + size_t(even(nNbr)) * sizeof(uint2) +
-                                        size_t(even(nInc)) * sizeof(float2) +
-                                        (size_t(nInc + sendPtr[e] - sendPtr[f]) * sizeof(uint32_t) + 15) / 16 * 16;
-                    if (size > kClusterMaxTile || nInc > 0xFFFF)
+                                        size_t(nPair) * sizeof(float4) +
+                                        (size_t(nPair + sendPtr[e] - sendPtr[f]) * sizeof(uint32_t) + 15) / 16 * 16;
+                    if (size > kClusterMaxTile || nPair > 0xFFFF)
                         return false;
                     hTile.push_back(make_int2(int32_t(bytes / 16), int32_t(size)));
                     tileFirst.push_back(f);
@@ -828,30 +994,30 @@ class VbdSystem
             while (e < nFree && e - f < kClusterTileVertices && part[solveList[e]] == part[solveList[f]] &&
                    color[solveList[e]] == color[solveList[f]] && meshOf(solveList[e]) == meshOf(solveList[f]))
                 ++e;
-            int32_t const nNbr = hostNbrPtr[e] - hostNbrPtr[f], nInc = incPtrH[e] - incPtrH[f];
+            int32_t const nNbr = hostNbrPtr[e] - hostNbrPtr[f], nPair = pairs.ptr[e] - pairs.ptr[f];
             size_t const nbrs  = kClusterTileVertices * sizeof(ClusterEntry);
-            size_t const mats = nbrs + size_t(even(nNbr)) * sizeof(uint2), slots = mats + size_t(even(nInc)) * sizeof(float2);
-            size_t const copies = slots + size_t(nInc) * sizeof(uint32_t);
+            size_t const mats = nbrs + size_t(even(nNbr)) * sizeof(uint2), slots = mats + size_t(nPair) * sizeof(float4);
+            size_t const copies = slots + size_t(nPair) * sizeof(uint32_t);
             for (int32_t s = f; s < f + kClusterTileVertices; ++s)
             {
                 ClusterEntry en{};
                 en.vertex = -1;
                 if (s < e)
                 {
-                    size_t const n0 = nbrs / 8 + size_t(hostNbrPtr[s] - hostNbrPtr[f]), i0 = size_t(incPtrH[s] - incPtrH[f]);
+                    size_t const n0 = nbrs / 8 + size_t(hostNbrPtr[s] - hostNbrPtr[f]), i0 = size_t(pairs.ptr[s] - pairs.ptr[f]);
                     en.vertex = solveList[s];
                     en.solve  = s;
                     en.nbr    = uint32_t(n0) | uint32_t(hostNbrPtr[s + 1] - hostNbrPtr[s]) << 16;
-                    en.inc    = uint32_t(mats / 8 + i0) | uint32_t(incPtrH[s + 1] - incPtrH[s]) << 16;
+                    en.pair   = uint32_t(mats / 16 + i0) | uint32_t(pairs.ptr[s + 1] - pairs.ptr[s]) << 16;
                     en.slot   = uint32_t(ownSlot[solveList[s]]) | uint32_t(sendPtr[s + 1] - sendPtr[s]) << 16;
                     en.words  = uint32_t(slots / 4 + i0) | uint32_t(copies / 4 + size_t(sendPtr[s] - sendPtr[f])) << 16;
-                    hAt[s] = make_int4(int32_t(at / 16 + 2 * size_t(s - f)), int32_t(at / 8 + n0), int32_t((at + mats) / 8 + i0), 0);
+                    hAt[s] = make_int4(int32_t(at / 16 + 2 * size_t(s - f)), int32_t(at / 8 + n0), int32_t((at + mats) / 16 + i0), 0);
                 }
                 std::memcpy(hData.data() + at + size_t(s - f) * sizeof(en), &en, sizeof(en));
             }
             for (int32_t j = hostNbrPtr[f]; j < hostNbrPtr[e]; ++j)
                 std::memcpy(hData.data() + at + nbrs + size_t(j - hostNbrPtr[f]) * sizeof(uint2), &nbrSlot[j], sizeof(uint32_t));
-            std::memcpy(hData.data() + at + slots, slotsH.data() + incPtrH[f], size_t(nInc) * sizeof(uint32_t));
+            std::memcpy(hData.data() + at + slots, pairs.slots.data() + pairs.ptr[f], size_t(nPair) * sizeof(uint32_t));
             std::memcpy(hData.data() + at + copies, hSend.data() + sendPtr[f], size_t(sendPtr[e] - sendPtr[f]) * sizeof(uint32_t));
         }
         std::vector<int32_t> hPtr(size_t(parts) + 1, 0);
@@ -1235,19 +1401,28 @@ class VbdSystem
         }
         meanDegree = nFree > 0 ? double(degSum) / nFree : 0.0;
 
-        // Neighbour lists, in first-use order over the vertex's incidences and
-        // corners ((local + 1 + m) & 3, the order the sweep visits them).
-        std::vector<uint2> hNbr;
-        hNbr.reserve(hInc.size());
-        std::vector<uint32_t> hSlots(hInc.size(), 0u);
-        hostNbrPtr.assign(size_t(nFree) + 1, 0);
-        stagedOk = true;
+        // Neighbour lists, in first-use order over the vertex's incidences and corners ((local + 1 + m) &
+        // 3), and the pairs of incidences: ranges of the solve list on several host threads, joined in
+        // order.
+        struct Range
         {
+            PairTables pairs;
+            std::vector<uint2> nbr;
+            std::vector<int32_t> nbrPtr;
+            bool wide = false; // a vertex with more than 256 neighbours
+        };
+        auto lists = [&](int32_t begin, int32_t end) {
+            Range r;
+            r.pairs.reserve(size_t(hIncPtr[end] - hIncPtr[begin]) / 2 + size_t(end - begin));
+            r.nbr.reserve(size_t(hIncPtr[end] - hIncPtr[begin]));
             std::vector<uint32_t> list;
+            std::vector<LinkTriangle> link;
+            PairMatcher matcher;
             std::vector<int32_t> seen(size_t(nV), -1), where(size_t(nV), 0); // last entry that lists v, its slot there
-            for (int32_t s = 0; s < nFree; ++s)
+            for (int32_t s = begin; s < end; ++s)
             {
                 list.clear();
+                link.clear();
                 for (int32_t k = hIncPtr[s]; k < hIncPtr[s + 1]; ++k)
                 {
                     uint32_t const q  = hInc[k];
@@ -1255,7 +1430,7 @@ class VbdSystem
                     int const il      = int(q & 3u);
                     uint32_t const c4[4] = {t.x, t.y, t.z, t.w};
                     uint32_t const own = c4[il] >> 30;
-                    uint32_t slots     = 0;
+                    LinkTriangle tri{q, {0, 0, 0}};
                     for (int m = 0; m < 3; ++m)
                     {
                         uint32_t const ca = c4[(il + 1 + m) & 3];
@@ -1266,16 +1441,44 @@ class VbdSystem
                             where[v] = int32_t(list.size());
                             list.push_back(v | ((ca >> 30) < own ? 0x80000000u : 0u));
                         }
-                        slots |= uint32_t(where[v]) << (8 * m);
+                        tri.slot[m] = where[v];
                     }
-                    hSlots[k] = slots; // meaningful only while the list has at most 256 entries
+                    link.push_back(tri);
                 }
-                if (list.size() > 256)
-                    stagedOk = false;
+                matcher.pair(link, list.size(), r.pairs);
+                r.pairs.ptr.push_back(int32_t(r.pairs.inc.size()));
+                r.wide = r.wide || list.size() > 256;
                 for (uint32_t a : list)
-                    hNbr.push_back(make_uint2(a, 0u));
-                hostNbrPtr[s + 1] = int32_t(hNbr.size());
+                    r.nbr.push_back(make_uint2(a, 0u));
+                r.nbrPtr.push_back(int32_t(r.nbr.size()));
             }
+            return r;
+        };
+        std::vector<uint2> hNbr;
+        PairTables pairs;
+        pairs.ptr.assign(1, 0);
+        hostNbrPtr.assign(1, 0);
+        stagedOk = true;
+        {
+            int32_t const ranges = std::clamp<int32_t>(nFree / 300, 1, std::clamp<int32_t>(int32_t(std::thread::hardware_concurrency()), 1, 8));
+            std::vector<std::future<Range>> rest;
+            for (int32_t k = 1; k < ranges; ++k)
+                rest.push_back(std::async(std::launch::async, lists, int32_t(int64_t(nFree) * k / ranges), int32_t(int64_t(nFree) * (k + 1) / ranges)));
+            auto join = [&](Range const& r) {
+                int32_t const p0 = int32_t(pairs.inc.size()), n0 = int32_t(hNbr.size());
+                for (int32_t p : r.pairs.ptr)
+                    pairs.ptr.push_back(p0 + p);
+                for (int32_t n : r.nbrPtr)
+                    hostNbrPtr.push_back(n0 + n);
+                pairs.inc.insert(pairs.inc.end(), r.pairs.inc.begin(), r.pairs.inc.end());
+                pairs.slots.insert(pairs.slots.end(), r.pairs.slots.begin(), r.pairs.slots.end());
+                pairs.sign.insert(pairs.sign.end(), r.pairs.sign.begin(), r.pairs.sign.end());
+                hNbr.insert(hNbr.end(), r.nbr.begin(), r.nbr.end());
+                stagedOk = stagedOk && !r.wide;
+            };
+            join(lists(0, int32_t(int64_t(nFree) / ranges)));
+            for (auto& f : rest)
+                join(f.get());
         }
         hostRecords = std::move(hrec);
 
@@ -1349,9 +1552,17 @@ class VbdSystem
         nbrPtr.upload(hostNbrPtr.data(), hostNbrPtr.size(), stream);
         nbr.allocate(hNbr.size());
         nbr.upload(hNbr.data(), hNbr.size(), stream);
-        incMat.allocate(hInc.size());
-        incSlots.allocate(hInc.size());
-        incSlots.upload(hSlots.data(), hInc.size(), stream);
+        if (!stagedOk)
+            pairs.split(hIncPtr, hInc); // slots do not fit bytes: each incidence by itself
+        pairPtr.allocate(pairs.ptr.size());
+        pairPtr.upload(pairs.ptr.data(), pairs.ptr.size(), stream);
+        pairMat.allocate(pairs.inc.size());
+        pairSlots.allocate(pairs.inc.size());
+        pairSlots.upload(pairs.slots.data(), pairs.inc.size(), stream);
+        pairInc.allocate(pairs.inc.size());
+        pairInc.upload(pairs.inc.data(), pairs.inc.size(), stream);
+        pairSign.allocate(pairs.inc.size());
+        pairSign.upload(pairs.sign.data(), pairs.inc.size(), stream);
         diag.allocate(size_t(nFree));
         std::vector<TetGeometry> hGeometry(static_cast<size_t>(nT));
         for (int32_t e = 0; e < nT; ++e)
@@ -1362,7 +1573,7 @@ class VbdSystem
         dLambda.allocate(size_t(nT));
         incPtr.upload(hIncPtr.data(), hIncPtr.size(), stream);
         inc.upload(hInc.data(), hInc.size(), stream);
-        if (!stagedOk || clusterBlocks == 0 || !buildCluster(part, color, hsolve, hIncPtr, hSlots, hNbr))
+        if (!stagedOk || clusterBlocks == 0 || !buildCluster(part, color, hsolve, pairs, hNbr))
             clusterBlocks = 0;
         uploadMaterial();
         if (stagedOk)
@@ -1504,7 +1715,10 @@ class VbdSystem
         p.incPtr   = incPtr.get();
         p.inc      = inc.get();
         p.nbrPtr   = nbrPtr.get();
-        p.incMat   = incMat.get();
+        p.pairPtr  = pairPtr.get();
+        p.pairInc  = pairInc.get();
+        p.pairSign = pairSign.get();
+        p.pairMat  = pairMat.get();
         p.nbr      = nbr.get();
         p.tileData = clusterBlocks > 0 ? tileData.get() : nullptr;
         p.tileAt   = tileAt.get();

@@ -16,8 +16,8 @@ namespace {
 // l takes incidences l, l+L, ...; the 10 accumulated floats are then reduced with xor shuffles
 // and lane 0 applies damping, inertia and the 3x3 Newton step, writing x in place.  Vertices of a
 // colour share no tet, so the in-place write races with no reader of this launch.  The vertex's
-// neighbours give its mu term (8 bytes each: index, K), then each incidence its volume term from
-// (kappa, sigma) and the three other corners' current positions: no rest position is read.
+// neighbours give its mu term (8 bytes each: index, K), then each pair of incidences its volume terms
+// from their (kappa, sigma) and the four other corners' current positions: no rest position is read.
 //
 // CHEB: the Chebyshev update of the reference (applied to all vertices after each full sweep,
 // sim/vbd/ChebyshevIntegrator.cpp:15-32) is fused in.  Only vertex i's own values enter its
@@ -41,27 +41,18 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) sweep_kernel(SweepParams
     int i       = 0;
     float xi[3] = {0.f, 0.f, 0.f};
     int k = 0, k1 = 0, n = 0, n1 = 0;
-    uint32_t q0 = 0u, q1 = 0u;
-    uint4 t     = make_uint4(0u, 0u, 0u, 0u);
-    float2 mt   = make_float2(0.f, 0.f);
+    float4 mt   = make_float4(0.f, 0.f, 0.f, 0.f);
     // Prologue on data no earlier launch writes (mesh tables): with programmatic dependent launch
     // it overlaps the previous colour's tail.
     if (valid)
     {
         i  = __ldg(p.solve + s);
-        n  = __ldg(p.nbrPtr + s) + lane;
+        n  = __ldg(p.nbrPtr + s);
         n1 = __ldg(p.nbrPtr + s + 1);
-        k1 = __ldg(p.incPtr + s + 1);
-        k  = __ldg(p.incPtr + s) + lane;
-        // Software pipeline: the records of incidence k+L and the incidence word of k+2L are in
-        // flight while incidence k's corners are gathered and its block accumulated.
-        q0 = k < k1 ? __ldg(p.inc + k) : 0u;
-        q1 = k + L < k1 ? __ldg(p.inc + k + L) : 0u;
+        k1 = __ldg(p.pairPtr + s + 1);
+        k  = __ldg(p.pairPtr + s) + lane;
         if (k < k1)
-        {
-            t  = __ldg(&p.tets[q0 >> 2].v);
-            mt = __ldg(p.incMat + k);
-        }
+            mt = __ldg(p.pairMat + k);
     }
     // Positions are written by the previous launches: wait for them (no-op without PDL), then let
     // the next colour's grid start its own prologue.
@@ -70,44 +61,46 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) sweep_kernel(SweepParams
     if (valid)
     {
         load3(CHEB ? p.hprev[i] : p.x[i], xi);
-        for (; n < n1; n += L)
+        // The edge vector to a vertex whose word has bit 31 set when it is read from x.
+        auto edge = [&](uint32_t word, float* d) {
+            float4 const xa = __ldg((CHEB && !(word >> 31) ? p.hprev : p.x) + (word & kIndexMask));
+            d[0]            = xa.x - xi[0];
+            d[1]            = xa.y - xi[1];
+            d[2]            = xa.z - xi[2];
+        };
+        for (int j = n + lane; j < n1; j += L)
         {
-            uint2 const a     = __ldg(p.nbr + n);
-            float4 const xa   = __ldg((CHEB && !(a.x >> 31) ? p.hprev : p.x) + (a.x & kIndexMask));
-            float const d[3]  = {xa.x - xi[0], xa.y - xi[1], xa.z - xi[2]};
+            uint2 const a = __ldg(p.nbr + j);
+            float d[3];
+            edge(a.x, d);
             accumulate_neighbour(b, d, __uint_as_float(a.y));
         }
         for (; k < k1; k += L)
         {
-            int const il = int(q0 & 3u);
-            uint4 tn     = make_uint4(0u, 0u, 0u, 0u);
-            float2 mtn   = make_float2(0.f, 0.f);
-            if (k + L < k1)
+            float4 const mn = k + L < k1 ? __ldg(p.pairMat + k + L) : make_float4(0.f, 0.f, 0.f, 0.f);
+            float d[4][3];
+            if (p.pairSlots)
             {
-                tn  = __ldg(&p.tets[q1 >> 2].v);
-                mtn = __ldg(p.incMat + k + L);
-            }
-            uint32_t const q2 = k + 2 * L < k1 ? __ldg(p.inc + k + 2 * L) : 0u;
-            uint32_t const own = corner(t, il) >> 30;
-            float d[3][3];
+                uint32_t const q = __ldg(p.pairSlots + k);
 #pragma unroll
-            for (int m = 0; m < 3; ++m)
-            {
-                uint32_t const ta = corner(t, (il + 1 + m) & 3);
-                uint32_t const j  = ta & kIndexMask;
-                float4 const* src = p.x;
-                if (CHEB && (ta >> 30) > own)
-                    src = p.hprev;
-                float4 const xa = __ldg(src + j);
-                d[m][0] = xa.x - xi[0];
-                d[m][1] = xa.y - xi[1];
-                d[m][2] = xa.z - xi[2];
+                for (int m = 0; m < 4; ++m)
+                    edge(__ldg(&p.nbr[n + int((q >> (8 * m)) & 0xFFu)].x), d[m]);
             }
-            accumulate_incidence(b, d, mt.y, mt.x);
-            q0 = q1;
-            q1 = q2;
-            t  = tn;
-            mt = mtn;
+            else
+            {
+                uint32_t const q   = __ldg(&p.pairInc[k].x);
+                uint4 const t      = __ldg(&p.tets[q >> 2].v);
+                uint32_t const own = corner(t, int(q & 3u)) >> 30;
+#pragma unroll
+                for (int m = 0; m < 3; ++m)
+                {
+                    uint32_t const ta = corner(t, int((q + 1u + m) & 3u));
+                    edge((ta & kIndexMask) | ((ta >> 30) < own ? 0x80000000u : 0u), d[m]);
+                }
+                d[3][0] = d[2][0], d[3][1] = d[2][1], d[3][2] = d[2][2];
+            }
+            accumulate_pair(b, d[0], d[1], d[2], d[3], mt.x, mt.y, mt.z, mt.w);
+            mt = mn;
         }
     }
     finish_vertex<L, CHEB, REC, CONTACT>(p, b, valid, lane, i, s, xi);
@@ -117,12 +110,13 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) sweep_kernel(SweepParams
 // tets reference only ~14 distinct neighbours, so instead of gathering three corners' positions
 // per incidence, the vertex's lanes load each neighbour's current position once, add its mu term and
 // put the edge vector to it into the vertex's slice of the block's slab (a float4 per neighbour), and
-// the incidence loop reads the edge vectors back through its three slot bytes.  The slab slice of solve
+// the loop over pairs of incidences reads the edge vectors back through its four slot bytes.  The slab slice of solve
 // entry s starts at nbrPtr[s] - nbrPtr[first entry of the block].  The lanes of a vertex share a
-// warp, so __syncwarp orders the staging.  What a solve reads of the rest state (8 B per neighbour, 12 B
-// per incidence) streams from L2 for every update and bounds a large mesh: with the mu terms kept per
-// incidence (24 B each, 4 B per neighbour) the 270,641-vertex beam took 2.76 ms per 50-iteration step,
-// now 2.36 ms.
+// warp, so __syncwarp orders the staging.  What a solve reads of the rest state (8 B per neighbour, 20 B
+// per pair of incidences) streams from L2 for every update and bounds a large mesh: with the mu terms
+// kept per incidence (24 B each, 4 B per neighbour) the 270,641-vertex beam took 2.76 ms per
+// 50-iteration step, with 12 B per incidence and three edge vectors read for
+// each 2.24 ms, now 1.85 ms.
 template <int L, bool CHEB, bool REC = false, bool CONTACT = false>
 __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) staged_sweep_kernel(SweepParams p)
 {
@@ -141,9 +135,9 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) staged_sweep_kernel(Swee
     float xi[3] = {0.f, 0.f, 0.f};
     int k = 0, k1 = 0, n0 = 0, n1 = 0, base = 0;
     uint32_t q0 = 0u, q1 = 0u;
-    float2 mt0 = make_float2(0.f, 0.f), mt1 = mt0;
+    float4 mt0 = make_float4(0.f, 0.f, 0.f, 0.f), mt1 = mt0;
     // The mesh tables are not written by any launch of the step: the vertex's first neighbour
-    // records and first two incidence records are loaded before griddepcontrol.wait, so that
+    // records and first two pairs are loaded before griddepcontrol.wait, so that
     // only the position loads remain on the path after it.
     int constexpr kPreNbr = 4;
     uint2 pre[kPreNbr];
@@ -156,21 +150,21 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) staged_sweep_kernel(Swee
         n0   = __ldg(p.nbrPtr + s);
         n1   = __ldg(p.nbrPtr + s + 1);
         base = n0 - nb0;
-        k1   = __ldg(p.incPtr + s + 1);
-        k    = __ldg(p.incPtr + s) + lane;
+        k1   = __ldg(p.pairPtr + s + 1);
+        k    = __ldg(p.pairPtr + s) + lane;
 #pragma unroll
         for (int m = 0; m < kPreNbr; ++m)
             if (n0 + lane + m * L < n1)
                 pre[m] = __ldg(p.nbr + n0 + lane + m * L);
         if (k < k1)
         {
-            q0  = __ldg(p.incSlots + k);
-            mt0 = __ldg(p.incMat + k);
+            q0  = __ldg(p.pairSlots + k);
+            mt0 = __ldg(p.pairMat + k);
         }
         if (k + L < k1)
         {
-            q1  = __ldg(p.incSlots + k + L);
-            mt1 = __ldg(p.incMat + k + L);
+            q1  = __ldg(p.pairSlots + k + L);
+            mt1 = __ldg(p.pairMat + k + L);
         }
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -202,17 +196,17 @@ __global__ void __launch_bounds__(256, CONTACT ? 2 : 4) staged_sweep_kernel(Swee
     __syncwarp();
     if (valid)
     {
-        // Two incidences' records in flight ahead of the one being accumulated.
+        // Two pairs' records in flight ahead of the one being accumulated.
         for (; k < k1; k += L)
         {
             uint32_t q2 = 0u;
-            float2 mt2  = make_float2(0.f, 0.f);
+            float4 mt2  = make_float4(0.f, 0.f, 0.f, 0.f);
             if (k + 2 * L < k1)
             {
-                q2  = __ldg(p.incSlots + k + 2 * L);
-                mt2 = __ldg(p.incMat + k + 2 * L);
+                q2  = __ldg(p.pairSlots + k + 2 * L);
+                mt2 = __ldg(p.pairMat + k + 2 * L);
             }
-            staged_incidence(b, slab + base, q0, mt0);
+            staged_pair(b, slab + base, q0, mt0);
             q0  = q1;
             mt0 = mt1;
             q1  = q2;
@@ -371,9 +365,9 @@ __global__ void tet_material_kernel(StiffnessParams p)
     p.tets[e].mat = make_float4(float(w * mu), float(w * la), float(1.0 + mu / la), 0.f);
 }
 
-// Rest-state constants of one solve entry per warp: lanes take the entry's incidences for
-// (kappa, sigma), then its neighbours, each lane adding the b of every incidence that holds its
-// neighbour (in incidence order).  pbgb_vbd_set_material with this kernel takes 0.09 ms for 24,000
+// Rest-state constants of one solve entry per warp: lanes take the entry's pairs of incidences, then its
+// neighbours, each lane adding the b of every incidence that holds its neighbour (in incidence order).
+// pbgb_vbd_set_material with this kernel takes 0.09 ms for 24,000
 // tets and 0.49 ms for 197,000 (most of it the host's checks and the upload of 16 B per tet); with the
 // records formed on the host and uploaded (24 B per incidence) it took 0.88 and 8.2 ms.
 __global__ void __launch_bounds__(256) stiffness_kernel(StiffnessParams p)
@@ -383,14 +377,23 @@ __global__ void __launch_bounds__(256) stiffness_kernel(StiffnessParams p)
     if (s >= p.nFree)
         return;
     int const k0 = p.incPtr[s], k1 = p.incPtr[s + 1], n0 = p.nbrPtr[s], n1 = p.nbrPtr[s + 1];
-    for (int k = k0 + lane; k < k1; k += 32)
+    int const j0 = p.pairPtr[s], j1 = p.pairPtr[s + 1];
+    for (int j = j0 + lane; j < j1; j += 32)
     {
-        uint32_t const q = p.inc[k];
+        uint2 const q   = p.pairInc[j];
+        unsigned const f = p.pairSign[j];
         double b[3], kappa, sigma;
-        corner_stiffness(p.geometry[q >> 2], p.mu[q >> 2], p.lambda[q >> 2], int(q & 3u), b, kappa, sigma);
-        p.incMat[k] = make_float2(float(kappa), float(sigma));
+        corner_stiffness(p.geometry[q.x >> 2], p.mu[q.x >> 2], p.lambda[q.x >> 2], int(q.x & 3u), b, kappa, sigma);
+        float4 m = make_float4(float(f & 1u ? -kappa : kappa), float(sigma), 0.f, 0.f);
+        if (!(f & 4u))
+        {
+            corner_stiffness(p.geometry[q.y >> 2], p.mu[q.y >> 2], p.lambda[q.y >> 2], int(q.y & 3u), b, kappa, sigma);
+            m.z = float(f & 2u ? -kappa : kappa);
+            m.w = float(sigma);
+        }
+        p.pairMat[j] = m;
         if (p.tileData)
-            reinterpret_cast<float2*>(p.tileData)[p.tileAt[s].z + k - k0] = p.incMat[k];
+            reinterpret_cast<float4*>(p.tileData)[p.tileAt[s].z + j - j0] = m;
     }
     double sum = 0.0;
     for (int j = n0 + lane; j < n1; j += 32)
@@ -515,7 +518,7 @@ cudaError_t launch_sweep(SweepParams const& p, int lanes, int block, bool chebys
     int64_t const n = int64_t(p.end - p.begin) * lanes;
     if (n <= 0)
         return cudaSuccess;
-    if (!p.incMat || !p.diag || !p.nbrPtr || !p.nbr || stagedBytes > kStagedMaxBytes || (stagedBytes > 0 && !p.incSlots))
+    if (!p.pairMat || !p.pairPtr || !p.diag || !p.nbrPtr || !p.nbr || stagedBytes > kStagedMaxBytes || (stagedBytes > 0 ? !p.pairSlots : !p.pairInc))
         return cudaErrorInvalidValue;
     // Contact terms exist only in the two-buffer sweep (a contact partner of the same colour is
     // read as it was before the pass): a one-buffer launch with contact lists is a caller error.
@@ -534,7 +537,7 @@ cudaError_t launch_sweep_record(SweepParams const& p, int lanes, int block, bool
     int64_t const n = int64_t(p.end - p.begin) * lanes;
     if (n <= 0)
         return cudaSuccess;
-    if (!p.tape || p.fc || !p.incMat || !p.diag || !p.nbrPtr || !p.nbr || stagedBytes > kStagedMaxBytes || (stagedBytes > 0 && !p.incSlots))
+    if (!p.tape || p.fc || !p.pairMat || !p.pairPtr || !p.diag || !p.nbrPtr || !p.nbr || stagedBytes > kStagedMaxBytes || (stagedBytes > 0 ? !p.pairSlots : !p.pairInc))
         return cudaErrorInvalidValue;
     int const g = blocks_for(n, block);
     return chebyshev ? launch_sweep_t<true, true>(p, lanes, g, block, pdl, s, stagedBytes)

@@ -6,9 +6,10 @@
 //   X     : float4 per vertex, rest positions (the shape-function gradients are recomputed from
 //           them, which keeps a tet record at 32 bytes)
 //   tets  : one 32-byte TetRecord per tet (below)
-//   solve : free vertices, colour-major; inside a colour sorted by decreasing degree
+//   solve : free vertices, colour-major; inside a colour (and part of the cluster step) sorted by
+//           decreasing degree
 //   incPtr: offsets of each solved vertex's incidences; inc: (tet << 2 | local index), tets
-//           ascending
+//           ascending (the reversed sweeps; the forward ones read pairs of incidences)
 //
 // A tet record is read by each of its 4 vertices in 4 different colour passes of an iteration;
 // being 32-byte aligned it costs exactly one sector per visit, and the records, incidences and
@@ -43,8 +44,6 @@ struct SweepParams
     float4 const* __restrict__ xtilde; // inertial target
     TetRecord const* __restrict__ tets;
     int32_t const* __restrict__ solve;
-    int32_t const* __restrict__ incPtr;
-    uint32_t const* __restrict__ inc;
     int32_t begin;
     int32_t end;
     float h;
@@ -72,14 +71,18 @@ struct SweepParams
     float muC;
     float muF;
     float epsv;
-    // Rest-state constants of the solves (vbd_math.cuh), solve order.  Incidence k: incMat[k] =
-    // (kappa, sigma), incSlots[k] = the three other corners' positions in the vertex's neighbour list
-    // in bytes 0-2 (corner order (local + 1 + m) & 3; staged sweep only).  Solve entry s: diag[s] = the
-    // constant s of its block and its distinct neighbours nbr[nbrPtr[s] .. nbrPtr[s+1]), each (vertex
-    // index in bits 0-29, bit 31 set when the neighbour has a lower colour, so that the two-buffer
-    // sweep reads it from x rather than hprev; K as bits).
-    float2 const* __restrict__ incMat;
-    uint32_t const* __restrict__ incSlots;
+    // Rest-state constants of the solves (vbd_math.cuh), solve order.  Pair j of incidences (of solve
+    // entry s: pairPtr[s] <= j < pairPtr[s+1]): pairMat[j] = (kappa, sigma) of its two incidences,
+    // pairSlots[j] = the positions of A, B, C, D in the vertex's neighbour list in bytes 0-3, pairInc[j]
+    // = the incidence words (tet << 2 | local).  Solve entry s: diag[s] = the constant s of its block and
+    // its distinct neighbours nbr[nbrPtr[s] .. nbrPtr[s+1]), each (vertex index in bits 0-29, bit 31 set
+    // when the neighbour has a lower colour, so that the two-buffer sweep reads it from x rather than
+    // hprev; K as bits).  pairSlots is nullptr when a vertex has more than 256 neighbours; each incidence
+    // then is a pair of its own in the corner order (local + 1 + m) & 3.
+    int32_t const* __restrict__ pairPtr;
+    float4 const* __restrict__ pairMat;
+    uint32_t const* __restrict__ pairSlots;
+    uint2 const* __restrict__ pairInc;
     float const* __restrict__ diag;
     int32_t const* __restrict__ nbrPtr;
     uint2 const* __restrict__ nbr;
@@ -144,10 +147,13 @@ struct StiffnessParams
     int32_t const* __restrict__ incPtr;
     uint32_t const* __restrict__ inc;
     int32_t const* __restrict__ nbrPtr;
-    float2* __restrict__ incMat;
+    int32_t const* __restrict__ pairPtr;
+    uint2 const* __restrict__ pairInc;
+    uint8_t const* __restrict__ pairSign; // bit 0, 1: kappa of the first, second incidence negated; 2: no second
+    float4* __restrict__ pairMat;
     uint2* __restrict__ nbr; // .y written
     // The cluster step's tiles (nullptr: none), which hold the same constants: per solve entry, the
-    // offsets of its entry (16-byte units), first neighbour and first incidence (8-byte units).
+    // offsets of its entry (16-byte units), first neighbour (8-byte units) and first pair (16-byte units).
     unsigned char* __restrict__ tileData;
     int4 const* __restrict__ tileAt;
     float* __restrict__ diag;
@@ -177,7 +183,7 @@ size_t constexpr kStagedMaxBytes = 200 * 1024;
 // Bytes of one staged neighbour: its current position (float4).
 size_t constexpr kStagedSlotBytes = sizeof(float4);
 cudaError_t prepare_staged_sweeps();
-// Writes the tets' material words (wg mu, wg lambda, 1 + mu/lambda) and incMat, nbr's K and diag of
+// Writes the tets' material words (wg mu, wg lambda, 1 + mu/lambda) and pairMat, nbr's K and diag of
 // every solve entry; sums in FP64, each result rounded once.
 cudaError_t launch_stiffness(StiffnessParams const& p, cudaStream_t s);
 cudaError_t launch_begin_substep(SubstepParams const& p, cudaStream_t s);

@@ -122,7 +122,8 @@ PBGB_HD void accumulate_tet(VertexBlock<T>& b, T const (&d)[3][3], T const (&G)[
 // The mu terms are linear in the positions with constant coefficients, so summed over the vertex's
 // tetrahedra they depend on one number per distinct neighbour j, K_oj = sum_e b_oj, and s_o =
 // -sum_j K_oj is a constant of the vertex: both are summed in FP64 and rounded once.  An incidence is
-// left with kappa_o and sigma.
+// left with kappa_o and sigma, and the sweeps take incidences in pairs that share a face (accumulate_pair),
+// which need four edge vectors instead of six.
 
 // What a tet's geometry contributes to these constants: the dot products G_a . G_b (01 02 03 12 13
 // 23), gamma_0 and the quadrature weight, in FP64.
@@ -175,6 +176,23 @@ PBGB_HD void accumulate_neighbour(VertexBlock<T>& b, T const* d, T K)
         b.g[r] += K * d[r];
 }
 
+// Adds the volume term of a tetrahedron with d_0 = A, d_1 - d_0 = u, d_2 - d_0 = v.
+template <class T>
+PBGB_HD void accumulate_volume(VertexBlock<T>& b, T const* A, T const* u, T const* v, T sigma, T kappa)
+{
+    T const p[3] = {sigma * (u[1] * v[2] - u[2] * v[1]), sigma * (u[2] * v[0] - u[0] * v[2]),
+                    sigma * (u[0] * v[1] - u[1] * v[0])};
+    T const coef = kappa - (A[0] * p[0] + A[1] * p[1] + A[2] * p[2]);
+    for (int r = 0; r < 3; ++r)
+        b.g[r] += coef * p[r];
+    b.C[0] += p[0] * p[0];
+    b.C[1] += p[0] * p[1];
+    b.C[2] += p[0] * p[2];
+    b.C[3] += p[1] * p[1];
+    b.C[4] += p[1] * p[2];
+    b.C[5] += p[2] * p[2];
+}
+
 // Adds one incidence's volume term.  d[m] = x_{a_m} - x_o in the corner order (o + 1 + m) & 3.
 template <class T>
 PBGB_HD void accumulate_incidence(VertexBlock<T>& b, T const (&d)[3][3], T sigma, T kappa)
@@ -185,17 +203,24 @@ PBGB_HD void accumulate_incidence(VertexBlock<T>& b, T const (&d)[3][3], T sigma
         u[r] = d[1][r] - d[0][r];
         v[r] = d[2][r] - d[0][r];
     }
-    T const p[3] = {sigma * (u[1] * v[2] - u[2] * v[1]), sigma * (u[2] * v[0] - u[0] * v[2]),
-                    sigma * (u[0] * v[1] - u[1] * v[0])};
-    T const coef = kappa - (d[0][0] * p[0] + d[0][1] * p[1] + d[0][2] * p[2]);
+    accumulate_volume(b, d[0], u, v, sigma, kappa);
+}
+
+// Adds a pair of incidences whose other corners are (A, B, C) and (A, C, D): two tetrahedra that share
+// the face o A C.  The corner order of either is any permutation of (o + 1 + m) & 3; an odd one turns n
+// around and with it the sign of kappa.  A second incidence with zero constants adds zeros.
+template <class T>
+PBGB_HD void accumulate_pair(VertexBlock<T>& b, T const* A, T const* B, T const* C, T const* D, T kappa1, T sigma1, T kappa2, T sigma2)
+{
+    T u[3], v[3], w[3];
     for (int r = 0; r < 3; ++r)
-        b.g[r] += coef * p[r];
-    b.C[0] += p[0] * p[0];
-    b.C[1] += p[0] * p[1];
-    b.C[2] += p[0] * p[2];
-    b.C[3] += p[1] * p[1];
-    b.C[4] += p[1] * p[2];
-    b.C[5] += p[2] * p[2];
+    {
+        u[r] = B[r] - A[r];
+        v[r] = C[r] - A[r];
+        w[r] = D[r] - A[r];
+    }
+    accumulate_volume(b, A, u, v, sigma1, kappa1);
+    accumulate_volume(b, A, v, w, sigma2, kappa2);
 }
 
 // Elastic block with Rayleigh damping (sim/vbd/Kernels.h:179-191): H = s I + C, g from the
