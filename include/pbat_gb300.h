@@ -454,6 +454,14 @@ PBGB_API int pbgb_bvh_visits(pbgb_bvh* b, int32_t* visits);
 /* Boxes of nS simplices of k (1..4) vertices over nP points (gpu/geometry/Aabb.cu:56-80,
  * Aabb::Construct(P, S)): lower / upper 3 floats per simplex. */
 PBGB_API int pbgb_simplex_boxes(int32_t nP, const float* P, int32_t nS, const int32_t* S, int32_t k, float* lower, float* upper);
+/* The same calls with arrays by rows (3 x n floats, k x nS indices of index_bytes = 4 or 8 bytes, as the
+ * reference's column-per-entity arrays lie in a row-major matrix); at least one point, box and simplex.
+ * The transposition and the checks of the indices run on the device. */
+PBGB_API int pbgb_bvh_build_columns(pbgb_bvh* b, int32_t n, const float* lower, const float* upper, const float* wmin3, const float* wmax3);
+PBGB_API int pbgb_bvh_nearest_simplices_columns(pbgb_bvh* b, int32_t nq, const float* X, int32_t nP, const float* P, int32_t nS,
+                                                const void* S, int32_t index_bytes, int32_t k, int32_t* nn);
+PBGB_API int pbgb_simplex_boxes_columns(int32_t nP, const float* P, int32_t nS, const void* S, int32_t index_bytes, int32_t k,
+                                        float* lower, float* upper);
 PBGB_API const char* pbgb_bvh_last_error(pbgb_bvh* b);
 
 /*

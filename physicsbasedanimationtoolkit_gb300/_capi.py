@@ -154,6 +154,9 @@ _SIGNATURES = [
     ("pbgb_bvh_nearest_simplices", C.c_int, [_vp, _i32, _vp, _i32, _vp, _i32, _vp, _i32, _vp]),
     ("pbgb_bvh_visits", C.c_int, [_vp, _vp]),
     ("pbgb_simplex_boxes", C.c_int, [_i32, _vp, _i32, _vp, _i32, _vp, _vp]),
+    ("pbgb_bvh_build_columns", C.c_int, [_vp, _i32, _vp, _vp, _vp, _vp]),
+    ("pbgb_bvh_nearest_simplices_columns", C.c_int, [_vp, _i32, _vp, _i32, _vp, _i32, _vp, _i32, _i32, _vp]),
+    ("pbgb_simplex_boxes_columns", C.c_int, [_i32, _vp, _i32, _vp, _i32, _i32, _vp, _vp]),
     ("pbgb_bvh_last_error", C.c_char_p, [_vp]),
     ("pbgb_ccd_create", C.c_int, [_i32, _i32, _vp, _i32, _vp, _vp, C.POINTER(_vp)]),
     ("pbgb_ccd_destroy", C.c_int, [_vp]),

@@ -82,6 +82,8 @@ struct pbgb_bvh
     int64_t pcap     = 0;
     unsigned long long* count = nullptr;
     cudaStream_t stream       = nullptr;
+    unsigned char* work = nullptr; // inputs of the *_columns calls, grown to the largest one
+    size_t workBytes    = 0;
     std::string error;
 
     ~pbgb_bvh()
@@ -89,7 +91,7 @@ struct pbgb_bvh
         if (stream)
             cudaStreamSynchronize(stream);
         pbgb::bvh_release(B);
-        void* ptrs[] = {lo, hi, qlo, qhi, pairs, count};
+        void* ptrs[] = {lo, hi, qlo, qhi, pairs, count, work};
         for (void* p : ptrs)
             if (p)
                 cudaFree(p);
@@ -122,6 +124,22 @@ struct pbgb_bvh
         ck(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     }
 
+    // At least `bytes` of device memory that only the calling entry point uses until it returns.
+    unsigned char* workspace(size_t bytes)
+    {
+        if (workBytes < bytes)
+        {
+            ck(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+            if (work)
+                cudaFree(work);
+            work      = nullptr;
+            workBytes = 0;
+            work      = dalloc<unsigned char>(bytes);
+            workBytes = bytes;
+        }
+        return work;
+    }
+
     int check_flags()
     {
         int32_t f = 0;
@@ -130,6 +148,11 @@ struct pbgb_bvh
         if (f)
         {
             ck(cudaMemsetAsync(B.flags, 0, sizeof(int32_t), stream), "cudaMemsetAsync");
+            if (f & pbgb::kBvhErrIndex)
+            {
+                error = "simplex index out of range";
+                return PBGB_ERR_INVALID_ARGUMENT;
+            }
             error = (f & pbgb::kBvhErrStackOverflow) ? "BVH traversal stack (64) overflowed"
                                                       : "BVH deeper than 64 levels";
             return PBGB_ERR_INTERNAL;
@@ -214,6 +237,43 @@ PBGB_API int pbgb_bvh_build(pbgb_bvh* b, int32_t n, const float* lower, const fl
         return bvh_fail(b, PBGB_ERR_INVALID_ARGUMENT, "pbgb_bvh_build: expected 1 <= n <= capacity and non-null boxes");
     return bvh_guard(b, [&] {
         b->upload_boxes(n, lower, upper, b->lo, b->hi);
+        b->n = n;
+        ck(pbgb::bvh_build(b->B, n, b->lo, b->hi, make_float3(wmin[0], wmin[1], wmin[2]),
+                           make_float3(wmax[0], wmax[1], wmax[2]), b->stream),
+           "bvh_build");
+        return b->check_flags();
+    });
+}
+
+// Consecutive 256-byte aligned pieces of a workspace.
+namespace {
+struct Pieces
+{
+    size_t bytes = 0;
+    size_t add(size_t n)
+    {
+        size_t const at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    }
+};
+} // namespace
+
+PBGB_API int pbgb_bvh_build_columns(pbgb_bvh* b, int32_t n, const float* lower, const float* upper, const float* wmin, const float* wmax)
+{
+    if (!b)
+        return bvh_fail(nullptr, PBGB_ERR_INVALID_ARGUMENT, "null BVH");
+    if (n < 1 || n > b->capacity || !lower || !upper || !wmin || !wmax)
+        return bvh_fail(b, PBGB_ERR_INVALID_ARGUMENT, "pbgb_bvh_build_columns: expected 1 <= n <= capacity and non-null boxes");
+    return bvh_guard(b, [&] {
+        size_t const bytes = sizeof(float) * 3 * size_t(n);
+        Pieces at;
+        size_t const l = at.add(bytes), u = at.add(bytes);
+        unsigned char* const w = b->workspace(at.bytes);
+        ck(cudaMemcpyAsync(w + l, lower, bytes, cudaMemcpyHostToDevice, b->stream), "H2D");
+        ck(cudaMemcpyAsync(w + u, upper, bytes, cudaMemcpyHostToDevice, b->stream), "H2D");
+        ck(pbgb::pack_columns(reinterpret_cast<float const*>(w + l), n, b->lo, b->stream), "pack_columns");
+        ck(pbgb::pack_columns(reinterpret_cast<float const*>(w + u), n, b->hi, b->stream), "pack_columns");
         b->n = n;
         ck(pbgb::bvh_build(b->B, n, b->lo, b->hi, make_float3(wmin[0], wmin[1], wmin[2]),
                            make_float3(wmax[0], wmax[1], wmax[2]), b->stream),
@@ -423,6 +483,49 @@ PBGB_API int pbgb_bvh_nearest_simplices(
     });
 }
 
+PBGB_API int pbgb_bvh_nearest_simplices_columns(
+    pbgb_bvh* b,
+    int32_t nq,
+    const float* X,
+    int32_t nP,
+    const float* P,
+    int32_t nS,
+    const void* S,
+    int32_t index_bytes,
+    int32_t k,
+    int32_t* nn)
+{
+    if (!b)
+        return bvh_fail(nullptr, PBGB_ERR_INVALID_ARGUMENT, "null BVH");
+    if (b->n < 1 || nq < 1 || !X || !nn || nP < 1 || !P || nS != b->n || !S || (k != 3 && k != 4) ||
+        (index_bytes != 4 && index_bytes != 8))
+        return bvh_fail(b, PBGB_ERR_INVALID_ARGUMENT,
+                        "pbgb_bvh_nearest_simplices_columns: expected the built BVH's simplices (nS = boxes), k = 3 or 4");
+    return bvh_guard(b, [&] {
+        size_t const xBytes = sizeof(float) * 3 * size_t(nq), pBytes = sizeof(float) * 3 * size_t(nP);
+        size_t const sBytes = size_t(index_bytes) * size_t(nS) * size_t(k);
+        Pieces at;
+        size_t const xr = at.add(xBytes), pr = at.add(pBytes), sr = at.add(sBytes);
+        size_t const x4 = at.add(sizeof(float4) * size_t(nq)), p4 = at.add(sizeof(float4) * size_t(nP));
+        size_t const s4 = at.add(sizeof(int32_t) * size_t(nS) * size_t(k)), out = at.add(sizeof(int32_t) * size_t(nq));
+        unsigned char* const w = b->workspace(at.bytes);
+        cudaStream_t const st  = b->stream;
+        ck(cudaMemcpyAsync(w + xr, X, xBytes, cudaMemcpyHostToDevice, st), "H2D");
+        ck(cudaMemcpyAsync(w + pr, P, pBytes, cudaMemcpyHostToDevice, st), "H2D");
+        ck(cudaMemcpyAsync(w + sr, S, sBytes, cudaMemcpyHostToDevice, st), "H2D");
+        auto* const X4 = reinterpret_cast<float4*>(w + x4);
+        auto* const P4 = reinterpret_cast<float4*>(w + p4);
+        auto* const I  = reinterpret_cast<int32_t*>(w + s4);
+        auto* const N  = reinterpret_cast<int32_t*>(w + out);
+        ck(pbgb::pack_columns(reinterpret_cast<float const*>(w + xr), nq, X4, st), "pack_columns");
+        ck(pbgb::pack_columns(reinterpret_cast<float const*>(w + pr), nP, P4, st), "pack_columns");
+        ck(pbgb::pack_simplices(w + sr, index_bytes, nS, k, nP, I, b->B.flags, st), "pack_simplices");
+        ck(pbgb::bvh_nearest_simplices(pbgb::view_of(b->B, b->n), nq, X4, P4, I, k, N, b->B.flags, st), "bvh_nearest_simplices");
+        ck(cudaMemcpyAsync(nn, N, sizeof(int32_t) * size_t(nq), cudaMemcpyDeviceToHost, st), "D2H");
+        return b->check_flags(); // synchronizes
+    });
+}
+
 PBGB_API int pbgb_bvh_visits(pbgb_bvh* b, int32_t* visits)
 {
     if (!b)
@@ -482,6 +585,49 @@ PBGB_API int pbgb_simplex_boxes(int32_t nP, const float* P, int32_t nS, const in
     {
         return bvh_fail(nullptr, PBGB_ERR_INTERNAL, e.what());
     }
+}
+
+PBGB_API int pbgb_simplex_boxes_columns(int32_t nP, const float* P, int32_t nS, const void* S, int32_t index_bytes, int32_t k, float* lower, float* upper)
+{
+    if (nP < 1 || !P || nS < 1 || !S || !lower || !upper || k < 1 || k > 4 || (index_bytes != 4 && index_bytes != 8))
+        return bvh_fail(nullptr, PBGB_ERR_INVALID_ARGUMENT, "pbgb_simplex_boxes_columns: invalid argument");
+    return bvh_guard(nullptr, [&] {
+        cudaStream_t s = nullptr;
+        ck(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
+        struct StreamGuard
+        {
+            cudaStream_t s;
+            ~StreamGuard() { cudaStreamDestroy(s); }
+        } guard{s};
+        size_t const pBytes = sizeof(float) * 3 * size_t(nP), sBytes = size_t(index_bytes) * size_t(nS) * size_t(k);
+        size_t const bBytes = sizeof(float) * 3 * size_t(nS);
+        Pieces at;
+        size_t const pr = at.add(pBytes), sr = at.add(sBytes), p4 = at.add(sizeof(float4) * size_t(nP));
+        size_t const s4 = at.add(sizeof(int32_t) * size_t(nS) * size_t(k)), lo4 = at.add(sizeof(float4) * size_t(nS));
+        size_t const hi4 = at.add(sizeof(float4) * size_t(nS)), lr = at.add(bBytes), ur = at.add(bBytes), fl = at.add(sizeof(int32_t));
+        Scratch<unsigned char> w{at.bytes};
+        auto* const P4    = reinterpret_cast<float4*>(w.p + p4);
+        auto* const I     = reinterpret_cast<int32_t*>(w.p + s4);
+        auto* const lo    = reinterpret_cast<float4*>(w.p + lo4);
+        auto* const hi    = reinterpret_cast<float4*>(w.p + hi4);
+        auto* const flags = reinterpret_cast<int32_t*>(w.p + fl);
+        ck(cudaMemsetAsync(flags, 0, sizeof(int32_t), s), "cudaMemsetAsync");
+        ck(cudaMemcpyAsync(w.p + pr, P, pBytes, cudaMemcpyHostToDevice, s), "H2D");
+        ck(cudaMemcpyAsync(w.p + sr, S, sBytes, cudaMemcpyHostToDevice, s), "H2D");
+        ck(pbgb::pack_columns(reinterpret_cast<float const*>(w.p + pr), nP, P4, s), "pack_columns");
+        ck(pbgb::pack_simplices(w.p + sr, index_bytes, nS, k, nP, I, flags, s), "pack_simplices");
+        ck(pbgb::simplex_boxes(nS, k, P4, I, lo, hi, s), "simplex_boxes");
+        ck(pbgb::unpack_columns(lo, nS, reinterpret_cast<float*>(w.p + lr), s), "unpack_columns");
+        ck(pbgb::unpack_columns(hi, nS, reinterpret_cast<float*>(w.p + ur), s), "unpack_columns");
+        int32_t f = 0;
+        ck(cudaMemcpyAsync(lower, w.p + lr, bBytes, cudaMemcpyDeviceToHost, s), "D2H");
+        ck(cudaMemcpyAsync(upper, w.p + ur, bBytes, cudaMemcpyDeviceToHost, s), "D2H");
+        ck(cudaMemcpyAsync(&f, flags, sizeof(int32_t), cudaMemcpyDeviceToHost, s), "D2H");
+        ck(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+        if (f)
+            return bvh_fail(nullptr, PBGB_ERR_INVALID_ARGUMENT, "pbgb_simplex_boxes: simplex index out of range");
+        return int(PBGB_OK);
+    });
 }
 
 PBGB_API const char* pbgb_bvh_last_error(pbgb_bvh* b)

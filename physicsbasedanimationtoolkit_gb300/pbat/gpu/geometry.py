@@ -23,6 +23,24 @@ def _points(a, what):
     return np.ascontiguousarray(a.T)
 
 
+def _by_rows(*arrays):
+    """The arrays as float32, when each is a non-empty 3 x n array that lies row after row (the library
+    then transposes on the device); None when one does not."""
+    out = []
+    for a in arrays:
+        a = np.asarray(a, dtype=np.float32)
+        if a.ndim != 2 or a.shape[0] != 3 or a.shape[1] == 0 or not a.flags.c_contiguous:
+            return None
+        out.append(a)
+    return out
+
+
+def _index_rows(S):
+    """A k x n index array row after row, as 4- or 8-byte integers."""
+    S = np.asarray(S)
+    return np.ascontiguousarray(S, dtype=S.dtype if S.dtype in (np.int32, np.int64) else np.int32)
+
+
 class Aabb:
     """Axis-aligned boxes in 3 dimensions (reference: bindings/pypbat/gpu/geometry/Aabb.cpp).
     ``construct(min, max)`` takes the corners; ``construct(P, S)`` computes the boxes of the
@@ -43,8 +61,17 @@ class Aabb:
         if "P" in kwargs or "S" in kwargs or (len(args) == 2 and np.asarray(args[1]).dtype.kind in "iu"):
             P = kwargs.get("P", args[0] if args else None)
             S = kwargs.get("S", args[1] if len(args) > 1 else None)
-            pts = _points(P, "P")
             simp = np.asarray(S)
+            rows = _by_rows(P)
+            if rows and simp.ndim == 2 and 1 <= simp.shape[0] <= 4 and simp.shape[1] > 0:
+                (pts,), idx = rows, _index_rows(simp)
+                k, nS = idx.shape
+                lo, hi = np.empty((3, nS), np.float32), np.empty((3, nS), np.float32)
+                _capi.check_bvh(_capi.lib().pbgb_simplex_boxes_columns(
+                    pts.shape[1], pts.ctypes.data, nS, idx.ctypes.data, idx.itemsize, k, lo.ctypes.data, hi.ctypes.data))
+                self._lo, self._hi = lo, hi
+                return
+            pts = _points(P, "P")
             if simp.ndim != 2 or not 1 <= simp.shape[0] <= 4:
                 raise ValueError("expected S as a K x |#simplices| array, K = 1..4")
             k, nS = simp.shape
@@ -123,9 +150,16 @@ class Bvh:
             upper = kwargs.pop("upper", None) if "upper" in kwargs else rest.pop(0)
         min = kwargs.pop("min", None) if "min" in kwargs else rest.pop(0)  # noqa: A001 (reference names)
         max = kwargs.pop("max", None) if "max" in kwargs else rest.pop(0)  # noqa: A001
-        lo, hi = self._rows(lower), self._rows(upper)
         wmin = np.ascontiguousarray(min, dtype=np.float32).ravel()
         wmax = np.ascontiguousarray(max, dtype=np.float32).ravel()
+        rows = _by_rows(lower, upper)
+        if rows and rows[0].shape == rows[1].shape:
+            lo, hi = rows
+            _capi.check_bvh(_capi.lib().pbgb_bvh_build_columns(self._h, lo.shape[1], lo.ctypes.data, hi.ctypes.data,
+                                                               wmin.ctypes.data, wmax.ctypes.data), self._h)
+            self.n = lo.shape[1]
+            return
+        lo, hi = self._rows(lower), self._rows(upper)
         _capi.check_bvh(_capi.lib().pbgb_bvh_build(self._h, lo.shape[0], lo.ctypes.data, hi.ctypes.data,
                                                    wmin.ctypes.data, wmax.ctypes.data), self._h)
         self.n = lo.shape[0]
@@ -171,9 +205,17 @@ class Bvh:
             cap = int(count.value)
 
     def _nearest(self, X, V, S, k):
+        simp = np.asarray(S)
+        rows = _by_rows(X, V)
+        if rows and simp.ndim == 2 and simp.shape[0] == k and simp.shape[1] > 0:
+            (pts, verts), idx = rows, _index_rows(simp)
+            nn = np.full(pts.shape[1], -1, np.int32)
+            _capi.check_bvh(_capi.lib().pbgb_bvh_nearest_simplices_columns(
+                self._h, pts.shape[1], pts.ctypes.data, verts.shape[1], verts.ctypes.data, idx.shape[1],
+                idx.ctypes.data, idx.itemsize, k, nn.ctypes.data), self._h)
+            return nn
         pts = _points(X, "X")
         verts = _points(V, "V")
-        simp = np.asarray(S)
         if simp.ndim != 2 or simp.shape[0] != k:
             raise ValueError(f"expected a {k} x |#simplices| index array")
         rows = np.ascontiguousarray(simp.T, dtype=np.int32)

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 import oracle_lib as O
-from physicsbasedanimationtoolkit_gb300 import meshgen, pbat
+from physicsbasedanimationtoolkit_gb300 import _capi, meshgen, pbat
 
 pytestmark = pytest.mark.gpu
 
@@ -312,3 +312,33 @@ def test_nearest_triangle_among_exact_ties(n, scale, offset, height):
     for k in range(Q.shape[0]):
         ties = order[d[k, order] == d[k].min()][:8]
         assert nn[k] == ties[-1], (k, Q[k], ties, nn[k])
+
+
+@pytest.mark.parametrize("itype", [np.int64, np.int32, np.uint16])
+@pytest.mark.parametrize("n", [1, 255, 1000])
+def test_arrays_by_rows_equal_arrays_by_columns(n, itype):
+    """Row-major 3 x n arrays go to the device as they lie, others are transposed on the host: the same
+    boxes, hierarchy and nearest triangles either way, and the same refusal of a bad index."""
+    rng = np.random.default_rng(n)
+    P = rng.uniform(-1, 1, (3, n + 2)).astype(np.float32)
+    F = np.stack([np.arange(n), np.arange(n) + 1, np.arange(n) + 2]).astype(itype)
+    Q = rng.uniform(-1, 1, (3, 77)).astype(np.float32)
+    out = []
+    for order in "CF":
+        p, f, q = (np.array(a, order=order) for a in (P, F, Q))
+        boxes = pbat.gpu.geometry.Aabb()
+        boxes.construct(p, f)
+        bvh = pbat.gpu.geometry.Bvh(n)
+        bvh.build(np.array(boxes.min, order=order), np.array(boxes.max, order=order), [-1, -1, -1], [1, 1, 1])
+        nn = bvh.point_triangle_nearest_neighbours(boxes, q, p, f)
+        out.append((boxes.min, boxes.max, bvh.ordering, bvh.parent, nn))
+        bad = np.array(F, order=order)
+        bad[2, n - 1] = n + 2
+        for call in (lambda: boxes.construct(p, bad), lambda: bvh.point_triangle_nearest_neighbours(boxes, q, p, bad)):
+            with pytest.raises(_capi.PbgbError) as err:
+                call()
+            assert err.value.code == 1 and "out of range" in str(err.value)
+        # The refusal leaves the hierarchy usable.
+        np.testing.assert_array_equal(bvh.point_triangle_nearest_neighbours(boxes, q, p, f), nn)
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
