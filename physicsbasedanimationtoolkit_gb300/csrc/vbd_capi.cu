@@ -682,12 +682,12 @@ class VbdSystem
     // 327 (alone); n = 2,369: 32 lanes 450 / 179, 8 lanes 300 / 137, 4 lanes 329 / 137; n = 8,400: 8 lanes
     // 472 / 205, 4 lanes 421 / 255; n = 18,260: 8 lanes 641 / 456, 4 lanes 681 / 308; n = 33,600
     // (Chebyshev): 8 lanes 1,296 / 1,149, 4 lanes 944 / 744, 2 lanes 1,212 / 732; blocks of 256 with 4
-    // lanes were 1 to 25 % slower.  Contact steps: 4 lanes at any size (9 cubes of 11^3, 30 iterations:
-    // 1,041 / 393, 8 lanes 1,075 / 425, 32 lanes 1,361 / 505; 4 cubes of 6^3, 20 iterations: 691 / 246, 32
-    // lanes 712 / 250).  A batch's persistent kernel takes blocks of 256 and 4 lanes, or 2 when its colours
-    // are large enough that only throughput counts (40 cubes of 12^3 to 30^3, Chebyshev, n = 59,000:
-    // 4 lanes 1.02 ms, 2 lanes 1.17 ms, blocks of 128 1.41 ms; 64 cubes of 6^3 to 32^3, n = 87,000: 2 lanes
-    // 2.32 ms, 4 lanes 2.58 ms, blocks of 128 4.2 ms).
+    // lanes were 1 to 25 % slower.  Contact steps, n = 171 (4 cubes of 6^3, 20 iterations): 8 lanes 669 /
+    // 234, 4 lanes 700 / 245, 32 lanes 664 / 238; n = 1,944 (9 cubes of 11^3, 30 iterations): 4 lanes 1,031
+    // / 395, 8 lanes 1,001 / 408, 32 lanes 1,303 / 496.  A batch's persistent kernel takes blocks of 256
+    // and 4 lanes, or 2 when its colours are large enough that only throughput counts (40 cubes of 12^3 to
+    // 30^3, Chebyshev, n = 59,000: 4 lanes 1.02 ms, 2 lanes 1.17 ms, blocks of 128 1.41 ms; 64 cubes of 6^3
+    // to 32^3, n = 87,000: 2 lanes 2.32 ms, 4 lanes 2.58 ms, blocks of 128 4.2 ms).
     int launchLanes() const
     {
         if (lanes > 0)
@@ -696,7 +696,7 @@ class VbdSystem
         if (nMeshes > 1)
             return perColor < 4096 ? 32 : (perColor < 70000 ? 4 : 2);
         if (contact)
-            return 4;
+            return perColor < 1000 ? 8 : 4;
         return perColor < 1000 ? 32 : (perColor < 12000 ? 8 : 4);
     }
 
