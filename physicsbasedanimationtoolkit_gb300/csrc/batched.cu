@@ -20,6 +20,16 @@ __device__ __forceinline__ void add_release(int32_t* q, int32_t v)
     asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(q), "r"(v) : "memory");
 }
 
+__device__ __forceinline__ void copy_async(int4* to, int4 const* from)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(uint32_t(__cvta_generic_to_shared(to))), "l"(from) : "memory");
+}
+
+__device__ __forceinline__ void copy_async_wait()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 __device__ __forceinline__ unsigned long long global_ns()
 {
     unsigned long long t;
@@ -40,7 +50,7 @@ __device__ bool wait_for(BatchedStepParams const& p, int32_t const* counter, int
     {
         if (load_acquire(counter) >= need)
             return true;
-        if (*reinterpret_cast<int32_t const volatile*>(p.control + 1) != 0)
+        if (*reinterpret_cast<int32_t const volatile*>(p.words + kBatchWordStride) != 0)
             return false;
         if (static_cast<long long>(global_ns() - t0) > p.waitNs)
             break;
@@ -48,13 +58,15 @@ __device__ bool wait_for(BatchedStepParams const& p, int32_t const* counter, int
         sleep = sleep < 1024 ? 2 * sleep : sleep;
     }
     atomicOr(p.flags + 1, 1);
-    atomicExch(p.control + 1, 1);
+    atomicExch(p.words + kBatchWordStride, 1);
     return false;
 }
 
 // Bound by memory: DRAM for batches larger than L2 (20 B per pair of incidences, 8 B per neighbour, the
 // positions that leave L2 between two colours of a mesh).  64 cubes of 6^3 to 32^3, 20 iterations: 3.05
-// ms with 24 B per incidence, 2.75 ms with 12 B, 2.37 ms with pairs and 2 lanes.
+// ms with 24 B per incidence, 2.75 ms with 12 B, 2.37 ms with pairs and 2 lanes, 2.28 ms with four
+// neighbours in flight per lane and 4 lanes, 2.26 ms with the counters on lines of their own, 2.08 ms
+// with blocks of 64, 2.06 ms with the table of one iteration (its first step 3.2 ms, 11.5 ms before).
 //
 // Colour sweep of solve entries [begin, end) by the whole block: sub-tiles of blockDim / L vertices,
 // each staged and solved like staged_sweep_kernel (the same arithmetic in the same order), with the
@@ -64,8 +76,9 @@ __device__ bool wait_for(BatchedStepParams const& p, int32_t const* counter, int
 // the records evict-first, ld.global.cs, doubled the DRAM reads of a 256-mesh step: a record's
 // sector left L2 before the neighbouring lanes had read their parts of it.)
 template <int L, bool CHEB>
-__device__ __forceinline__ void sweep_tile(SweepParams const& p, int begin, int end, float4* slab)
+__device__ __forceinline__ void sweep_tile(BatchedStepParams const& bp, SweepParams const& p, int32_t const volatile* iteration, int begin, int end, float4* slab)
 {
+    constexpr int kNbrs = L >= 16 ? 1 : (L >= 8 ? 2 : 4);
     int const per  = int(blockDim.x) / L;
     int const lane = int(threadIdx.x) & (L - 1);
     for (int f = begin; f < end; f += per)
@@ -99,13 +112,21 @@ __device__ __forceinline__ void sweep_tile(SweepParams const& p, int begin, int 
                 mt1 = __ldg(p.pairMat + k + L);
             }
             load3(Mem<true>::ld((CHEB ? p.hprev : p.x) + i), xi);
-            for (int j = n0 + lane; j < n1; j += L)
+            // kNbrs neighbours' records, then their positions, in flight together.
+            for (int j = n0 + lane; j < n1; j += kNbrs * L)
             {
-                uint2 const a     = __ldg(p.nbr + j);
-                float4 const* src = p.x;
-                if (CHEB && !(a.x >> 31))
-                    src = p.hprev;
-                stage_neighbour(b, slab + base + j - n0, Mem<true>::ld(src + (a.x & kIndexMask)), xi, __uint_as_float(a.y));
+                uint2 a[kNbrs];
+                float4 xa[kNbrs];
+#pragma unroll
+                for (int u = 0; u < kNbrs; ++u)
+                    a[u] = __ldg(p.nbr + min(j + u * L, n1 - 1));
+#pragma unroll
+                for (int u = 0; u < kNbrs; ++u)
+                    xa[u] = Mem<true>::ld((CHEB && !(a[u].x >> 31) ? p.hprev : p.x) + (a[u].x & kIndexMask));
+#pragma unroll
+                for (int u = 0; u < kNbrs; ++u)
+                    if (j + u * L < n1)
+                        stage_neighbour(b, slab + base + j + u * L - n0, xa[u], xi, __uint_as_float(a[u].y));
             }
         }
         __syncwarp();
@@ -127,7 +148,17 @@ __device__ __forceinline__ void sweep_tile(SweepParams const& p, int begin, int 
                 mt1 = mt2;
             }
         }
-        finish_vertex<L, CHEB, false, false, true>(p, b, valid, lane, i, s, xi);
+        if constexpr (CHEB)
+        {
+            // Read now: held over the loops, they would not fit the registers.
+            SweepParams q = p;
+            q.k           = *iteration;
+            q.omega       = __ldg(bp.omega + q.k);
+            q.hcur        = q.k & 1 ? bp.H1 : bp.H0;
+            finish_vertex<L, CHEB, false, false, true>(q, b, valid, lane, i, s, xi);
+        }
+        else
+            finish_vertex<L, CHEB, false, false, true>(p, b, valid, lane, i, s, xi);
         if (f + per < end)
             __syncthreads(); // the next sub-tile reuses the slab
     }
@@ -137,47 +168,79 @@ template <int L, bool CHEB>
 __global__ void __launch_bounds__(256, 4) batched_step_kernel(BatchedStepParams p)
 {
     extern __shared__ float4 slab[];
-    __shared__ int32_t sItem;
-    __shared__ int32_t sSkip;
+    // Words of the item to run and (filled at its end) of the one after it: x = -1, no items left; y = -1, the
+    // wait gave up.
+    __shared__ int4 sItem[2], sNeed[2];
+    __shared__ int32_t sIter[2];
+    // Group of the last ticket (thread 0): its first ticket, iteration (-1: begin items, iterations: end
+    // items) and substep; poison: substep -1 in sSub.
+    __shared__ int32_t sBase, sGroup, sSubstep, sSub;
     int32_t next = 0;
+    auto fetch   = [&](int32_t it, int slot) {
+        if (it >= p.nItems)
+        {
+            sItem[slot].x = -1;
+            return;
+        }
+        // Tickets only grow: step from group to group (two integer divisions took 0.2 us an item).
+        int32_t base = sBase, k = sGroup, s = sSubstep, at = 0;
+        for (;;)
+        {
+            int32_t const n = k < 0 ? p.nBegin : (k < p.iterations ? p.nSweep : p.nEnd);
+            if (it - base < n)
+                break;
+            base += n;
+            if (k == p.iterations)
+            {
+                k = -1;
+                ++s;
+            }
+            else
+                ++k;
+        }
+        at = it - base + (k < 0 ? 0 : (k < p.iterations ? p.nBegin : p.nBegin + p.nSweep));
+        copy_async(&sItem[slot], &p.items[at].a);
+        copy_async(&sNeed[slot], &p.items[at].b);
+        sBase       = base;
+        sGroup      = k;
+        sSubstep    = s;
+        sSub        = it == p.poison ? -1 : s;
+        sIter[slot] = max(k, 0);
+    };
     if (threadIdx.x == 0)
-        next = atomicAdd(p.control, 1);
-    for (;;)
+    {
+        sBase = sSubstep = 0;
+        sGroup           = -1;
+        fetch(atomicAdd(p.words, 1), 0);
+    }
+    for (int slot = 0;; slot ^= 1)
     {
         if (threadIdx.x == 0)
         {
-            int32_t const it = next;
-            sItem            = it;
-            sSkip            = 0;
-            if (it < p.nItems)
+            copy_async_wait();
+            int32_t const mesh = sItem[slot].x;
+            if (mesh >= 0)
             {
-                next            = atomicAdd(p.control, 1); // taken now, used after this item
-                int4 const a    = __ldg(&p.items[it].a);
-                int32_t const n = it == p.poison ? INT_MAX : __ldg(&p.items[it].b.x);
-                if (!wait_for(p, p.done + a.x, n))
-                    sSkip = 1;
+                int4 const n       = sNeed[slot];
+                int32_t const need = sSub < 0 ? INT_MAX : n.x + sIter[slot] * n.y + sSub * n.z;
+                next               = atomicAdd(p.words, 1); // taken now, used after this item
+                if (!wait_for(p, p.words + (2 + mesh) * kBatchWordStride, need))
+                    sItem[slot].y = -1;
             }
         }
         __syncthreads();
-        int32_t const it = sItem;
-        if (it >= p.nItems)
+        int4 const a = sItem[slot];
+        if (a.x < 0)
             break;
-        int4 const a = __ldg(&p.items[it].a);
-        if (!sSkip)
+        if (a.y >= 0)
         {
-            int const kind = a.y & 3;
+            int const kind = a.y;
             if (kind == kBatchSweep)
             {
                 SweepParams q = p.sweep;
                 if constexpr (CHEB)
-                {
-                    int const kk = a.y >> 2;
-                    q.k          = kk;
-                    q.omega      = __ldg(p.omega + kk);
-                    q.hprev      = (kk + 1) & 1 ? p.H1 : p.H0;
-                    q.hcur       = kk & 1 ? p.H1 : p.H0;
-                }
-                sweep_tile<L, CHEB>(q, a.z, a.w, slab);
+                    q.hprev = (sIter[slot] + 1) & 1 ? p.H1 : p.H0;
+                sweep_tile<L, CHEB>(p, q, &sIter[slot], a.z, a.w, slab);
             }
             else if (kind == kBatchBegin)
             {
@@ -190,11 +253,14 @@ __global__ void __launch_bounds__(256, 4) batched_step_kernel(BatchedStepParams 
                     end_substep_vertex<true>(p.sub, v);
             }
         }
+        // The next item's words load while the block's other warps finish this one.
+        if (threadIdx.x == 0)
+            fetch(next, slot ^ 1);
         __syncthreads();
         if (threadIdx.x == 0)
         {
             __threadfence();
-            add_release(p.done + a.x, 1);
+            add_release(p.words + (2 + sItem[slot].x) * kBatchWordStride, 1);
         }
     }
 }
@@ -243,7 +309,7 @@ cudaError_t launch_batched_step(BatchedStepParams const& p, int lanes, int block
     if (p.nItems <= 0)
         return cudaSuccess;
     if (grid < 1 || block < 32 || block > 256 || block % lanes != 0 || smem > kStagedMaxBytes || !p.items ||
-        !p.control || !p.done || !p.flags || !p.sweep.pairMat || !p.sweep.pairSlots || !p.sweep.nbrPtr || (chebyshev && (!p.H0 || !p.H1 || !p.omega)))
+        !p.words || !p.flags || !p.sweep.pairMat || !p.sweep.pairSlots || !p.sweep.nbrPtr || (chebyshev && (!p.H0 || !p.H1 || !p.omega)))
         return cudaErrorInvalidValue;
     return chebyshev ? launch_c<true>(p, lanes, block, grid, smem, s) : launch_c<false>(p, lanes, block, grid, smem, s);
 }

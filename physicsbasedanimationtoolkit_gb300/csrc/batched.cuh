@@ -6,12 +6,17 @@
 // vertices (begin), a tile of one colour's solve entries for one iteration (sweep), and the
 // velocity update of a range of vertices (end).  A mesh's items form a chain of stages -- begin,
 // then (iteration k, colour c) for k, c ascending, then end -- and every item of a stage needs
-// every item of the mesh's previous stage finished.  Items sit in one array, ordered by stage
-// time (substep, iteration, colour) and then by mesh, and blocks take them in that order from an
+// every item of the mesh's previous stage finished.  Items are ordered by stage time (substep,
+// iteration, colour) and then by mesh, and blocks take them in that order from an
 // atomic ticket; a block waits (bounded) until the mesh's completion counter reaches the item's
 // requirement, runs the item, and adds one to the counter.  So a mesh moves to its next colour as
 // soon as its own previous colour is done, whatever the other meshes are doing, and no launch or
 // grid-wide barrier separates colours.
+//
+// The table holds one substep's begin items, one iteration's sweep items and one substep's end
+// items; the ticket says which substep and iteration an item is of.  (A table of the whole step, 64 cubes
+// of 6^3 to 32^3, 20 iterations, tiles of 16 vertices: 28 MB, built on the host in 11.5 ms at the first
+// step of a kind, and read from DRAM once a step.)
 //
 // Progress: a block holds at most two tickets, the item it runs and the next one it took; the
 // lowest unfinished item is always some block's running item (the other ticket a block holds is
@@ -32,8 +37,10 @@ int constexpr kBatchBegin = 0; // inertial target and initial guess of vertices 
 int constexpr kBatchSweep = 1; // colour sweep of solve entries [begin, end)
 int constexpr kBatchEnd   = 2; // velocity update of vertices [begin, end)
 
-// One work item, two int4: (mesh, kind | iteration << 2, begin, end), (need, 0, 0, 0); need =
-// completed items of the mesh required before it starts.
+int constexpr kBatchWordStride = 32;
+
+// One work item, two int4: (mesh, kind, begin, end), (need, per iteration, per substep, 0): in iteration k
+// of substep s it needs need + k * per iteration + s * per substep completed items of the mesh.
 struct BatchItemWords
 {
     int4 a;
@@ -47,10 +54,15 @@ struct BatchedStepParams
     float4* H0;           // two-buffer sweep (Chebyshev): iterate buffers, nullptr for one buffer
     float4* H1;
     float const* omega;   // Chebyshev weight of each iteration
-    BatchItemWords const* items;
-    int32_t nItems;
-    int32_t* control;     // [0] ticket, [1] abort; cleared before every launch
-    int32_t* done;        // per mesh: completed items; cleared before every launch
+    BatchItemWords const* items; // nBegin + nSweep + nEnd
+    int32_t nBegin, nSweep, nEnd;
+    int32_t iterations;   // 0 when nSweep is
+    int32_t nItems;       // of the step: substeps * (nBegin + iterations * nSweep + nEnd)
+    // Words kBatchWordStride apart, cleared before every launch: [0] ticket, [1] abort, then per mesh its
+    // completed items.  Each has a cache line of its own: with the words side by side, the blocks that
+    // poll one mesh's counter held up the ticket and every other counter of the line, 21 ns an item
+    // whatever its size.
+    int32_t* words;
     int32_t* flags;       // flags[1] |= 1 when a wait gave up
     long long waitNs;     // time limit of one wait
     int32_t poison;       // item whose requirement is never met (tests of the time limit); -1: none

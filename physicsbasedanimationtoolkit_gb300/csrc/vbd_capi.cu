@@ -506,14 +506,15 @@ class VbdSystem
     {
         int32_t iters = -1, sub = -1, lanes = 0, block = 0, tile = 0;
         float dt      = 0.f;
-        int32_t nItems = 0, grid = 0;
+        int32_t nBegin = 0, nSweep = 0, nEnd = 0; // items of the table
+        int32_t nItems = 0, grid = 0;             // of the step
         size_t smem = 0;
     } plan;
     int32_t batchTile = 1; // sub-tiles of blockDim / lanes vertices per sweep item
     long long batchWaitNs = kBatchWaitNs;
     int32_t batchPoison   = -1;
     DeviceArray<BatchItemWords> batchItems;
-    DeviceArray<int32_t> batchCounters; // [0] ticket, [1] abort, then one completion counter per mesh
+    DeviceArray<int32_t> batchCounters; // BatchedStepParams::words
     DeviceArray<float> batchOmega;
 
     // Cluster step (cluster_step.cuh): the parts of every mesh and their tables, made at creation
@@ -684,17 +685,19 @@ class VbdSystem
     // (Chebyshev): 8 lanes 1,296 / 1,149, 4 lanes 944 / 744, 2 lanes 1,212 / 732; blocks of 256 with 4
     // lanes were 1 to 25 % slower.  Contact steps, n = 171 (4 cubes of 6^3, 20 iterations): 8 lanes 669 /
     // 234, 4 lanes 700 / 245, 32 lanes 664 / 238; n = 1,944 (9 cubes of 11^3, 30 iterations): 4 lanes 1,031
-    // / 395, 8 lanes 1,001 / 408, 32 lanes 1,303 / 496.  A batch's persistent kernel takes blocks of 256
-    // and 4 lanes, or 2 when its colours are large enough that only throughput counts (40 cubes of 12^3 to
-    // 30^3, Chebyshev, n = 59,000: 4 lanes 1.02 ms, 2 lanes 1.17 ms, blocks of 128 1.41 ms; 64 cubes of 6^3
-    // to 32^3, n = 87,000: 2 lanes 2.32 ms, 4 lanes 2.58 ms, blocks of 128 4.2 ms).
+    // / 395, 8 lanes 1,001 / 408, 32 lanes 1,303 / 496.  A batch's persistent kernel
+    // (batches past the cluster step) takes blocks of 64, as many as fit, and 4 lanes: an item is then 16
+    // vertices of one colour, and the wait for a colour ends with few warps idle.  us per step (blocks of 64
+    // / 128 / 256, then 64 with 2 and 8 lanes): 2 cubes of 12^3 and 30^3, 10 iterations 372 / 365 / 464, 518,
+    // 372; 40 of 12^3 to 30^3, 10 Chebyshev 838 / 849 / 887, 1,057, 1,424; 64 of 6^3 to 32^3, 20: 2,076 /
+    // 2,150 / 2,256, 2,302, 3,766; 256 of 10^3 to 14^3, 10: 819 / 851 / 932, 904, 1,465.
     int launchLanes() const
     {
         if (lanes > 0)
             return lanes;
         int const perColor = nColors > 0 ? nFree / nColors : nFree;
         if (nMeshes > 1)
-            return perColor < 4096 ? 32 : (perColor < 70000 ? 4 : 2);
+            return perColor < 1000 ? 32 : 4;
         if (contact)
             return perColor < 1000 ? 8 : 4;
         return perColor < 1000 ? 32 : (perColor < 12000 ? 8 : 4);
@@ -1354,7 +1357,7 @@ class VbdSystem
             }
         }
         this->nMeshes = nMeshes;
-        block         = nMeshes == 1 ? 128 : 256; // launchLanes
+        block         = nMeshes == 1 ? 128 : 64; // launchLanes
         meshV0.assign(size_t(nMeshes) + 1, 0);
         for (int32_t b = 0; b < nMeshes; ++b)
             meshV0[b + 1] = meshV0[b] + descs[b].n_vertices;
@@ -2053,8 +2056,8 @@ class VbdSystem
                !profiling;
     }
 
-    // Work items of the persistent step for (iterations, substeps) and the current launch shape,
-    // in stage order (substep, then begin / iteration and colour / end), meshes in order inside a
+    // Work items of the persistent step for (iterations, substeps) and the current launch shape
+    // (batched.cuh), in stage order (begin / colour / end), meshes in order inside a
     // stage, tiles in order inside a mesh; each item records how many of its mesh's items must be
     // complete first.  Stage order keeps a whole stage of items (every mesh's colour) between two
     // stages of one mesh, well over the items the resident blocks hold at once, so a block rarely
@@ -2100,34 +2103,55 @@ class VbdSystem
         check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
         std::vector<BatchItemWords> items;
         std::vector<int32_t> count(size_t(nMeshes), 0);
-        auto emit = [&](int32_t b, int kind, int32_t k, int32_t lo, int32_t hi, int32_t step) {
+        auto emit = [&](int32_t b, int kind, int32_t lo, int32_t hi, int32_t step) {
             int32_t const need = count[b];
             for (int32_t f = lo; f < hi; f += step)
             {
                 int32_t const e = std::min(f + step, hi);
-                items.push_back(BatchItemWords{make_int4(b, kind | (k << 2), f, e), make_int4(need, 0, 0, 0)});
+                items.push_back(BatchItemWords{make_int4(b, kind, f, e), make_int4(need, 0, 0, 0)});
                 ++count[b];
             }
         };
-        for (int32_t s = 0; s < substeps; ++s)
+        for (int32_t b = 0; b < nMeshes; ++b)
+            emit(b, kBatchBegin, meshV0[b], meshV0[b + 1], tileV);
+        std::vector<int32_t> const before = count;
+        size_t const nBegin = items.size();
+        for (int32_t c = 0; c < nColors; ++c)
+            for (int32_t b = 0; b < nMeshes; ++b)
+                emit(b, kBatchSweep, meshSolve[b][2 * c], meshSolve[b][2 * c + 1], tileE);
+        std::vector<int32_t> perIteration(count);
+        size_t const nSweep = items.size() - nBegin;
+        for (int32_t b = 0; b < nMeshes; ++b)
         {
-            for (int32_t b = 0; b < nMeshes; ++b)
-                emit(b, kBatchBegin, 0, meshV0[b], meshV0[b + 1], tileV);
-            for (int32_t k = 0; k < iterations; ++k)
-                for (int32_t c = 0; c < nColors; ++c)
-                    for (int32_t b = 0; b < nMeshes; ++b)
-                        emit(b, kBatchSweep, k, meshSolve[b][2 * c], meshSolve[b][2 * c + 1], tileE);
-            for (int32_t b = 0; b < nMeshes; ++b)
-                emit(b, kBatchEnd, 0, meshV0[b], meshV0[b + 1], tileV);
+            perIteration[b] -= before[b];
+            count[b] = 0; // the end items' need is filled in below
+            emit(b, kBatchEnd, meshV0[b], meshV0[b + 1], tileV);
         }
-        if (items.size() > size_t(INT32_MAX))
+        size_t const nEnd = items.size() - nBegin - nSweep;
+        // Tickets go a little past the items (two per block).
+        int64_t const perSubstep = int64_t(nBegin) + int64_t(iterations) * int64_t(nSweep) + int64_t(nEnd);
+        if (perSubstep > (int64_t(INT32_MAX) - (1 << 20)) / substeps)
             return false;
+        int64_t const nItems = perSubstep * substeps;
+        for (size_t i = 0; i < items.size(); ++i)
+        {
+            int32_t const b = items[i].a.x;
+            if (items[i].a.y == kBatchSweep)
+                items[i].b.y = perIteration[b];
+            else if (items[i].a.y == kBatchEnd)
+            {
+                // k = iterations in an end item's ticket.
+                items[i].b.x = before[b];
+                items[i].b.y = perIteration[b];
+            }
+            items[i].b.z = before[b] + iterations * perIteration[b] + count[b];
+        }
         check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
         batchItems.allocate(std::max<size_t>(items.size(), 1));
         if (!items.empty())
             check(cudaMemcpy(batchItems.get(), items.data(), sizeof(BatchItemWords) * items.size(), cudaMemcpyHostToDevice),
                   "H2D");
-        batchCounters.allocate(2 + size_t(nMeshes));
+        batchCounters.allocate((2 + size_t(nMeshes)) * kBatchWordStride);
         std::vector<float> om(size_t(std::max(iterations, 1)), 1.f);
         double omega = 0.0;
         for (int32_t k = 0; k < iterations; ++k)
@@ -2137,9 +2161,13 @@ class VbdSystem
         }
         batchOmega.allocate(om.size());
         check(cudaMemcpy(batchOmega.get(), om.data(), sizeof(float) * om.size(), cudaMemcpyHostToDevice), "H2D");
-        plan.nItems = int32_t(items.size());
+        plan.nBegin = int32_t(nBegin);
+        plan.nSweep = int32_t(nSweep);
+        plan.nEnd   = int32_t(nEnd);
+        plan.nItems = int32_t(nItems);
         plan.smem   = smem;
-        plan.grid   = int32_t(std::min<int64_t>(int64_t(perSM) * sms, std::max<int64_t>(plan.nItems, 1)));
+        // Never more items ready than one iteration, or begin or end, has.
+        plan.grid = int32_t(std::min<int64_t>(int64_t(perSM) * sms, std::max<int64_t>({plan.nBegin, plan.nSweep, plan.nEnd, 1})));
         return true;
     }
 
@@ -2169,13 +2197,16 @@ class VbdSystem
         bp.H1      = cheb ? h1.get() : nullptr;
         bp.omega   = batchOmega.get();
         bp.items   = batchItems.get();
+        bp.nBegin  = plan.nBegin;
+        bp.nSweep  = plan.nSweep;
+        bp.nEnd    = plan.nEnd;
         bp.nItems  = plan.nItems;
-        bp.control = batchCounters.get();
-        bp.done    = batchCounters.get() + 2;
+        bp.iterations = plan.nSweep > 0 ? iterations : 0;
+        bp.words   = batchCounters.get();
         bp.flags   = flags.get();
         bp.waitNs  = batchWaitNs;
         bp.poison  = batchPoison;
-        check(cudaMemsetAsync(batchCounters.get(), 0, sizeof(int32_t) * (2 + size_t(nMeshes)), stream), "memset");
+        check(cudaMemsetAsync(batchCounters.get(), 0, sizeof(int32_t) * batchCounters.size(), stream), "memset");
         check(launch_batched_step(bp, plan.lanes, plan.block, plan.grid, plan.smem, cheb, stream), "batched_step");
     }
 

@@ -115,3 +115,30 @@ def test_debug_hook_rejects_out_of_range_limits():
     assert L.pbgb_debug_batched_wait(B.handle, 5_000_000_000, -1) == 1
     assert L.pbgb_debug_batched_wait(B.handle, 1_000_000, -2) == 1
 
+
+
+# The ticket kernel itself, which small batches reach only through the hook (2^30: no item has that
+# number): no iteration, one, several substeps (the ticket tells begin, sweep and end items apart), tiles
+# of one warp, more blocks than items of a stage, and a mesh without a free vertex.
+@pytest.mark.parametrize("rho", [None, 0.9])
+@pytest.mark.parametrize("lanes,block,tile,iterations,substeps",
+                         [(0, 64, 1, 6, 1), (4, 64, 1, 0, 2), (4, 32, 1, 1, 3), (1, 256, 2, 5, 2), (16, 64, 3, 4, 1)])
+@pytest.mark.parametrize("n_meshes,nmin,nmax", [(2, 1, 2), (9, 1, 11)])
+def test_ticket_kernel_equals_colour_launches(rho, lanes, block, tile, iterations, substeps, n_meshes, nmin, nmax):
+    meshes = meshgen.batch_workload(n_meshes=n_meshes, nmin=nmin, nmax=nmax, seed=5)
+    meshes[0]["dbc"] = np.arange(meshes[0]["X"].shape[0])
+    datas = make_datas(meshes, rho)
+    P, U = pbat.gpu.vbd.BatchedIntegrator(datas), pbat.gpu.vbd.BatchedIntegrator(datas)
+    for I in (P, U):
+        I.lanes_per_vertex = lanes
+        _capi.check(_capi.lib().pbgb_vbd_set_block_size(I.handle, block), I.handle)
+    _capi.check(_capi.lib().pbgb_debug_batched_wait(P.handle, 2_000_000_000, 2**30), P.handle)
+    P.batch_tile = tile
+    U.persistent = False
+    for _ in range(2):
+        P.step(1 / 60, iterations, substeps)
+        U.step(1 / 60, iterations, substeps)
+    P.synchronize()
+    assert P.launches_per_step(iterations, substeps) == 1
+    np.testing.assert_array_equal(P.x, U.x)
+    np.testing.assert_array_equal(P.v, U.v)
