@@ -781,10 +781,26 @@ class VbdSystem
     // 24 cubes of 6^3 to 12^3 hexes: 2 blocks each 319, 4 blocks 220, 8 blocks 273; 200 cubes of 2^3 to
     // 8^3: 1 block 290, 2 blocks 476).
     // Limits: one mesh of 8,820 free vertices takes 322 us in a cluster and 321 us in colour launches,
-    // 11,638 take 377 and 362 us; batches of larger meshes keep every SM busy with the persistent
-    // kernel's tickets (64 cubes of 6^3 to 32^3: 2.8 ms, in clusters 4.0 ms), smaller ones wait there
-    // (10 cubes of 8^3 to 28^3, Chebyshev: 0.81 ms, in clusters 0.37 ms).
-    static int32_t constexpr kClusterSingleFree = 9000, kClusterBatchFree = 24000, kClusterBatchTotal = 400000;
+    // 11,638 take 377 and 362 us.  A batch's alternative is the ticket kernel, us per 10-iteration step
+    // there / in clusters.  Every mesh gets as many blocks as the largest, so mixed batches pay for idle
+    // blocks once there are more than the GPU holds: 64 of 4^3 to 28^3 (451,000 free) 937 / 1,024, 48 of
+    // them 841 / 764, 256 of 4^3 to 16^3 (422,000) 660 / 680, 128 of 4^3 to 20^3 (373,000) 796 / 690; like
+    // ones do not: 256 of 12^3 to 14^3 (659,000) 999 / 893, 512 of 10^3 to 14^3 (1,076,000) 1,720 / 1,315,
+    // 2,000 of 4^3 to 8^3 (668,000, 0.58 of the largest on average) 1,122 / 1,357.  Large parts stream their
+    // tables: 64 of 20^3 to 22^3 (652,000, 11,600 the largest) 999 / 917, 40 of 24^3 to 26^3 1,047 / 1,243.
+    // Past 24,000 vertices the cluster has 16 blocks, of which few find room at a time: 7 of 8^3 to 30^3
+    // (57,000) 533 / 239, 16 of 4^3 to 30^3 (125,000) 587 / 569, 32 of them (265,000) 724 / 804.
+    static int32_t constexpr kClusterSingleFree = 9000, kClusterBatchTotal = 400000;
+    static int32_t constexpr kClusterBatchLarge = 24000, kClusterBatchLargeTotal = 125000;
+    static int32_t constexpr kClusterBatchSmall = 12000; // with 0.65 of the largest on average: no limit
+    bool clusterPays(int64_t largest) const
+    {
+        if (nMeshes == 1)
+            return nFree <= kClusterSingleFree;
+        if (largest > kClusterBatchLarge)
+            return nFree <= kClusterBatchLargeTotal;
+        return nFree <= kClusterBatchTotal || (largest <= kClusterBatchSmall && 20 * int64_t(nFree) >= 13 * largest * nMeshes);
+    }
     int32_t chooseParts(std::vector<float4> const& X, std::vector<int32_t> const& color, std::vector<TetRecord> const& records,
                         std::vector<int32_t> const& vPtr, std::vector<uint32_t> const& vInc, bool hasContact, std::vector<int32_t>& part) const
     {
@@ -798,7 +814,7 @@ class VbdSystem
                 free[b] += color[v] >= 0 ? 1 : 0;
             largest = std::max(largest, free[b]);
         }
-        if (nMeshes == 1 ? nFree > kClusterSingleFree : (largest > kClusterBatchFree || nFree > kClusterBatchTotal))
+        if (!clusterPays(largest))
             return 0;
         int sms = 0;
         check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
