@@ -59,6 +59,79 @@ struct AdjointSweepParams
 // pdl: programmatic dependent launch (the kernel waits before reading the adjoints).
 cudaError_t launch_adjoint_sweep(AdjointSweepParams const& p, int lanes, int block, bool pdl, cudaStream_t s);
 
+// The reversed substep of a small mesh, in three kernels instead of a launch per colour and iteration:
+//
+//  * blocks: what an update of o adds to the adjoint of a neighbour j is linear in w_o, with a 3x3 block
+//    that only the tape decides.  All blocks of several iterations are formed at once, one lane per edge
+//    (o, j) over the tets around it, and their sum per o, the own adjoint's;
+//  * chain: the iterations and colours in turn, in one block.  A vertex gathers the blocks
+//    of its solved neighbours times their w -- of higher colours, which this iteration has formed, and of
+//    lower colours, from the iteration reversed before -- then forms its own w and keeps it.  No adjoint
+//    is added to by another vertex: no atomics, and the same bits in every run;
+//  * material: the sensitivities of every tet, linear in w too, from the kept w of all iterations.
+//
+// In the scatter (launch_adjoint_sweep) each colour waits for the previous one's launch, the tets'
+// arithmetic and its atomics: 4.3 us a colour and iteration, the chain 1.2 us (81 vertices).
+struct AdjointChain
+{
+    // Edges (o, j) by solve entry o: entries edgePtr[s] .. edgePtr[s + 1], each with its place in j's
+    // gather list and its tets, incidence codes tet << 4 | corner of o << 2 | index of j among the others.
+    int32_t const* edgePtr;
+    int32_t const* edgePlace;
+    int32_t const* tetPtr; // per edge
+    uint32_t const* tetCode;
+    // Gather lists by vertex j: solve entries of the neighbours, higher colours in gatherPtr[j] ..
+    // gatherMid[j], lower ones (all of them for a vertex that is never solved) up to gatherPtr[j + 1].
+    // gatherAt: their places in the chain's shared memory.
+    int32_t const* gatherPtr;
+    int32_t const* gatherMid;
+    int32_t const* gather;
+    int32_t const* gatherAt;
+    int32_t const* solve;
+    int32_t const* fixed; // the vertices that are never solved
+    int32_t const* entry; // solve entry of a vertex, -1: never solved
+    int32_t const* colorPtr;
+    float4 const* X;
+    TetRecord const* tets;
+    float const* m;
+    // Tape: iterate k at x + k nV, raw sweep result at raw + k nV, inverse matrices at tape + 2 k nFree.
+    float4 const* x;
+    float4 const* raw;
+    float4 const* tape;
+    float4 const* xs;
+    // Per iteration from kLo: block rows (2 float4 and a float per gather entry) and own sums (3 float4
+    // per solve entry); w of every iteration.
+    float4* block0;
+    float4* block1;
+    float* block2;
+    float4* own;
+    float4* w;
+    float4* ubar;
+    float4* xtbar;
+    float4* xsbar;
+    float4* yp;  // Chebyshev carries, nullptr without
+    float4* ypp;
+    float const* omega; // Chebyshev weights per iteration
+    double* dlogmu;
+    double* dloglambda;
+    int32_t nV, nT, nFree, nFixed, nEdges, nColors, iterations;
+    int32_t kLo, kHi;
+    float D, h2;
+};
+
+int constexpr kAdjointChainThreads = 512, kAdjointChainLanes = 8, kAdjointChainAhead = 2, kAdjointChainColors = 64;
+int constexpr kAdjointChainGroups = kAdjointChainThreads / kAdjointChainLanes;
+size_t constexpr kAdjointChainMaxBytes = 200 * 1024;
+
+cudaError_t launch_adjoint_blocks(AdjointChain const& p, cudaStream_t s);
+// Iterations kHi - 1 .. kLo in one block of `groups` groups of lanes, a multiple of 4 and at least the
+// largest colour, with smem bytes of shared memory (adjoint_chain_smem).
+cudaError_t launch_adjoint_chain(AdjointChain const& p, int groups, size_t smem, cudaStream_t s);
+size_t adjoint_chain_smem(int nColors, int groups, bool chebyshev);
+// Whether a block has that much; also prepares the kernel for it.
+bool adjoint_chain_fits(size_t smem);
+cudaError_t launch_adjoint_material(AdjointChain const& p, cudaStream_t s);
+
 // Start of a reversed substep: ubar = xbar + vbar / h (v = (x - xt)/h), xtbar = xsbar = 0, and the
 // Chebyshev carries yp = ypp = 0 (nullable).
 cudaError_t launch_adjoint_begin(int32_t n, float const* xbar, float const* vbar, float4* ubar, float4* xtbar, float4* xsbar,

@@ -486,6 +486,15 @@ class VbdSystem
     DeviceArray<float> adjX, adjV, adjP, adjZero;
     DeviceArray<double> adjMu, adjLa;
 
+    // Reversed substeps of small meshes (AdjointChain): the lists, made at the first
+    // pbgb_vbd_adjoint_reserve (chainEdges = -1: not yet, 0: none), and the workspace of chainSpan iterations.
+    int32_t chainEdges = -1, chainSpan = 0, chainGroups = 0;
+    size_t chainSmem = 0;
+    DeviceArray<int32_t> chainEdgePtr, chainPlace, chainTetPtr, chainGatherPtr, chainGatherMid, chainGather, chainEntry, chainColor, chainFixed, chainGatherAt;
+    DeviceArray<uint32_t> chainCode;
+    DeviceArray<float4> chainBlock0, chainBlock1, chainOwn, chainW;
+    DeviceArray<float> chainBlock2, chainOmega;
+
     // Batch layout: mesh b's vertices are [meshV0[b], meshV0[b+1]); its free vertices of colour c
     // are solve entries [meshSolve[b][2c], meshSolve[b][2c+1]) (inside colour c of the system,
     // meshes in order).
@@ -1786,6 +1795,7 @@ class VbdSystem
         ubar.allocate(size_t(nV));
         xtbar.allocate(size_t(nV));
         xsbar.allocate(size_t(nV));
+        reserveAdjointChain(iterations);
         if (nV > 0)
             check(cudaMemsetAsync(adjZero.get(), 0, sizeof(float) * 3 * size_t(nV), stream), "memset");
         tapeSlots = slots;
@@ -1793,6 +1803,239 @@ class VbdSystem
         slotH.assign(size_t(slots), 0.f);
         slotKD.assign(size_t(slots), 0.f);
         slotStrategy.assign(size_t(slots), -1);
+    }
+
+    // Bytes of blocks formed at a time: some 60 iterations of the largest mesh that takes the chain.
+    static size_t constexpr kAdjointChainBytes = size_t(16) << 20;
+
+    bool adjointChained() const { return persistent && chainSpan > 0; }
+
+    void releaseAdjointChain()
+    {
+        chainSpan = 0;
+        for (auto* a : {&chainBlock0, &chainBlock1, &chainOwn, &chainW})
+            a->release();
+        chainBlock2.release();
+        chainOmega.release();
+    }
+
+    void reserveAdjointChain(int32_t iterations)
+    {
+        releaseAdjointChain();
+        if (chainEdges < 0)
+            buildAdjointChain();
+        if (chainEdges == 0 || iterations <= 0)
+            return;
+        size_t const perIteration = size_t(chainEdges) * 36 + size_t(nFree) * 48;
+        int32_t const span        = int32_t(std::clamp<size_t>(kAdjointChainBytes / perIteration, 1, size_t(std::min(iterations, 65535))));
+        try
+        {
+            chainBlock0.allocate(size_t(span) * size_t(chainEdges));
+            chainBlock1.allocate(size_t(span) * size_t(chainEdges));
+            chainBlock2.allocate(size_t(span) * size_t(chainEdges));
+            chainOwn.allocate(size_t(span) * size_t(nFree) * 3);
+            chainW.allocate(size_t(iterations) * size_t(nFree));
+            chainOmega.allocate(size_t(iterations));
+        }
+        catch (std::exception const&)
+        {
+            // No room: the sweeps with atomics need none.
+            cudaGetLastError();
+            releaseAdjointChain();
+            return;
+        }
+        std::vector<float> om(static_cast<size_t>(iterations));
+        double omega = 0.0;
+        for (int32_t k = 0; k < iterations; ++k)
+        {
+            omega         = chebyshev_omega<double>(k, rho * rho, omega, chebFormula);
+            om[size_t(k)] = float(omega);
+        }
+        check(cudaMemcpy(chainOmega.get(), om.data(), sizeof(float) * om.size(), cudaMemcpyHostToDevice), "H2D");
+        chainSpan = span;
+    }
+
+    // The lists of AdjointChain from the incidences.  Only for meshes whose largest colour one block takes
+    // in a single round.  us per rollout of 3 steps of 15 iterations, forward and backward (some 1,300 of
+    // them host work), sweeps with atomics / chain: 81 vertices 1,954 / 1,699, 325 vertices 2,217 / 1,955,
+    // 539 vertices (63 a colour) 2,313 / 2,119; two rounds 576 vertices 2,207 / 2,558; in a cluster of
+    // blocks 931 vertices 2,270 / 2,293, 2,800 vertices 2,395 / 2,597 (its barrier took 2.5 us a colour).
+    void buildAdjointChain()
+    {
+        chainEdges = 0;
+        int32_t largest = 0;
+        for (int32_t c = 0; c < nColors; ++c)
+            largest = std::max(largest, colorPtr[c + 1] - colorPtr[c]);
+        chainGroups = (largest + 3) / 4 * 4;
+        if (nFree <= 0 || chainGroups > kAdjointChainGroups || nColors > kAdjointChainColors || nT >= (1 << 28))
+            return;
+        chainSmem = adjoint_chain_smem(nColors, chainGroups, acceleration == PBGB_ACCEL_CHEBYSHEV);
+        if (!adjoint_chain_fits(chainSmem))
+            return;
+        std::vector<TetRecord> t(static_cast<size_t>(nT));
+        std::vector<int32_t> sv(static_cast<size_t>(nFree)), ip(size_t(nFree) + 1);
+        std::vector<uint32_t> in(inc.size());
+        auto get = [&](void* dst, void const* src, size_t n) { check(cudaMemcpy(dst, src, n, cudaMemcpyDeviceToHost), "D2H"); };
+        get(t.data(), tets.get(), sizeof(TetRecord) * t.size());
+        get(sv.data(), solve.get(), 4 * sv.size());
+        get(ip.data(), incPtr.get(), 4 * ip.size());
+        get(in.data(), inc.get(), 4 * in.size());
+        std::vector<int32_t> entry(size_t(nV), -1), colorOf(size_t(nV), -1);
+        for (int32_t c = 0; c < nColors; ++c)
+            for (int32_t s = colorPtr[c]; s < colorPtr[c + 1]; ++s)
+            {
+                entry[sv[s]]   = s;
+                colorOf[sv[s]] = c;
+            }
+        // Edges (o, j) and their tets in the order of o's incidences.
+        std::vector<int32_t> edgePtr(size_t(nFree) + 1, 0), to, tetPtr(1, 0), place, where(size_t(nV), -1), stamp(size_t(nV), -1), count;
+        std::vector<uint32_t> code(size_t(ip[nFree]) * 3);
+        std::vector<int32_t> higher(size_t(nV), 0), lower(size_t(nV), 0);
+        for (int32_t s = 0; s < nFree; ++s)
+        {
+            int32_t const first = int32_t(to.size()), o = sv[s];
+            auto corners = [&](auto&& f) {
+                for (int32_t k = ip[s]; k < ip[s + 1]; ++k)
+                {
+                    uint4 const v        = t[in[k] >> 2].v;
+                    uint32_t const a4[4] = {v.x, v.y, v.z, v.w};
+                    uint32_t const il    = in[k] & 3u;
+                    for (uint32_t m = 0; m < 3; ++m)
+                        f(int32_t(a4[(il + 1 + m) & 3] & kIndexMask), ((in[k] >> 2) << 4) | (il << 2) | m);
+                }
+            };
+            corners([&](int32_t j, uint32_t) {
+                if (stamp[j] != s)
+                {
+                    stamp[j] = s;
+                    where[j] = int32_t(to.size());
+                    to.push_back(j);
+                    count.push_back(0);
+                    ++(colorOf[j] >= 0 && colorOf[o] > colorOf[j] ? higher : lower)[j];
+                }
+                ++count[where[j]];
+            });
+            int32_t at = tetPtr.back();
+            for (int32_t n = first; n < int32_t(to.size()); ++n)
+            {
+                int32_t const c = count[n];
+                count[n]        = at; // where the edge's next tet goes
+                at += c;
+                tetPtr.push_back(at);
+            }
+            corners([&](int32_t j, uint32_t c) { code[count[where[j]]++] = c; });
+            edgePtr[s + 1] = int32_t(to.size());
+        }
+        std::vector<int32_t> fixed;
+        for (int32_t j = 0; j < nV; ++j)
+            if (entry[j] < 0)
+                fixed.push_back(j);
+        // Places in the chain: by colour, chainGroups each.
+        std::vector<int32_t> held(static_cast<size_t>(nFree));
+        for (int32_t c = 0; c < nColors; ++c)
+            for (int32_t s = colorPtr[c]; s < colorPtr[c + 1]; ++s)
+                held[s] = c * chainGroups + s - colorPtr[c];
+        std::vector<int32_t> gatherPtr(size_t(nV) + 1, 0), gatherMid(size_t(nV), 0), gather(to.size());
+        std::vector<int32_t> gatherAt(to.size());
+        place.resize(to.size());
+        for (int32_t j = 0; j < nV; ++j)
+        {
+            gatherMid[j]     = gatherPtr[j] + higher[j];
+            gatherPtr[j + 1] = gatherMid[j] + lower[j];
+            higher[j]        = gatherPtr[j];
+            lower[j]         = gatherMid[j];
+        }
+        for (int32_t s = 0; s < nFree; ++s)
+            for (int32_t n = edgePtr[s]; n < edgePtr[s + 1]; ++n)
+            {
+                int32_t const j = to[n];
+                place[n]        = (colorOf[j] >= 0 && colorOf[sv[s]] > colorOf[j] ? higher : lower)[j]++;
+                gather[place[n]]   = s;
+                gatherAt[place[n]] = held[s];
+            }
+        auto put = [&](auto& array, auto const& host) {
+            array.allocate(host.size());
+            if (!host.empty())
+                check(cudaMemcpy(array.get(), host.data(), sizeof(host[0]) * host.size(), cudaMemcpyHostToDevice), "H2D");
+        };
+        try
+        {
+            put(chainEdgePtr, edgePtr);
+            put(chainPlace, place);
+            put(chainTetPtr, tetPtr);
+            put(chainCode, code);
+            put(chainGatherPtr, gatherPtr);
+            put(chainGatherMid, gatherMid);
+            put(chainGather, gather);
+            put(chainGatherAt, gatherAt);
+            put(chainEntry, entry);
+            put(chainColor, colorPtr);
+            put(chainFixed, fixed);
+        }
+        catch (std::exception const&)
+        {
+            cudaGetLastError();
+            for (auto* a : {&chainEdgePtr, &chainPlace, &chainTetPtr, &chainGatherPtr, &chainGatherMid, &chainGather, &chainEntry, &chainColor, &chainFixed, &chainGatherAt})
+                a->release();
+            chainCode.release();
+            return;
+        }
+        chainEdges = int32_t(to.size());
+    }
+
+    // Reverses the iterations of the substep in `slot` (after adjoint_begin).
+    void enqueueAdjointChain(int32_t slot, double* dlogmu, double* dloglambda)
+    {
+        bool const cheb = acceleration == PBGB_ACCEL_CHEBYSHEV;
+        AdjointChain a{};
+        a.edgePtr    = chainEdgePtr.get();
+        a.edgePlace  = chainPlace.get();
+        a.tetPtr     = chainTetPtr.get();
+        a.tetCode    = chainCode.get();
+        a.gatherPtr  = chainGatherPtr.get();
+        a.gatherMid  = chainGatherMid.get();
+        a.gather     = chainGather.get();
+        a.gatherAt   = chainGatherAt.get();
+        a.solve      = solve.get();
+        a.entry      = chainEntry.get();
+        a.fixed      = chainFixed.get();
+        a.nFixed     = nV - nFree;
+        a.colorPtr   = chainColor.get();
+        a.X          = X.get();
+        a.tets       = tets.get();
+        a.m          = m.get();
+        a.x          = slotX(slot, 0);
+        a.raw        = slotRaw(slot, 0);
+        a.tape       = slotTape(slot, 0);
+        a.xs         = slotStart(slot, 0);
+        a.block0     = chainBlock0.get();
+        a.block1     = chainBlock1.get();
+        a.block2     = chainBlock2.get();
+        a.own        = chainOwn.get();
+        a.w          = chainW.get();
+        a.ubar       = ubar.get();
+        a.xtbar      = xtbar.get();
+        a.xsbar      = xsbar.get();
+        a.yp         = cheb ? ycarry.get() : nullptr;
+        a.ypp        = cheb ? ycarry2.get() : nullptr;
+        a.omega      = chainOmega.get();
+        a.dlogmu     = dlogmu;
+        a.dloglambda = dloglambda;
+        a.nV         = nV;
+        a.nT         = nT;
+        a.nFree      = nFree;
+        a.nEdges     = chainEdges;
+        a.nColors    = nColors;
+        a.iterations = tapeIters;
+        a.D          = slotKD[slot] / slotH[slot];
+        a.h2         = slotH[slot] * slotH[slot];
+        for (a.kHi = tapeIters; a.kHi > 0; a.kHi = a.kLo)
+        {
+            a.kLo = std::max(0, a.kHi - chainSpan);
+            check(launch_adjoint_blocks(a, stream), "adjoint_blocks");
+            check(launch_adjoint_chain(a, chainGroups, chainSmem, stream), "adjoint_chain");
+        }
+        check(launch_adjoint_material(a, stream), "adjoint_material");
     }
 
     void checkDifferentiable() const
@@ -2000,6 +2243,18 @@ class VbdSystem
             check(launch_adjoint_begin(nV, xbar, vbar, ubar.get(), xtbar.get(), xsbar.get(), cheb ? ycarry.get() : nullptr,
                                        cheb ? ycarry2.get() : nullptr, h, stream),
                   "adjoint_begin");
+            auto const finish = [&] {
+                check(launch_adjoint_end(nV, xbar, vbar, pbar, ubar.get(), xtbar.get(), xsbar.get(), slotStart(slot, 1),
+                                         slotStart(slot, 2), aext.get(), h, slotStrategy[slot],
+                                         semantics == PBGB_SEMANTICS_GPU ? 1 : 0, stream),
+                      "adjoint_end");
+            };
+            if (adjointChained())
+            {
+                enqueueAdjointChain(slot, dlogmu, dloglambda);
+                finish();
+                continue;
+            }
             AdjointSweepParams a{};
             a.X          = X.get();
             a.tets       = tets.get();
@@ -2034,10 +2289,7 @@ class VbdSystem
                           "adjoint_sweep");
                 }
             }
-            check(launch_adjoint_end(nV, xbar, vbar, pbar, ubar.get(), xtbar.get(), xsbar.get(), slotStart(slot, 1),
-                                     slotStart(slot, 2), aext.get(), h, slotStrategy[slot],
-                                     semantics == PBGB_SEMANTICS_GPU ? 1 : 0, stream),
-                  "adjoint_end");
+            finish();
         }
     }
 

@@ -677,6 +677,46 @@ PBGB_HD void adjoint_tet_finish(AdjointTetPre<T> const& q, T const* w, T const* 
             c[m][r] = M[0][r] * q.G[m][0] + M[1][r] * q.G[m][1] + M[2][r] * q.G[m][2];
 }
 
+// One tet's part of the 3x3 block that takes w to the adjoint of its other corner 0, c[0] of
+// adjoint_tet_finish as a matrix applied to w:
+//   mu gg_0 I + lambda p cg^T + sA [. x y],  y = F (G_0 x go),  p = (cof F) G_0 - delta x y
+// (sum_c G_0c dcol(a)_c = a x y for any a).  Adds mu gg_0 to diag, sA y to s and lambda p cg^T to R
+// (R[r][q], row r); adjoint_block forms the block from the sums.
+template <class T>
+PBGB_HD void adjoint_edge(T const (&d)[3][3], T const (&e)[3][3], T const (&G)[3][3], T const* delta, T muw, T law, T& diag, T* s, T (&R)[3][3])
+{
+    AdjointTetPre<T> q;
+    adjoint_tet_prepare(d, e, G, delta, q);
+    T h[3], y[3], p[3];
+    h[0] = G[0][1] * q.go[2] - G[0][2] * q.go[1];
+    h[1] = G[0][2] * q.go[0] - G[0][0] * q.go[2];
+    h[2] = G[0][0] * q.go[1] - G[0][1] * q.go[0];
+    for (int r = 0; r < 3; ++r)
+        y[r] = q.f[0][r] * h[0] + q.f[1][r] * h[1] + q.f[2][r] * h[2];
+    for (int r = 0; r < 3; ++r)
+    {
+        int const r1 = (r + 1) % 3, r2 = (r + 2) % 3;
+        p[r] = law * (q.k[0][r] * G[0][0] + q.k[1][r] * G[0][1] + q.k[2][r] * G[0][2] - (delta[r1] * y[r2] - delta[r2] * y[r1]));
+    }
+    T const sA = law * (q.Jm1 - q.cB) - muw;
+    diag += muw * (q.go[0] * G[0][0] + q.go[1] * G[0][1] + q.go[2] * G[0][2]);
+    for (int r = 0; r < 3; ++r)
+    {
+        s[r] += sA * y[r];
+        for (int c = 0; c < 3; ++c)
+            R[r][c] += p[r] * q.cg[c];
+    }
+}
+
+// The block of the sums of adjoint_edge: b[3 r + q], row r.
+template <class T>
+PBGB_HD void adjoint_block(T diag, T const* s, T const (&R)[3][3], T* b)
+{
+    b[0] = R[0][0] + diag, b[1] = R[0][1] + s[2], b[2] = R[0][2] - s[1];
+    b[3] = R[1][0] - s[2], b[4] = R[1][1] + diag, b[5] = R[1][2] + s[0];
+    b[6] = R[2][0] + s[1], b[7] = R[2][1] - s[0], b[8] = R[2][2] + diag;
+}
+
 template <class T>
 PBGB_HD void adjoint_tet(
     T const (&d)[3][3],

@@ -86,3 +86,29 @@ def test_recorded_cluster_rollout_equals_colour_launches(shape, rho):
     # The same tape; the reversed sweeps add to neighbours' adjoints with FP32 atomics in any order.
     for a, b in zip(out[0][2:], out[1][2:]):
         assert np.linalg.norm(a - b) <= 1e-4 * np.linalg.norm(b)
+
+
+# The reversed chain of small meshes (blocks, chain, material sensitivities) against the sweeps with
+# atomics: one hex, a turn that fills its groups exactly or not, colours up to the limit and past it (both
+# sides take the sweeps then), iterations past one workspace, and the two sums it does not share with plain
+# iterations (damping, Chebyshev carries).  Both sum the same FP32 terms in other orders; two runs of the
+# chain give the same bits.
+@pytest.mark.parametrize("rho,kD", [(None, 0.0), (0.85, 0.0), (None, 1e-3), (0.8, 1e-3)])
+@pytest.mark.parametrize("shape,iterations", [((1, 1, 1), 3), ((4, 3, 2), 1), ((7, 3, 3), 7), ((10, 6, 6), 4), ((10, 6, 6), 70), ((15, 5, 5), 4)])
+def test_reversed_chain_equals_sweeps_with_atomics(shape, iterations, rho, kD):
+    torch = pytest.importorskip("torch")
+    d = data_of(*shape, rho=rho, kD=kD, strategy=2)
+    weight = torch.tensor(np.random.default_rng(3).uniform(-1, 1, (d.X.shape[1], 3)), dtype=torch.float32, device="cuda")
+    out = []
+    for on in (True, True, False):
+        I = pbat.gpu.vbd.Integrator(d)
+        set_persistent(I, on)
+        x0 = torch.tensor(np.ascontiguousarray(d.X.T), dtype=torch.float32, device="cuda", requires_grad=True)
+        v0 = torch.tensor(np.ascontiguousarray(d.v.T), dtype=torch.float32, device="cuda", requires_grad=True)
+        mu, lam = (torch.tensor(m, requires_grad=True) for m in d.lame)
+        x, v = pbat.gpu.vbd.rollout(I, mu, lam, x0, v0, dt=1 / 60, iterations=iterations, steps=2, substeps=2)
+        ((weight * x).sum() + (v ** 2).sum()).backward()
+        out.append([g.grad.cpu().numpy() for g in (x0, v0, mu, lam)])
+    for a, b, c in zip(*out):
+        np.testing.assert_array_equal(a, b) if shape != (15, 5, 5) else None
+        assert np.linalg.norm(a - c) <= 1e-4 * np.linalg.norm(c)
