@@ -1795,7 +1795,7 @@ class VbdSystem
         ubar.allocate(size_t(nV));
         xtbar.allocate(size_t(nV));
         xsbar.allocate(size_t(nV));
-        reserveAdjointChain(iterations);
+        reserveAdjointChain(slots > 0 ? iterations : 0);
         if (nV > 0)
             check(cudaMemsetAsync(adjZero.get(), 0, sizeof(float) * 3 * size_t(nV), stream), "memset");
         tapeSlots = slots;
@@ -1822,9 +1822,11 @@ class VbdSystem
     void reserveAdjointChain(int32_t iterations)
     {
         releaseAdjointChain();
+        if (iterations <= 0)
+            return;
         if (chainEdges < 0)
             buildAdjointChain();
-        if (chainEdges == 0 || iterations <= 0)
+        if (chainEdges == 0)
             return;
         size_t const perIteration = size_t(chainEdges) * 36 + size_t(nFree) * 48;
         int32_t const span        = int32_t(std::clamp<size_t>(kAdjointChainBytes / perIteration, 1, size_t(std::min(iterations, 65535))));
