@@ -228,7 +228,7 @@ PBGB_API int pbgb_vbd_set_damping(pbgb_vbd* h, float kD);
 PBGB_API int pbgb_vbd_set_strategy(pbgb_vbd* h, int32_t strategy);
 /* Threads per block of the vertex sweep (the reference clamps to [32, 256]). */
 PBGB_API int pbgb_vbd_set_block_size(pbgb_vbd* h, int32_t block_size);
-/* Lanes cooperating on one vertex: 1, 2, 4, 8, 16 or 32 (0 = autotuned). */
+/* Lanes cooperating on one vertex: 1, 2, 4, 8, 16 or 32 (0 = by size, or autotuned). */
 PBGB_API int pbgb_vbd_set_lanes_per_vertex(pbgb_vbd* h, int32_t lanes);
 /* Autotuner: times one step of (dt, iterations, substeps) for every lanes-per-vertex in
  * {1,2,4,8,16,32} x block size in {64,128,256}, keeps the fastest for this handle and caches it per
@@ -266,8 +266,12 @@ PBGB_API int pbgb_vbd_step_graph_kernels(pbgb_vbd* h, int64_t* kernels);
  * summed sweep intervals in milliseconds and the number of sweep kernel launches they cover. */
 PBGB_API int pbgb_vbd_set_sweep_timing(pbgb_vbd* h, int32_t enable);
 PBGB_API int pbgb_vbd_sweep_timing(pbgb_vbd* h, double* milliseconds, int64_t* sweep_launches);
-/* Persistent batched step (handles of several meshes; no counterpart in the reference, which steps
- * one mesh per integrator, gpu/impl/vbd/Integrator.cu:82-103).  On by default: one kernel launch
+/* Steps in one launch (no counterpart in the reference, which launches one kernel per colour,
+ * gpu/impl/vbd/Integrator.cu:82-103).  On by default, for plain VBD and Chebyshev without contact: small
+ * and middle meshes and batches of them step in thread-block clusters, one per mesh, and small meshes
+ * reverse a recorded step in one block; pbgb_vbd_set_persistent(h, 0) turns both off and steps with one
+ * launch per colour, with the same positions (reversed steps then add with atomics, in any order).
+ * Batches past the clusters' sizes take the persistent batched step: one kernel launch
  * per step advances every mesh, each mesh moving to its next colour as soon as its own previous
  * colour is done (per-mesh completion counters, bounded waits: a wait that gives up makes the next
  * synchronizing call return PBGB_ERR_TIMEOUT).  Used for plain VBD and Chebyshev without contact
