@@ -35,21 +35,26 @@ __device__ __forceinline__ uint32_t quantise(float c)
     return static_cast<uint32_t>(q);
 }
 
-// Also copies each box into one 32-byte record (lower, upper), so that the box pass gathers one
-// sector per leaf where it would read two half-used ones from the two input arrays.
-__global__ void morton_kernel(int32_t n, float4 const* __restrict__ lo, float4 const* __restrict__ hi, float3 wmin, float3 ext, uint32_t* __restrict__ codes, int32_t* __restrict__ inds, float4* __restrict__ packed)
+// Box i's code.  Also copies the box into one 32-byte record (lower, upper), so that the box pass
+// gathers one sector per leaf where it would read two half-used ones from the two input arrays.
+__device__ __forceinline__ uint32_t code_and_pack(int i, float4 const* lo, float4 const* hi, float3 wmin, float3 ext, float4* packed)
 {
-    int const i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
     float4 const b = lo[i], e = hi[i];
     packed[2 * size_t(i)]     = b;
     packed[2 * size_t(i) + 1] = e;
     uint32_t const x = quantise(normalised(b.x, e.x, wmin.x, ext.x));
     uint32_t const y = quantise(normalised(b.y, e.y, wmin.y, ext.y));
     uint32_t const z = quantise(normalised(b.z, e.z, wmin.z, ext.z));
-    codes[i]         = expand_bits(x) * 4u + expand_bits(y) * 2u + expand_bits(z);
-    inds[i]          = i;
+    return expand_bits(x) * 4u + expand_bits(y) * 2u + expand_bits(z);
+}
+
+__global__ void morton_kernel(int32_t n, float4 const* __restrict__ lo, float4 const* __restrict__ hi, float3 wmin, float3 ext, uint32_t* __restrict__ codes, int32_t* __restrict__ inds, float4* __restrict__ packed)
+{
+    int const i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n)
+        return;
+    codes[i] = code_and_pack(i, lo, hi, wmin, ext, packed);
+    inds[i]  = i;
 }
 
 // --- stable LSD radix sort, 8-bit digits ------------------------------------------------------
@@ -312,6 +317,114 @@ __global__ void __launch_bounds__(kSortThreads, 3) radix_scatter_kernel(
         uint32_t const g = offsets[size_t(d) * tiles + tile] + (uint32_t(j) - localStart[d]);
         kout[g]          = k;
         vout[g]          = sval[j];
+    }
+}
+
+// Codes and sort of at most a tile of boxes in one block: the keys stay in shared memory over the four
+// passes, each ranked like radix_scatter_kernel's tile (a warp takes `rounds` runs of 32 keys).  A build
+// of few boxes is bound by its launches: 13 of them here become one.  A build and a nearest query from host
+// arrays: 840 boxes 332 -> 282 us, 1,980 boxes 379 -> 322, 4,050 boxes 425 -> 381; the contact step of 4 cubes
+// of 6^3 (20 iterations) 708 -> 691 us.  Past a tile the passes fill several SMs.
+__global__ void __launch_bounds__(kSortThreads) sort_tile_kernel(
+    int32_t n,
+    int rounds,
+    float4 const* __restrict__ lo,
+    float4 const* __restrict__ hi,
+    float3 wmin,
+    float3 ext,
+    float4* __restrict__ packed,
+    uint32_t* __restrict__ codes,
+    int32_t* __restrict__ inds)
+{
+    __shared__ uint32_t skey[kTile];
+    __shared__ int32_t sval[kTile];
+    __shared__ uint32_t wcount[kWarps][kBuckets];
+    __shared__ uint32_t warpTotal[kWarps];
+    int const t               = threadIdx.x;
+    int const lane            = t & 31;
+    int const warp            = t >> 5;
+    int const base            = warp * (rounds * 32) + lane;
+    unsigned const lanesBelow = (1u << lane) - 1u;
+    for (int i = t; i < n; i += kSortThreads)
+    {
+        skey[i] = code_and_pack(i, lo, hi, wmin, ext, packed);
+        sval[i] = i;
+    }
+    for (int shift = 0; shift < 32; shift += 8)
+    {
+        for (int q = t; q < kWarps * kBuckets; q += kSortThreads)
+            (&wcount[0][0])[q] = 0;
+        __syncthreads();
+        uint32_t key[kSortRounds], rank[kSortRounds];
+        int32_t val[kSortRounds];
+#pragma unroll
+        for (int r = 0; r < kSortRounds; ++r)
+        {
+            if (r >= rounds)
+                break;
+            int const i      = base + r * 32;
+            bool const valid = i < n;
+            key[r]           = valid ? skey[i] : 0u;
+            val[r]           = valid ? sval[i] : 0;
+            uint32_t const d = valid ? (key[r] >> shift) & 0xFFu : uint32_t(kBuckets);
+            unsigned peers   = 0xffffffffu;
+#pragma unroll
+            for (int bit = 0; bit < 9; ++bit)
+            {
+                unsigned const m = __ballot_sync(0xffffffffu, (d >> bit) & 1u);
+                peers &= ((d >> bit) & 1u) ? m : ~m;
+            }
+            unsigned const below  = __popc(peers & lanesBelow);
+            uint32_t const before = valid ? wcount[warp][d] : 0u;
+            rank[r]               = ((before + below) << 8) | (d & 0xFFu);
+            __syncwarp();
+            if (valid && below == 0)
+                wcount[warp][d] = before + __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        uint32_t c = 0;
+        for (int w = 0; w < kWarps; ++w)
+            c += wcount[w][t];
+        uint32_t inc = c;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1)
+        {
+            uint32_t const y = __shfl_up_sync(0xffffffffu, inc, off);
+            if (lane >= off)
+                inc += y;
+        }
+        if (lane == 31)
+            warpTotal[warp] = inc;
+        __syncthreads();
+        uint32_t start = inc - c;
+        for (int w = 0; w < warp; ++w)
+            start += warpTotal[w];
+        for (int w = 0; w < kWarps; ++w)
+        {
+            uint32_t const m = wcount[w][t];
+            wcount[w][t]     = start;
+            start += m;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSortRounds; ++r)
+        {
+            if (r >= rounds)
+                break;
+            if (base + r * 32 < n)
+            {
+                uint32_t const pos = wcount[warp][rank[r] & 0xFFu] + (rank[r] >> 8);
+                skey[pos]          = key[r];
+                sval[pos]          = val[r];
+            }
+        }
+        __syncthreads();
+    }
+    for (int i = t; i < n; i += kSortThreads)
+    {
+        codes[i] = skey[i];
+        inds[i]  = sval[i];
     }
 }
 
@@ -699,6 +812,11 @@ cudaError_t sort_impl(BvhBuffers const& B, int32_t n, float4 const* lo, float4 c
     if (n <= 0)
         return cudaSuccess;
     float3 const ext = make_float3(wmax.x - wmin.x, wmax.y - wmin.y, wmax.z - wmin.z);
+    if (n <= kTile)
+    {
+        sort_tile_kernel<<<1, kSortThreads, 0, s>>>(n, blocks(n, kSortThreads), lo, hi, wmin, ext, B.packed, B.codes, B.inds);
+        return cudaGetLastError();
+    }
     morton_kernel<<<blocks(n, 256), 256, 0, s>>>(n, lo, hi, wmin, ext, B.codes, B.inds, B.packed);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
@@ -766,7 +884,10 @@ int64_t bvh_build_kernels(int32_t n)
             total = nb;
         }
     };
-    // Morton, 4 x (count, scan, scatter), Karras (two or more boxes), boxes.
+    // Codes and sort, Karras (two or more boxes), boxes.
+    if (n <= kTile)
+        return 1 + (n > 1 ? 1 : 0) + 1;
+    // Morton, 4 x (count, scan, scatter), Karras, boxes.
     return 1 + 4 * (2 + scan(radix_counts_size(n))) + (n > 1 ? 1 : 0) + 1;
 }
 

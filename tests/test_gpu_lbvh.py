@@ -84,6 +84,20 @@ def test_random_boxes_with_duplicate_codes(n):
     assert_same(g, O.bvh_build(lo, hi, [0, 0, 0], [1.01, 1.01, 1.01]))
 
 
+# Codes and sort of one block: rounds of a warp partly filled, the tile full and one box past it; boxes
+# that share one code or a few (the sort must keep their order).
+@pytest.mark.parametrize("n", [31, 256, 257, 4095, 4096, 4097])
+@pytest.mark.parametrize("codes", [1, 5, 0])
+def test_sort_of_one_tile(n, codes):
+    rng = np.random.default_rng(n)
+    lo = rng.uniform(0, 1, (n, 3)).astype(np.float32)
+    if codes:
+        lo = lo[rng.integers(0, codes, n)]
+    hi = (lo + np.float32(0.01)).astype(np.float32)
+    _, g = gpu_build(lo, hi, [0, 0, 0], [1.01, 1.01, 1.01])
+    assert_same(g, O.bvh_build(lo, hi, [0, 0, 0], [1.01, 1.01, 1.01]))
+
+
 def test_overlap_pairs_equal_brute_force():
     w, lo, hi, wmin, wmax = scene_boxes(True)
     X = w["X"].astype(np.float32)
