@@ -682,6 +682,76 @@ __device__ __forceinline__ float point_tet_sqdist(float3 p, float3 a, float3 b, 
                  fminf(point_triangle_sqdist(p, c, a, d), point_triangle_sqdist(p, a, c, b)));
 }
 
+// What the simplices' shapes allow the computed distances to be off by, as three lengths that are the
+// largest over the leaves (all +inf when a bound cannot be trusted: a box that does not hold its simplex,
+// a face without area, a tetrahedron without volume, NaN):
+//   shape[0]: the largest edge h;
+//   shape[1]: h^3 / A^2 of a face with twice the area A (an inverse length).  The closest point of a
+//     triangle is formed from products of the size h^2 r^2, r the distance to its corners, over A^2, so it
+//     can lie 2^-17 r^2 h^3 / A^2 off the triangle (at most 22 roundings of 2^-24 in each of four terms);
+//   shape[2]: 2^-17 h^4 / V of a tetrahedron with six times the volume V: how far outside it point_in_tet
+//     may still take a point for an inner one (a face test of a point at distance r is wrong by up to
+//     16 * 2^-24 h^2 (h + r), and one of the four is at least r V / (3 h)).
+template <int K>
+__global__ void simplex_shape_kernel(BvhView V, float4 const* __restrict__ P, int32_t const* __restrict__ S, int32_t* __restrict__ shape)
+{
+    int const s = blockIdx.x * blockDim.x + threadIdx.x;
+    float h = 0.f, face = 0.f, slack = 0.f;
+    if (s < V.n)
+    {
+        float4 const lo = node_lo(V, V.n - 1 + s), hi = node_hi(V, V.n - 1 + s);
+        int32_t const* const c = S + size_t(node_link(lo)) * K;
+        float3 p[K];
+        bool ok = true;
+#pragma unroll
+        for (int a = 0; a < K; ++a)
+        {
+            p[a] = f3(P[c[a]]);
+            ok   = ok && lo.x <= p[a].x && lo.y <= p[a].y && lo.z <= p[a].z && p[a].x <= hi.x && p[a].y <= hi.y && p[a].z <= hi.z;
+        }
+        float h2 = 0.f, least = __int_as_float(0x7f800000); // longest edge, smallest A, squared
+#pragma unroll
+        for (int a = 0; a < K; ++a)
+#pragma unroll
+            for (int b = a + 1; b < K; ++b)
+            {
+                float3 const e = sub(p[b], p[a]);
+                h2             = fmaxf(h2, dot(e, e));
+#pragma unroll
+                for (int d = b + 1; d < K; ++d)
+                {
+                    float3 const n = cross(e, sub(p[d], p[a]));
+                    least          = fminf(least, dot(n, n));
+                }
+            }
+        h    = sqrtf(h2);
+        face = h * h2 / least;
+        ok   = ok && least >= 1e-30f && h2 <= 1e13f; // products up to (2^15 h)^2 h^2 neither vanish nor overflow
+        if constexpr (K == 4)
+        {
+            float const volume = fabsf(dot(sub(p[3], p[0]), cross(sub(p[1], p[0]), sub(p[2], p[0]))));
+            slack              = 0x1p-17f * h * (h * h2 / volume);
+            ok                 = ok && volume >= 1e-28f && volume > 0x1p-16f * h * h2;
+        }
+        if (!ok)
+            h = face = slack = __int_as_float(0x7f800000);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+    {
+        h     = fmaxf(h, __shfl_xor_sync(0xffffffffu, h, off));
+        face  = fmaxf(face, __shfl_xor_sync(0xffffffffu, face, off));
+        slack = fmaxf(slack, __shfl_xor_sync(0xffffffffu, slack, off));
+    }
+    if ((threadIdx.x & 31) == 0)
+    {
+        // Non-negative floats order as their bits do.
+        atomicMax(shape, __float_as_int(h));
+        atomicMax(shape + 1, __float_as_int(face));
+        atomicMax(shape + 2, __float_as_int(slack));
+    }
+}
+
 // Nearest simplex to each query point (gpu/impl/geometry/Bvh.cuh:347-474 with the callbacks of
 // gpu/geometry/Bvh.cu:123-260): depth-first branch and bound from the root (children pushed left
 // then right, so the right child is visited first), leaves pruned by their box, exact ties (eps 0)
@@ -691,9 +761,10 @@ __device__ __forceinline__ float point_tet_sqdist(float3 p, float3 a, float3 b, 
 // Bound by its chain of dependent node reads, one query per thread: the order of the visits is the
 // reference's, not the nearest first, so without a bound most of the tree's right side is read before
 // the nearest leaf is.  21,904 queries on 43,218 triangles: a whole build and query from host arrays
-// took 3.75 ms with this kernel at 1.5 ms; with the descent's bound 2.64 ms.
+// took 3.75 ms with this kernel at 1.5 ms; with the descent's bound 2.64 ms.  The shapes' pass and its
+// margin cost 0.02 ms of the 1.09 ms the same call takes now; without the bound it takes 2.22 ms.
 template <int K>
-__global__ void nearest_simplex_kernel(BvhView V, int32_t nq, float4 const* __restrict__ X, float4 const* __restrict__ P, int32_t const* __restrict__ S, int32_t* __restrict__ nn, int32_t* __restrict__ flags)
+__global__ void nearest_simplex_kernel(BvhView V, int32_t nq, float4 const* __restrict__ X, float4 const* __restrict__ P, int32_t const* __restrict__ S, float const* __restrict__ shape, int32_t* __restrict__ nn, int32_t* __restrict__ flags)
 {
     int const q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nq)
@@ -711,9 +782,11 @@ __global__ void nearest_simplex_kernel(BvhView V, int32_t nq, float4 const* __re
                       : point_tet_sqdist(x, f3(P[c[0]]), f3(P[c[1]]), f3(P[c[2]]), f3(P[c[K - 1]]));
     };
     // A bound on the nearest distance: the leaf reached by descending into the nearer child.  With it
-    // the scan below passes over subtrees whose box lies beyond it by more than the rounding of the two
-    // distances (some 1e-7 of the coordinates): none of their leaves can be nearest or tie, and no
-    // decision about one that can depends on them.
+    // the scan below passes over subtrees whose box lies beyond it by more than the computed distances
+    // can be off (simplex_shape_kernel; the coordinates' rounding): none of their leaves can be nearest
+    // or tie, and no decision about one that can depends on them.  Where no such margin holds (shapes,
+    // boxes that do not hold their simplices, queries so far away that the distances are noise, NaN)
+    // the bound is infinite or NaN and passes over nothing.
     int32_t node = 0;
     while (node < leafBegin)
     {
@@ -721,9 +794,18 @@ __global__ void nearest_simplex_kernel(BvhView V, int32_t nq, float4 const* __re
         float const dl = point_box_sqdist(x, node_lo(V, l), node_hi(V, l)), dr = point_box_sqdist(x, node_lo(V, r), node_hi(V, r));
         node           = dr <= dl ? r : l;
     }
-    float const reach  = sqrtf(distance(node_link(node_lo(V, node))));
-    float const margin = reach + 2e-6f * (fabsf(x.x) + fabsf(x.y) + fabsf(x.z) + reach);
-    float const bound  = margin * margin;
+    float const reach = sqrtf(distance(node_link(node_lo(V, node))));
+    float const h = shape[0], face = shape[1], slack = shape[2];
+    float4 const rl = node_lo(V, 0), rh = node_hi(V, 0);
+    float3 const far = make_float3(fmaxf(x.x - rl.x, rh.x - x.x), fmaxf(x.y - rl.y, rh.y - x.y), fmaxf(x.z - rl.z, rh.z - x.z));
+    float const size = fmaxf(fabsf(rl.x), fabsf(rh.x)) + fmaxf(fabsf(rl.y), fabsf(rh.y)) + fmaxf(fabsf(rl.z), fabsf(rh.z)) +
+                       fabsf(x.x) + fabsf(x.y) + fabsf(x.z);
+    // Up to r + h = 2^15 / face a leaf's error, e = 2^-17 face (r + h)^2, grows by at most half of its
+    // distance r: a leaf that lies m beyond the reach is computed farther than the reach by more than
+    // m / 2 - e, with e at the reach.  The picks hang on differences of up to twice e: m = 8 e.
+    bool const trusted = face * (sqrtf(dot(far, far)) + h) <= 32768.f;
+    float const margin = 0x1p-14f * face * (reach + h) * (reach + h) + 2.f * slack + 0x1p-18f * (size + reach);
+    float const bound  = trusted ? (reach + margin) * (reach + margin) : __int_as_float(0x7f800000);
     int32_t stack[kBvhStack];
     int top      = 0;
     stack[top++] = 0;
@@ -841,18 +923,31 @@ cudaError_t bvh_nearest_simplices(
     float4 const* P,
     int32_t const* S,
     int32_t k,
+    float* shape,
     int32_t* nn,
     int32_t* flags,
     cudaStream_t s)
 {
     if (nq <= 0)
         return cudaSuccess;
-    if (k == 3)
-        nearest_simplex_kernel<3><<<blocks(nq, 128), 128, 0, s>>>(V, nq, X, P, S, nn, flags);
-    else if (k == 4)
-        nearest_simplex_kernel<4><<<blocks(nq, 128), 128, 0, s>>>(V, nq, X, P, S, nn, flags);
-    else
+    if (k != 3 && k != 4)
         return cudaErrorInvalidValue;
+    cudaError_t const e = cudaMemsetAsync(shape, 0, 3 * sizeof(float), s);
+    if (e != cudaSuccess)
+        return e;
+    auto* const bits = reinterpret_cast<int32_t*>(shape);
+    if (k == 3)
+    {
+        if (V.n > 0)
+            simplex_shape_kernel<3><<<blocks(V.n, 256), 256, 0, s>>>(V, P, S, bits);
+        nearest_simplex_kernel<3><<<blocks(nq, 128), 128, 0, s>>>(V, nq, X, P, S, shape, nn, flags);
+    }
+    else
+    {
+        if (V.n > 0)
+            simplex_shape_kernel<4><<<blocks(V.n, 256), 256, 0, s>>>(V, P, S, bits);
+        nearest_simplex_kernel<4><<<blocks(nq, 128), 128, 0, s>>>(V, nq, X, P, S, shape, nn, flags);
+    }
     return cudaGetLastError();
 }
 

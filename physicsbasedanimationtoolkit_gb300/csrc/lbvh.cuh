@@ -123,6 +123,7 @@ cudaError_t simplex_boxes(int32_t nS, int32_t k, float4 const* P, int32_t const*
 // Nearest simplex to each query point (gpu/geometry/Bvh.cu PointTriangleNearestNeighbors /
 // PointTetrahedronNearestNeighbors): k = 3 (triangles) or 4 (tetrahedra) vertices per simplex;
 // nn[q] = the simplex the reference's callback leaves there (the last of the exact-tie list).
+// shape: three floats of the caller's, used until the launches are done.
 cudaError_t bvh_nearest_simplices(
     BvhView const& V,
     int32_t nq,
@@ -130,6 +131,7 @@ cudaError_t bvh_nearest_simplices(
     float4 const* P,
     int32_t const* S,
     int32_t k,
+    float* shape,
     int32_t* nn,
     int32_t* flags,
     cudaStream_t s);

@@ -471,10 +471,11 @@ PBGB_API int pbgb_bvh_nearest_simplices(
     return bvh_guard(b, [&] {
         Scratch<float4> dX{size_t(nq)}, dP{size_t(nP)};
         Scratch<int32_t> dS{size_t(nS) * size_t(k)}, dnn{size_t(nq)};
+        Scratch<float> shape{3};
         upload_points(X, nq, dX.p, b->stream);
         upload_points(P, nP, dP.p, b->stream);
         ck(cudaMemcpyAsync(dS.p, S, sizeof(int32_t) * size_t(nS) * size_t(k), cudaMemcpyHostToDevice, b->stream), "H2D");
-        ck(pbgb::bvh_nearest_simplices(pbgb::view_of(b->B, b->n), nq, dX.p, dP.p, dS.p, k, dnn.p, b->B.flags, b->stream),
+        ck(pbgb::bvh_nearest_simplices(pbgb::view_of(b->B, b->n), nq, dX.p, dP.p, dS.p, k, shape.p, dnn.p, b->B.flags, b->stream),
            "bvh_nearest_simplices");
         if (nq > 0)
             ck(cudaMemcpyAsync(nn, dnn.p, sizeof(int32_t) * size_t(nq), cudaMemcpyDeviceToHost, b->stream), "D2H");
@@ -508,6 +509,7 @@ PBGB_API int pbgb_bvh_nearest_simplices_columns(
         size_t const xr = at.add(xBytes), pr = at.add(pBytes), sr = at.add(sBytes);
         size_t const x4 = at.add(sizeof(float4) * size_t(nq)), p4 = at.add(sizeof(float4) * size_t(nP));
         size_t const s4 = at.add(sizeof(int32_t) * size_t(nS) * size_t(k)), out = at.add(sizeof(int32_t) * size_t(nq));
+        size_t const sh = at.add(3 * sizeof(float));
         unsigned char* const w = b->workspace(at.bytes);
         cudaStream_t const st  = b->stream;
         ck(cudaMemcpyAsync(w + xr, X, xBytes, cudaMemcpyHostToDevice, st), "H2D");
@@ -520,7 +522,8 @@ PBGB_API int pbgb_bvh_nearest_simplices_columns(
         ck(pbgb::pack_columns(reinterpret_cast<float const*>(w + xr), nq, X4, st), "pack_columns");
         ck(pbgb::pack_columns(reinterpret_cast<float const*>(w + pr), nP, P4, st), "pack_columns");
         ck(pbgb::pack_simplices(w + sr, index_bytes, nS, k, nP, I, b->B.flags, st), "pack_simplices");
-        ck(pbgb::bvh_nearest_simplices(pbgb::view_of(b->B, b->n), nq, X4, P4, I, k, N, b->B.flags, st), "bvh_nearest_simplices");
+        ck(pbgb::bvh_nearest_simplices(pbgb::view_of(b->B, b->n), nq, X4, P4, I, k, reinterpret_cast<float*>(w + sh), N, b->B.flags, st),
+           "bvh_nearest_simplices");
         ck(cudaMemcpyAsync(nn, N, sizeof(int32_t) * size_t(nq), cudaMemcpyDeviceToHost, st), "D2H");
         return b->check_flags(); // synchronizes
     });

@@ -356,3 +356,114 @@ def test_arrays_by_rows_equal_arrays_by_columns(n, itype):
         np.testing.assert_array_equal(bvh.point_triangle_nearest_neighbours(boxes, q, p, f), nn)
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+def scan_without_bound(bvh, lo, hi, x, distance):
+    """The nearest simplex as the query's depth-first scan leaves it: right child first, nodes passed over by
+    their box alone, ties of the smallest distance kept in a list of 8 whose last entry stays."""
+    t = bvh._topology()
+    n = lo.shape[0]
+    x = np.asarray(x, np.float32)
+
+    def box(k):
+        l, h = (t["ilo"][k], t["ihi"][k]) if k < n - 1 else (lo[t["inds"][k - n + 1]], hi[t["inds"][k - n + 1]])
+        d = np.maximum(np.maximum(l - x, x - h), 0).astype(np.float64)
+        return (d * d).sum()
+
+    stack, ties, best = [0], [], np.inf
+    while stack:
+        k = stack.pop()
+        if box(k) > best:
+            continue
+        if k < n - 1:
+            stack += [t["child"][k][0], t["child"][k][1]]
+            continue
+        i = int(t["inds"][k - n + 1])
+        d = distance(x, i)
+        if d < best:
+            best, ties = d, [i]
+        elif d <= best and len(ties) < 8:
+            ties.append(i)
+    return ties[-1] if ties else -1
+
+
+def boxes_and_tree(P, S):
+    boxes = pbat.gpu.geometry.Aabb()
+    boxes.construct(P.T, S.T)
+    bvh = pbat.gpu.geometry.Bvh(S.shape[0])
+    bvh.build(boxes, P.min(0) - 1, P.max(0) + 1)
+    return boxes, bvh
+
+
+def test_a_tetrahedron_on_a_line_is_its_own_nearest():
+    """No volume: every point of the space is at distance zero by the face tests, also far from the box."""
+    P = np.array([[0, 0, 0], [1, 0, 0], [2, 0, 0], [3, 0, 0]], np.float32)
+    T = np.array([[0, 1, 2, 3]])
+    boxes, bvh = boxes_and_tree(P, T)
+    Q = np.array([[0.5, 0, 0], [-4, 0, 0], [1, 7, 0], [90, -3, 2]], np.float32)
+    np.testing.assert_array_equal(bvh.point_tetrahedron_nearest_neighbours(boxes, Q.T, P.T, T.T), np.zeros(4, np.int32))
+
+
+@pytest.mark.parametrize("n", [1, 3, 40])
+def test_nearest_of_flat_tetrahedra_in_their_plane(n):
+    """Coplanar corners: a query of the plane is inside every tetrahedron by the face tests, so the scan takes the
+    first leaf it meets and the ties whose box holds the query."""
+    rng = np.random.default_rng(n)
+    P = np.concatenate([rng.integers(-64, 64, (4 * n, 2)), np.zeros((4 * n, 1))], 1).astype(np.float32)
+    T = np.arange(4 * n).reshape(n, 4)
+    boxes, bvh = boxes_and_tree(P, T)
+    Q = np.concatenate([rng.integers(-256, 256, (200, 2)), np.zeros((200, 1))], 1).astype(np.float32)
+    nn = bvh.point_tetrahedron_nearest_neighbours(boxes, Q.T, P.T, T.T)
+    lo, hi = boxes.min.T, boxes.max.T
+    expected = [scan_without_bound(bvh, lo, hi, q, lambda x, i: 0.0) for q in Q]
+    np.testing.assert_array_equal(nn, expected)
+
+
+@pytest.mark.parametrize("shift", [3.0, 64.0, -500.0])
+def test_nearest_triangles_with_boxes_of_an_earlier_pose(shift):
+    """The hierarchy was built before the triangles moved: what the scan returns depends on the boxes it passes
+    over, and is never nothing."""
+    n = 9
+    i, j = (a.ravel() for a in np.meshgrid(np.arange(n + 1), np.arange(n + 1), indexing="ij"))
+    P = np.stack([i, j, 0.0 * i], 1).astype(np.float32)
+    a, b = (c.ravel() for c in np.meshgrid(np.arange(n), np.arange(n), indexing="ij"))
+    v = a * (n + 1) + b
+    F = np.stack([v, v + n + 1, v + n + 2], 1)  # the half of each cell with u >= v
+    boxes, bvh = boxes_and_tree(P, F)
+    moved = P + np.array([shift, 0, 0], np.float32)
+    Q = np.concatenate([moved[:40] + [0.5, 0.25, 0], P[:40] + [0.5, 0.25, 2.0]]).astype(np.float32)
+
+    def distance(x, t):
+        # Dyadic coordinates: exact.
+        o = moved[F[t][0]].astype(np.float64)
+        u, w = x[0] - o[0], x[1] - o[1]
+        cu, cw = min(max(u, 0.0), 1.0), min(max(w, 0.0), 1.0)
+        if cw > cu:
+            cu = cw = min(max((u + w) / 2, 0.0), 1.0)
+        return (u - cu) ** 2 + (w - cw) ** 2 + float(x[2]) ** 2
+
+    nn = bvh.point_triangle_nearest_neighbours(boxes, Q.T, moved.T, F.T)
+    lo, hi = boxes.min.T, boxes.max.T
+    np.testing.assert_array_equal(nn, [scan_without_bound(bvh, lo, hi, q, distance) for q in Q])
+
+
+@pytest.mark.parametrize("k", [3, 4])
+@pytest.mark.parametrize("scale,offset,flat", [(1.0, 0.0, 1.0), (0.01, 30.0, 1.0), (1.0, 0.0, 1e-3), (100.0, -3e3, 1e-5)])
+def test_the_bound_changes_no_pick(k, scale, offset, flat):
+    """Random simplices, round and flat, queries near and far: the same picks as when the bound is off.  One
+    simplex lies far from every query; with a corner moved out of its box no bound is trusted."""
+    rng = np.random.default_rng(int(100 * scale) + k)
+    n = 700
+    c = rng.uniform(-1, 1, (n, 1, 3)) * scale
+    d = rng.uniform(-1, 1, (n, k, 3)) * scale * 0.05 * np.array([1, flat, flat**0.5])
+    P = (c + d).reshape(-1, 3) + offset
+    P[-k:] = offset + scale * 1e3 + d[0]
+    P = P.astype(np.float32)
+    S = np.arange(n * k).reshape(n, k)
+    boxes, bvh = boxes_and_tree(P, S)
+    Q = offset + scale * rng.uniform(-1, 1, (3000, 3)) * 10.0 ** rng.uniform(-2, 1, (3000, 1))
+    Q = np.concatenate([Q, P[rng.integers(0, (n - 1) * k, 500)]]).astype(np.float32)
+    query = bvh.point_triangle_nearest_neighbours if k == 3 else bvh.point_tetrahedron_nearest_neighbours
+    out = P.copy()
+    out[-1] += scale
+    np.testing.assert_array_equal(query(boxes, Q.T, P.T, S.T), query(boxes, Q.T, out.T, S.T))
