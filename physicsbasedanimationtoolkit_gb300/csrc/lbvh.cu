@@ -793,10 +793,10 @@ __global__ void pack_simplices_kernel(T const* __restrict__ rows, int32_t nS, in
     bool ok = true;
     for (int a = 0; a < k; ++a)
     {
-        int32_t const v           = int32_t(rows[size_t(a) * size_t(nS) + i]);
-        bool const in             = v >= 0 && v < nP;
-        ok                        = ok && in;
-        out[size_t(i) * k + a]    = in ? v : 0;
+        T const v              = rows[size_t(a) * size_t(nS) + i]; // compared at its own width
+        bool const in          = v >= 0 && v < T(nP);
+        ok                     = ok && in;
+        out[size_t(i) * k + a] = in ? int32_t(v) : 0;
     }
     if (!ok)
         atomicOr(flags, kBvhErrIndex);

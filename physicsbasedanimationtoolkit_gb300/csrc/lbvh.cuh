@@ -111,13 +111,13 @@ cudaError_t bvh_self_overlaps(
     int32_t* flags,
     cudaStream_t s);
 
-// Boxes of nS simplices of k (1..4) vertices each: S[k i + a] indexes P.
 // 3 x n floats by rows -> float4 per point (w = 0), and back.
 cudaError_t pack_columns(float const* rows, int32_t n, float4* out, cudaStream_t s);
 cudaError_t unpack_columns(float4 const* in, int32_t n, float* rows, cudaStream_t s);
 // k x nS indices by rows (4- or 8-byte integers) -> k per simplex; one outside [0, nP) becomes 0 and
 // raises kBvhErrIndex.
 cudaError_t pack_simplices(void const* rows, int32_t bytes, int32_t nS, int32_t k, int32_t nP, int32_t* out, int32_t* flags, cudaStream_t s);
+// Boxes of nS simplices of k (1..4) vertices each: S[k i + a] indexes P.
 cudaError_t simplex_boxes(int32_t nS, int32_t k, float4 const* P, int32_t const* S, float4* lo, float4* hi, cudaStream_t s);
 
 // Nearest simplex to each query point (gpu/geometry/Bvh.cu PointTriangleNearestNeighbors /

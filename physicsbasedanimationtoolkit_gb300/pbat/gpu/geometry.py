@@ -35,10 +35,18 @@ def _by_rows(*arrays):
     return out
 
 
+def _narrowed(S):
+    """The indices as 32-bit integers, those that do not fit as -1 (which the library refuses)."""
+    S = np.asarray(S)
+    if S.dtype.kind in "iu" and S.dtype.itemsize >= 4 and S.dtype != np.int32:
+        S = np.where((S < 0) | (S > np.iinfo(np.int32).max), -1, S.astype(np.int64))
+    return S.astype(np.int32, copy=False)
+
+
 def _index_rows(S):
     """A k x n index array row after row, as 4- or 8-byte integers."""
     S = np.asarray(S)
-    return np.ascontiguousarray(S, dtype=S.dtype if S.dtype in (np.int32, np.int64) else np.int32)
+    return np.ascontiguousarray(S if S.dtype in (np.int32, np.int64) else _narrowed(S))
 
 
 class Aabb:
@@ -75,7 +83,7 @@ class Aabb:
             if simp.ndim != 2 or not 1 <= simp.shape[0] <= 4:
                 raise ValueError("expected S as a K x |#simplices| array, K = 1..4")
             k, nS = simp.shape
-            S_rows = np.ascontiguousarray(simp.T, dtype=np.int32)
+            S_rows = np.ascontiguousarray(_narrowed(simp).T)
             lo = np.zeros((nS, 3), np.float32)
             hi = np.zeros((nS, 3), np.float32)
             _capi.check_bvh(_capi.lib().pbgb_simplex_boxes(pts.shape[0], pts.ctypes.data, nS, S_rows.ctypes.data, k,
@@ -218,7 +226,7 @@ class Bvh:
         verts = _points(V, "V")
         if simp.ndim != 2 or simp.shape[0] != k:
             raise ValueError(f"expected a {k} x |#simplices| index array")
-        rows = np.ascontiguousarray(simp.T, dtype=np.int32)
+        rows = np.ascontiguousarray(_narrowed(simp).T)
         nn = np.full(pts.shape[0], -1, np.int32)
         _capi.check_bvh(_capi.lib().pbgb_bvh_nearest_simplices(
             self._h, pts.shape[0], pts.ctypes.data, verts.shape[0], verts.ctypes.data, rows.shape[0],

@@ -467,3 +467,27 @@ def test_the_bound_changes_no_pick(k, scale, offset, flat):
     out = P.copy()
     out[-1] += scale
     np.testing.assert_array_equal(query(boxes, Q.T, P.T, S.T), query(boxes, Q.T, out.T, S.T))
+
+
+@pytest.mark.parametrize("itype", [np.int64, np.uint64, np.uint32])
+@pytest.mark.parametrize("order", "CF")
+@pytest.mark.parametrize("bad", [2**32 + 2, 2**63 + 1, 2**32 - 1, -1])
+def test_wide_indices_are_checked_before_they_are_narrowed(itype, order, bad):
+    """An index that is out of range is refused, whatever its low 32 bits are."""
+    if not np.iinfo(itype).min <= bad <= np.iinfo(itype).max:
+        pytest.skip("not a value of the type")
+    rng = np.random.default_rng(0)
+    P = np.array(rng.uniform(-1, 1, (3, 9)).astype(np.float32), order=order)
+    F = np.array(np.stack([np.arange(7), np.arange(7) + 1, np.arange(7) + 2]).astype(itype), order=order)
+    boxes = pbat.gpu.geometry.Aabb()
+    boxes.construct(P, F)
+    bvh = pbat.gpu.geometry.Bvh(7)
+    bvh.build(boxes, [-1, -1, -1], [1, 1, 1])
+    nn = bvh.point_triangle_nearest_neighbours(boxes, P, P, F)
+    wrong = F.copy(order="K")
+    wrong[1, 3] = bad
+    for call in (lambda: boxes.construct(P, wrong), lambda: bvh.point_triangle_nearest_neighbours(boxes, P, P, wrong)):
+        with pytest.raises(_capi.PbgbError) as err:
+            call()
+        assert err.value.code == 1 and "out of range" in str(err.value)
+    np.testing.assert_array_equal(bvh.point_triangle_nearest_neighbours(boxes, P, P, F), nn)
