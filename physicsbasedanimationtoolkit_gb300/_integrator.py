@@ -103,6 +103,9 @@ class IntegratorBase:
             rc = L.pbgb_vbd_create_batched(descs, len(batch), C.byref(h))
         _capi.check(rc)
         self._h = h
+        # The rollout (pbat.gpu.vbd.rollout) whose last segment the tape holds, and the one whose material
+        # is set; None after anything else wrote either.
+        self._tape_of = self._material_of = None
         self._keep = None  # the library copied everything during create
         nV, nT, nF, nC = (C.c_int32() for _ in range(4))
         _capi.check(L.pbgb_vbd_sizes(h, C.byref(nV), C.byref(nT), C.byref(nF), C.byref(nC)), h)
@@ -255,6 +258,7 @@ class IntegratorBase:
         lam = np.ascontiguousarray(lam, dtype=np.float64).ravel()
         if mu.size != self.n_tets or lam.size != self.n_tets:
             raise ValueError(f"expected {self.n_tets} Lame coefficients")
+        self._material_of = None
         _capi.check(_capi.lib().pbgb_vbd_set_material(self._h, mu.ctypes.data, lam.ctypes.data), self._h)
 
     # Device-pointer state access (|#vertices| x 3 float32 on the handle's device).  Stream-ordered
@@ -270,9 +274,11 @@ class IntegratorBase:
         _capi.check(getattr(_capi.lib(), fn)(self._h, C.c_void_p(ptr)), self._h)
 
     def adjoint_reserve(self, slots, iterations):
+        self._tape_of = None
         _capi.check(_capi.lib().pbgb_vbd_adjoint_reserve(self._h, int(slots), int(iterations)), self._h)
 
     def step_record(self, dt, iterations, substeps, slot):
+        self._tape_of = None
         _capi.check(_capi.lib().pbgb_vbd_step_record(self._h, float(dt), int(iterations), int(substeps), int(slot)),
                     self._h)
 

@@ -189,7 +189,9 @@ class _Rollout:
                 ctx.integ = integ
                 ctx.args = (dt, iterations, substeps, steps, every)
                 ctx.checkpoints = checkpoints
-                ctx.taped = True  # the tape holds the last segment until a backward reuses its slots
+                # The tape holds the last segment, and the integrator this material, until something else
+                # (a backward, another rollout on the integrator) takes their place.
+                ctx.rollout = integ._tape_of = integ._material_of = object()
                 ctx.final = (xT.clone(), vT.clone(), pT)
                 ctx.save_for_backward(mu, lam)
                 return xT, vT
@@ -208,7 +210,11 @@ class _Rollout:
                 pbar = torch.zeros((nV, 3), dtype=torch.float32, device=dev)
                 dlogmu = torch.zeros(nT, dtype=torch.float64, device=dev)
                 dloglambda = torch.zeros_like(dlogmu)
+                taped = integ._tape_of is ctx.rollout
                 integ.adjoint_reserve(min(every, steps) * substeps, iterations)
+                if integ._material_of is not ctx.rollout:
+                    integ.set_material(mu.detach().cpu().numpy(), lam.detach().cpu().numpy())
+                    integ._material_of = ctx.rollout
                 torch.cuda.synchronize(dev)
                 nseg = len(ctx.checkpoints)
                 for seg in reversed(range(nseg)):
@@ -218,10 +224,9 @@ class _Rollout:
                     integ._set_device("x", cx.data_ptr())
                     integ._set_device("v", cv.data_ptr())
                     integ._set_device("vprev", cp.data_ptr())
-                    if not (seg == nseg - 1 and ctx.taped):
+                    if not (seg == nseg - 1 and taped):
                         for t in range(start, end):
                             integ.step_record(dt, iterations, substeps, (t - start) * substeps)
-                    ctx.taped = False
                     for t in reversed(range(start, end)):
                         integ.step_adjoint((t - start) * substeps, substeps, xbar.data_ptr(), vbar.data_ptr(),
                                            dlogmu.data_ptr(), dloglambda.data_ptr(), pbar.data_ptr())
@@ -253,7 +258,8 @@ def rollout(integrator, mu, lam, x0, v0, dt=0.01, iterations=20, steps=1, subste
     damping, every initial guess (the adaptive guesses' factor is differentiated on the branch the
     forward took), no contact.  The previous velocities the integrator holds at the start (read by
     AdaptiveVbd) are part of the start state but not differentiated.  Backward leaves the
-    integrator at the rollout's end state.
+    integrator at the rollout's end state, with its material.  Several rollouts may be recorded on one
+    integrator before any backward; all but the last then re-run their last segment too.
     """
     if checkpoint_every < 1:
         raise ValueError("checkpoint_every must be >= 1")

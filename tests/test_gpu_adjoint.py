@@ -237,3 +237,46 @@ def test_adaptive_vbd_needs_the_state_entry_point():
         I.step_adjoint(0, 1, xb.data_ptr(), vb.data_ptr(), dm.data_ptr(), dl.data_ptr())
     I.step_adjoint(0, 1, xb.data_ptr(), vb.data_ptr(), dm.data_ptr(), dl.data_ptr(), pb.data_ptr())
     I.synchronize()
+
+
+@pytest.mark.parametrize("every", [2, 5])
+@pytest.mark.parametrize("iterations,first", [((6, 6), 0), ((6, 6), 1), ((4, 9), 0), ((9, 4), 1)])
+def test_rollouts_recorded_on_one_integrator_before_their_backward(every, iterations, first):
+    """Each backward reverses its own iterates with its own material, whichever comes first and whatever
+    the other rollout reserved: the gradients are those of an integrator per rollout, bit for bit (the mesh
+    is small enough for the reversed chain, which sums in a fixed order)."""
+    w = meshgen.adjoint_beam_workload(nx=5, ny=2, nz=2)
+    rng = np.random.default_rng(every)
+    inputs = []
+    for _ in range(2):
+        mu, lam = meshgen.lame(np.exp(w["logE"] + rng.uniform(-0.5, 0.5)), np.full(w["T"].shape[0], w["nu"]))
+        inputs.append((mu, lam, w["X"] + rng.uniform(-0.01, 0.01, w["X"].shape), rng.uniform(-1, 1, w["X"].shape)))
+
+    def forward(I, k):
+        mu, lam, x0, v0 = inputs[k]
+        leaves = [torch.tensor(mu, requires_grad=True), torch.tensor(lam, requires_grad=True),
+                  torch.tensor(x0, dtype=torch.float32, device="cuda", requires_grad=True),
+                  torch.tensor(v0, dtype=torch.float32, device="cuda", requires_grad=True)]
+        x, v = pbat.gpu.vbd.rollout(I, *leaves, dt=1 / 60, iterations=iterations[k], steps=3 + k, checkpoint_every=every)
+        return leaves, (x ** 2).sum() + (v ** 2).sum()
+
+    def gradients(leaves):
+        return [a.grad.cpu().numpy() for a in leaves]
+
+    alone = []
+    for k in range(2):
+        leaves, loss = forward(gpu_integrator(w), k)
+        loss.backward()
+        alone.append(gradients(leaves))
+    I = gpu_integrator(w)
+    both = [forward(I, k) for k in range(2)]
+    for k in (first, 1 - first):
+        both[k][1].backward()
+        for a, b in zip(gradients(both[k][0]), alone[k]):
+            np.testing.assert_array_equal(a, b)
+    # A material set by hand in between does not reach the gradients either.
+    leaves, loss = forward(I, 0)
+    I.set_material(*inputs[1][:2])
+    loss.backward()
+    for a, b in zip(gradients(leaves), alone[0]):
+        np.testing.assert_array_equal(a, b)
