@@ -513,6 +513,10 @@ PBGB_API int pbgb_debug_adjoint_tet(
  * follow.  With a poisoned item the step's wait gives up after wait_ns, the step ends with invalid
  * positions and the next synchronizing call returns PBGB_ERR_TIMEOUT; the context stays usable. */
 PBGB_API int pbgb_debug_batched_wait(pbgb_vbd* h, int64_t wait_ns, int32_t poison_item);
+/* The same for the steps that run in thread-block clusters: the time limit of one wait and one tile of
+ * the first block, counted over the step, that never arrives (-1, or a number the step does not reach:
+ * none). */
+PBGB_API int pbgb_debug_cluster_wait(pbgb_vbd* h, int64_t wait_ns, int32_t poison_tile);
 
 /* Host self-check of the closed-form vertex block (FP64): accumulates n incident tets and
  * applies damping, inertia and the Newton step exactly like the device sweep.  Arguments as the

@@ -66,30 +66,40 @@ __device__ __forceinline__ bool barrier_passed(uint32_t a, uint32_t parity)
     return done != 0u;
 }
 
-// Waits for the end of the barrier's phase `parity`.  After kMaxPolls tries (each suspends the thread
-// for up to some microseconds) it raises flags[1] and the block's give-up word, after which every wait
-// of the block returns at once: the step then ends with positions the host reports as not valid.
-int constexpr kMaxPolls = 1 << 22;
-__device__ __noinline__ void barrier_wait_slow(uint32_t a, uint32_t parity, int32_t volatile* gaveUp, int32_t* flags)
+__device__ __forceinline__ unsigned long long global_ns()
 {
-    for (int n = 0; n < kMaxPolls; ++n)
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Waits for the end of the barrier's phase `parity`; false when it gave up: after `ns` nanoseconds, or at
+// once when another wait of the block (gaveUp) or of the launch (flags[1], which the host reports) has.
+__device__ __noinline__ bool barrier_wait_slow(uint32_t a, uint32_t parity, int32_t volatile* gaveUp, int32_t* flags, long long ns)
+{
+    unsigned long long const t0 = global_ns();
+    for (;;)
     {
         if (barrier_passed(a, parity))
-            return;
-        if ((n & 15) == 15 && *gaveUp)
-            return;
+            return true;
+        if (*gaveUp || *reinterpret_cast<int32_t const volatile*>(flags + 1) ||
+            static_cast<long long>(global_ns() - t0) > ns)
+            break;
     }
     *gaveUp = 1;
     atomicOr(flags + 1, 1);
+    return false;
 }
 
-__device__ __forceinline__ void barrier_wait(uint64_t* bar, uint32_t parity, int32_t volatile* gaveUp, int32_t* flags)
+__device__ __forceinline__ bool barrier_wait(uint64_t* bar, uint32_t parity, int32_t volatile* gaveUp, int32_t* flags, long long ns)
 {
     uint32_t const a = shared_address(bar);
-    if (!barrier_passed(a, parity))
-        barrier_wait_slow(a, parity, gaveUp, flags);
+    return barrier_passed(a, parity) || barrier_wait_slow(a, parity, gaveUp, flags, ns);
 }
 
+// When a wait gives up, the tile that did not arrive is never read and a barrier whose phase did not end is
+// not arrived on again; the warps run down the step's block and cluster barriers.  The positions are then
+// not valid, which the host reports.
 template <int L, bool CHEB, bool REC, bool CLUSTER>
 __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_kernel(ClusterStepParams p)
 {
@@ -118,6 +128,7 @@ __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_k
     bool const resident   = nTiles <= p.stages;
     SubstepParams const& sub = p.sub;
     int32_t* const flags     = sub.flags;
+    long long const ns       = p.waitNs;
 
     if (threadIdx.x == 0)
     {
@@ -140,31 +151,48 @@ __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_k
     if (warp == warps)
     {
         // The producer: every tile of every iteration in order (once, when all stay).
-        int stage = 0;
+        int stage = 0, issued = 0;
         uint32_t round = 0;
+        bool issuing   = wlane == 0;
+        int const poison = blockIdx.x == 0 ? p.poison : -1; // a tile that never comes (tests)
         for (int ss = 0; ss < p.substeps; ++ss)
         {
             cluster_sync<CLUSTER>();
-            if (wlane == 0 && (!resident || ss == 0))
+            if (issuing && (!resident || ss == 0))
             {
                 int const passes = resident ? (p.iterations > 0 ? 1 : 0) : p.iterations;
-                for (int k = 0; k < passes; ++k)
+                for (int k = 0; k < passes && issuing; ++k)
                     for (int t = 0; t < nTiles; ++t)
                     {
-                        if (round > 0)
-                            barrier_wait(empty + stage, (round - 1) & 1u, gaveUp, flags);
+                        if (round > 0 && !barrier_wait(empty + stage, (round - 1) & 1u, gaveUp, flags, ns))
+                        {
+                            issuing = false;
+                            break;
+                        }
                         int2 const d = __ldg(p.tiles + tile0 + t);
                         barrier_expect(full + stage, uint32_t(d.y));
-                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                         shared_address(ring + size_t(stage) * size_t(p.stageBytes))),
-                                     "l"(p.tileData + size_t(d.x) * 16), "r"(d.y), "r"(shared_address(full + stage))
-                                     : "memory");
+                        if (issued != poison)
+                            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                             shared_address(ring + size_t(stage) * size_t(p.stageBytes))),
+                                         "l"(p.tileData + size_t(d.x) * 16), "r"(d.y), "r"(shared_address(full + stage))
+                                         : "memory");
+                        ++issued;
                         if (++stage == p.stages)
                         {
                             stage = 0;
                             ++round;
                         }
                     }
+            }
+            __syncwarp();
+            if (ss + 1 == p.substeps && wlane == 0)
+            {
+                // No copy is on its way when the block ends, also when a wait gave up.
+                unsigned long long const t0 = global_ns();
+                for (int i = max(issued - p.stages, 0); i < issued; ++i)
+                    while (i != poison && !barrier_passed(shared_address(full + i % p.stages), uint32_t(i / p.stages) & 1u) &&
+                           static_cast<long long>(global_ns() - t0) <= ns)
+                        ;
             }
             __syncwarp();
             if (CLUSTER || ss + 1 < p.substeps)
@@ -181,6 +209,7 @@ __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_k
     float4* const slab      = (CHEB ? B + p.ownedCapacity : B) + warp * p.slabPerWarp;
     int stage0 = 0;       // stage of the colour's first tile
     uint32_t round0 = 0u; // times the ring came round before it
+    bool solving    = true; // the warp's (no wait gave up)
 
     for (int ss = 0; ss < p.substeps; ++ss)
     {
@@ -246,6 +275,17 @@ __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_k
             uint32_t const phase = uint32_t(ss * p.iterations + k) & 1u;
             bool const first     = ss == 0 && k == 0; // resident tiles arrive during the first iteration
             int tile             = 0; // the colour's first tile in the part
+            // A warp takes the same tiles in every iteration, so that it has waited for each itself.  Once a wait
+            // of the block gave up: no second arrival on a barrier whose phase did not end, and little sent to
+            // blocks that stopped (they stop this one within an iteration, through what they do not send).
+            if (CLUSTER)
+                solving = solving && !__any_sync(0xffffffffu, *gaveUp);
+            if (!solving)
+            {
+                for (int c = 0; c < p.nColors; ++c)
+                    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+                continue;
+            }
             for (int c = 0; c < p.nColors; ++c)
             {
                 int2 const count       = color[c];
@@ -273,10 +313,14 @@ __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_k
                         // of `empty` tells the two apart: the warp's last tile lies at most a ring
                         // back, stages >= warps / L, so the tile two rings back is consumed.)
                         if (round > 0u)
-                            barrier_wait(empty + stage, (round - 1u) & 1u, gaveUp, flags);
+                            solving = solving && barrier_wait(empty + stage, (round - 1u) & 1u, gaveUp, flags, ns);
                     }
                     if (!resident || first)
-                        barrier_wait(full + stage, par, gaveUp, flags);
+                    {
+                        solving = __all_sync(0xffffffffu, solving && barrier_wait(full + stage, par, gaveUp, flags, ns));
+                        if (!solving)
+                            break;
+                    }
                     unsigned char const* const base = ring + size_t(stage) * size_t(p.stageBytes);
                     int4 const* const entry         = reinterpret_cast<int4 const*>(base) + 2 * ((g % L) * (32 / L) + wlane / L);
                     int4 const e0                   = entry[0];
@@ -382,7 +426,7 @@ __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_k
                 }
                 asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
                 if (CLUSTER && expects)
-                    barrier_wait(halo + c, phase, gaveUp, flags);
+                    barrier_wait(halo + c, phase, gaveUp, flags, ns);
             }
         }
 
@@ -396,6 +440,11 @@ __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_k
         if (CLUSTER || ss + 1 < p.substeps)
             cluster_sync<CLUSTER>();
     }
+    // Positions sent to a block that stopped waiting for them may still be on their way (a microsecond or
+    // so; there is no barrier left to tell): it stays until long after.
+    if (CLUSTER && *gaveUp)
+        for (int n = 0; n < 100; ++n)
+            __nanosleep(1000);
 }
 
 template <bool CHEB, bool REC, bool CLUSTER>

@@ -20,6 +20,10 @@
 // it, follow every read of b's old position.  The same holds for the phase of a colour's barrier: bytes
 // of the next iteration are sent only after the block has passed this iteration's wait.
 //
+// Every wait has a time limit.  Asking for a tile as a warp costs a vote per group where tiles are streamed: a
+// 5,040-vertex Chebyshev step of 2 x 15 iterations 125 -> 130 us among others; steps whose tiles stay are
+// as fast as without the limit (1331 vertices 58.2 us, 27 vertices 24.1).
+//
 // What bounds it: with a few solves per part and colour, the chain of one vertex solve (about 300
 // instructions of one warp, 0.8 us) times the colours; with many, shared memory (with three 16-byte reads per
 // incidence: L1 at 68 % with 272 vertices per block and colour, issue at 44 %).  A first version with a
@@ -75,6 +79,8 @@ struct ClusterStepParams
     int32_t slabPerWarp;   // staged neighbours of the warp that stages the most
     int32_t stages;        // ring slots
     int32_t stageBytes;    // largest tile, a multiple of 128
+    long long waitNs;      // time limit of one wait
+    int32_t poison;        // tile of the first block (counted over the step) that never arrives (tests of the limit); -1: none
     // Recording (REC): the tape of the substep's slot, advanced by its stride per substep.
     float4* __restrict__ tapeX;   // iterates X_0 .. X_K, nV each
     float4* __restrict__ tapeRaw; // Chebyshev: raw sweep results, nV each

@@ -539,6 +539,8 @@ class VbdSystem
     {
         int32_t lanes = 0, warps = 0, slabPerWarp = 0, stages = 0, resident = 0, residentRecord = 0;
     } clusterLaunch;
+    long long clusterWaitNs = kBatchWaitNs; // pbgb_debug_cluster_wait
+    int32_t clusterPoison   = -1;
     bool stepInCluster      = false; // the last step ran (or is being captured) as a cluster launch
     int32_t omegaIterations = -1; // iterations stepOmega holds the Chebyshev weights of
     DeviceArray<float> stepOmega;
@@ -1181,6 +1183,8 @@ class VbdSystem
         p.tileData       = tileData.get();
         p.iterations     = iterations;
         p.substeps       = substeps;
+        p.waitNs         = clusterWaitNs;
+        p.poison         = clusterPoison;
         if (record)
         {
             p.tapeX          = slotX(slot0, 0);
@@ -3210,13 +3214,14 @@ class VbdSystem
         check(cudaMemcpy(f, flags.get(), sizeof(f), cudaMemcpyDeviceToHost), "cudaMemcpy");
         if (f[1] != 0)
         {
-            check(cudaMemset(flags.get(), 0, sizeof(f)), "cudaMemset");
+            // On the handle's stream: the next step may raise them again.
+            check(cudaMemsetAsync(flags.get(), 0, sizeof(f), stream), "cudaMemsetAsync");
             lastError = "a bounded device wait of the persistent step gave up; the step's positions are not valid";
             return kTimeout;
         }
         if (f[0] != 0)
         {
-            check(cudaMemset(flags.get(), 0, sizeof(int32_t)), "cudaMemset");
+            check(cudaMemsetAsync(flags.get(), 0, sizeof(int32_t), stream), "cudaMemsetAsync");
             lastError = "non-finite positions or velocities detected on the device";
             return kNonFinite;
         }
@@ -3844,6 +3849,18 @@ PBGB_API int pbgb_debug_batched_wait(pbgb_vbd* h, int64_t wait_ns, int32_t poiso
         return fail(h, kInvalid, "pbgb_debug_batched_wait: expected 1 us <= wait_ns <= 2 s and poison_item >= -1");
     h->sys.batchWaitNs = wait_ns;
     h->sys.batchPoison = poison_item;
+    h->sys.invalidate();
+    return kOk;
+}
+
+PBGB_API int pbgb_debug_cluster_wait(pbgb_vbd* h, int64_t wait_ns, int32_t poison_tile)
+{
+    if (!h)
+        return fail(nullptr, kInvalid, "null handle");
+    if (wait_ns < 1000 || wait_ns > pbgb::kBatchWaitNs || poison_tile < -1)
+        return fail(h, kInvalid, "pbgb_debug_cluster_wait: expected 1 us <= wait_ns <= 2 s and poison_tile >= -1");
+    h->sys.clusterWaitNs = wait_ns;
+    h->sys.clusterPoison = poison_tile;
     h->sys.invalidate();
     return kOk;
 }

@@ -3,6 +3,8 @@ launches per colour: the per-vertex arithmetic, its order and the lanes are the 
 velocities must be equal bit for bit, whatever the number of blocks, the ring of tiles or the rounds of a
 colour; and a recorded rollout must tape the same iterates."""
 
+import time
+
 import numpy as np
 import pytest
 
@@ -112,3 +114,63 @@ def test_reversed_chain_equals_sweeps_with_atomics(shape, iterations, rho, kD):
     for a, b, c in zip(*out):
         np.testing.assert_array_equal(a, b) if shape != (15, 5, 5) else None
         assert np.linalg.norm(a - c) <= 1e-4 * np.linalg.norm(c)
+
+
+# A tile that never arrives: resident and streamed tiles, one block and several (the others then wait for
+# positions that do not come), the first tile and a later one, of a later iteration where tiles are streamed,
+# and a batch.  The step ends with PBGB_ERR_TIMEOUT soon after the limit, and after the hook is cleared the
+# same step from the same state is that of an integrator that never timed out.
+@pytest.mark.parametrize("shapes,lanes,tile", [([(2, 2, 2)], 0, 0), ([(9, 9, 9)], 4, 0), ([(9, 9, 9)], 0, 3),
+                                               ([(20, 20, 20)], 2, 0), ([(20, 20, 20)], 2, 40), ([(20, 20, 20)], 0, 25),
+                                               ([(2, 2, 2), (5, 5, 5), (7, 7, 7)], 0, 1)])
+@pytest.mark.parametrize("rho,substeps", [(None, 1), (0.85, 2)])
+def test_a_cluster_wait_that_runs_out_reports_a_timeout_and_the_context_survives(shapes, lanes, tile, rho, substeps):
+    datas = [data_of(*s, rho=rho, strategy=2) for s in shapes]
+    A, B = (pbat.gpu.vbd.BatchedIntegrator(datas) if len(datas) > 1 else pbat.gpu.vbd.Integrator(datas[0]) for _ in range(2))
+    for I in (A, B):
+        I.lanes_per_vertex = lanes
+    L = _capi.lib()
+    x0, v0 = A.x, A.v
+    for _ in range(2):
+        _capi.check(L.pbgb_debug_cluster_wait(A.handle, 5_000_000, tile), A.handle)
+        A.step(1 / 60, 8, substeps)
+        start = time.perf_counter()
+        with pytest.raises(_capi.PbgbError) as err:
+            A.synchronize()
+        assert err.value.code == 7
+        assert time.perf_counter() - start < 1.0
+        assert A.launches_per_step(8, substeps) == 1
+        _capi.check(L.pbgb_debug_cluster_wait(A.handle, 2_000_000_000, -1), A.handle)
+        A.x, A.v = x0, v0
+        A.step(1 / 60, 8, substeps)
+        A.synchronize()
+        if _ == 0:
+            B.step(1 / 60, 8, substeps)
+        np.testing.assert_array_equal(A.x, B.x)
+        np.testing.assert_array_equal(A.v, B.v)
+
+
+def test_a_recorded_cluster_step_that_times_out():
+    d = data_of(9, 9, 9, rho=0.85, strategy=2)
+    A, B = pbat.gpu.vbd.Integrator(d), pbat.gpu.vbd.Integrator(d)
+    L = _capi.lib()
+    x0, v0 = A.x, A.v
+    for I in (A, B):
+        I.adjoint_reserve(2, 6)
+    _capi.check(L.pbgb_debug_cluster_wait(A.handle, 5_000_000, 2), A.handle)
+    A.step_record(1 / 60, 6, 2, 0)
+    with pytest.raises(_capi.PbgbError) as err:
+        A.synchronize()
+    assert err.value.code == 7
+    _capi.check(L.pbgb_debug_cluster_wait(A.handle, 2_000_000_000, -1), A.handle)
+    A.x, A.v = x0, v0
+    for I in (A, B):
+        I.step_record(1 / 60, 6, 2, 0)
+    np.testing.assert_array_equal(A.x, B.x)
+
+
+def test_the_cluster_hook_rejects_out_of_range_limits():
+    I = pbat.gpu.vbd.Integrator(data_of(2, 2, 2))
+    L = _capi.lib()
+    for ns, tile in ((10, -1), (5_000_000_000, -1), (1_000_000, -2)):
+        assert L.pbgb_debug_cluster_wait(I.handle, ns, tile) == 1
