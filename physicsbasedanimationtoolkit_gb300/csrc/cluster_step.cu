@@ -55,14 +55,23 @@ __device__ __forceinline__ void barrier_arrive(uint64_t* bar, uint32_t count)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(shared_address(bar)), "r"(count) : "memory");
 }
 
-// Whether the barrier's phase `parity` is over (suspends the thread for a while when not).
+// Whether the barrier's phase `parity` is over (suspends the thread for a while when not).  CLUSTER: what
+// other blocks stored with the phase's bytes is then visible (an acquire at the block's scope orders the
+// block's own copies only).
+template <bool CLUSTER>
 __device__ __forceinline__ bool barrier_passed(uint32_t a, uint32_t parity)
 {
     uint32_t done;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(done)
-                 : "r"(a), "r"(parity)
-                 : "memory");
+    if constexpr (CLUSTER)
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(done)
+                     : "r"(a), "r"(parity)
+                     : "memory");
+    else
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(done)
+                     : "r"(a), "r"(parity)
+                     : "memory");
     return done != 0u;
 }
 
@@ -75,12 +84,13 @@ __device__ __forceinline__ unsigned long long global_ns()
 
 // Waits for the end of the barrier's phase `parity`; false when it gave up: after `ns` nanoseconds, or at
 // once when another wait of the block (gaveUp) or of the launch (flags[1], which the host reports) has.
+template <bool CLUSTER>
 __device__ __noinline__ bool barrier_wait_slow(uint32_t a, uint32_t parity, int32_t volatile* gaveUp, int32_t* flags, long long ns)
 {
     unsigned long long const t0 = global_ns();
     for (;;)
     {
-        if (barrier_passed(a, parity))
+        if (barrier_passed<CLUSTER>(a, parity))
             return true;
         if (*gaveUp || *reinterpret_cast<int32_t const volatile*>(flags + 1) ||
             static_cast<long long>(global_ns() - t0) > ns)
@@ -91,10 +101,11 @@ __device__ __noinline__ bool barrier_wait_slow(uint32_t a, uint32_t parity, int3
     return false;
 }
 
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool barrier_wait(uint64_t* bar, uint32_t parity, int32_t volatile* gaveUp, int32_t* flags, long long ns)
 {
     uint32_t const a = shared_address(bar);
-    return barrier_passed(a, parity) || barrier_wait_slow(a, parity, gaveUp, flags, ns);
+    return barrier_passed<CLUSTER>(a, parity) || barrier_wait_slow<CLUSTER>(a, parity, gaveUp, flags, ns);
 }
 
 // When a wait gives up, the tile that did not arrive is never read and a barrier whose phase did not end is
@@ -190,7 +201,7 @@ __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_k
                 // No copy is on its way when the block ends, also when a wait gave up.
                 unsigned long long const t0 = global_ns();
                 for (int i = max(issued - p.stages, 0); i < issued; ++i)
-                    while (i != poison && !barrier_passed(shared_address(full + i % p.stages), uint32_t(i / p.stages) & 1u) &&
+                    while (i != poison && !barrier_passed<false>(shared_address(full + i % p.stages), uint32_t(i / p.stages) & 1u) &&
                            static_cast<long long>(global_ns() - t0) <= ns)
                         ;
             }
@@ -206,7 +217,9 @@ __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_k
     int const nOwned  = __ldg(p.partOwned + part);
     int const threads = 32 * warps;
     int const lane    = int(threadIdx.x) & (L - 1);
-    float4* const slab      = (CHEB ? B + p.ownedCapacity : B) + warp * p.slabPerWarp;
+    float4* const slabs     = CHEB ? B + p.ownedCapacity : B;
+    float4* const slab      = slabs + warp * p.slabPerWarp;
+    float4* const XT        = slabs + warps * p.slabPerWarp; // own, with damping: the substep's start
     int stage0 = 0;       // stage of the colour's first tile
     uint32_t round0 = 0u; // times the ring came round before it
     bool solving    = true; // the warp's (no wait gave up)
@@ -245,6 +258,8 @@ __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_k
                 sub.xt[i]     = make_float4(x4.x, x4.y, x4.z, m);
                 sub.xtilde[i] = target;
                 T[j]          = make_float4(target.x, target.y, target.z, m / p.sweep.h2);
+                if (p.sweep.kD != 0.f)
+                    XT[j] = x4;
             }
             X[j] = x0;
             if constexpr (CHEB)
@@ -369,7 +384,7 @@ __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_k
                         float const xl[3] = {t4.x, t4.y, t4.z};
                         float xt[3]       = {0.f, 0.f, 0.f};
                         if (p.sweep.kD != 0.f)
-                            load3(sub.xt[e0.x], xt);
+                            load3(XT[own], xt);
                         b.s = __int_as_float(e1.z);
                         float H[6], gr[3];
                         elastic_system(b, xt, xi, p.sweep.h, p.sweep.kD, H, gr);
@@ -426,7 +441,7 @@ __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_k
                 }
                 asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
                 if (CLUSTER && expects)
-                    barrier_wait(halo + c, phase, gaveUp, flags, ns);
+                    barrier_wait<true>(halo + c, phase, gaveUp, flags, ns);
             }
         }
 
@@ -493,7 +508,8 @@ void configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int warps, in
 
 size_t cluster_step_smem(ClusterStepParams const& p, int warps, bool chebyshev)
 {
-    size_t const positions = chebyshev ? 2 * size_t(p.localCapacity) + size_t(p.ownedCapacity) : size_t(p.localCapacity);
+    size_t const positions = (chebyshev ? 2 * size_t(p.localCapacity) + size_t(p.ownedCapacity) : size_t(p.localCapacity)) +
+                             (p.sweep.kD != 0.f ? size_t(p.ownedCapacity) : 0);
     return size_t(p.stages) * size_t(p.stageBytes) + 2 * (size_t(p.stages) + size_t(p.nColors)) * sizeof(uint64_t) +
            (positions + size_t(p.ownedCapacity) + size_t(p.slabPerWarp) * size_t(warps)) * sizeof(float4);
 }

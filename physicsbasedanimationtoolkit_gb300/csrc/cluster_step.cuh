@@ -20,9 +20,13 @@
 // it, follow every read of b's old position.  The same holds for the phase of a colour's barrier: bytes
 // of the next iteration are sent only after the block has passed this iteration's wait.
 //
-// Every wait has a time limit.  Asking for a tile as a warp costs a vote per group where tiles are streamed: a
-// 5,040-vertex Chebyshev step of 2 x 15 iterations 125 -> 130 us among others; steps whose tiles stay are
-// as fast as without the limit (1331 vertices 58.2 us, 27 vertices 24.1).
+// What a block reads from global memory inside a substep goes to L2 (the acquire of other blocks' positions
+// empties L1), so the positions damping needs are in shared memory too: a 5,040-vertex Chebyshev step of
+// 2 x 15 damped iterations takes 126 us with them, 137 us without.
+//
+// Every wait has a time limit.  Asking for a tile as a warp costs a vote per group where tiles are streamed, 4
+// to 5 us of that step; steps whose tiles stay are as fast as without the limit (1331 vertices 58.5 us, 27
+// vertices 23.6, among others).
 //
 // What bounds it: with a few solves per part and colour, the chain of one vertex solve (about 300
 // instructions of one warp, 0.8 us) times the colours; with many, shared memory (with three 16-byte reads per
@@ -101,6 +105,7 @@ int constexpr kClusterMaxStages = 64;
 int constexpr kClusterMaxLocal = 32767;
 // Dynamic shared memory of a block.
 size_t constexpr kClusterMaxBytes = 226 * 1024;
+// (with p.sweep.kD set)
 size_t cluster_step_smem(ClusterStepParams const& p, int warps, bool chebyshev);
 // Launches nMeshes clusters of `blocks` blocks.
 cudaError_t launch_cluster_step(ClusterStepParams const& p, int lanes, int warps, int blocks, int nMeshes, bool chebyshev, bool record, cudaStream_t s);

@@ -538,6 +538,7 @@ class VbdSystem
     struct ClusterLaunch
     {
         int32_t lanes = 0, warps = 0, slabPerWarp = 0, stages = 0, resident = 0, residentRecord = 0;
+        bool damped = false; // damping keeps more in shared memory
     } clusterLaunch;
     long long clusterWaitNs = kBatchWaitNs; // pbgb_debug_cluster_wait
     int32_t clusterPoison   = -1;
@@ -1088,6 +1089,7 @@ class VbdSystem
         p.slabPerWarp   = c.slabPerWarp;
         p.stages        = c.stages;
         p.stageBytes    = clusterStage;
+        p.sweep.kD      = kD;
         return p;
     }
 
@@ -1099,10 +1101,11 @@ class VbdSystem
             return false;
         bool const cheb = acceleration == PBGB_ACCEL_CHEBYSHEV;
         int const L     = lanesToUse();
-        if (clusterLaunch.lanes != L)
+        if (clusterLaunch.lanes != L || clusterLaunch.damped != (kD != 0.f))
         {
             ClusterLaunch c;
             c.lanes            = L;
+            c.damped           = kD != 0.f;
             c.warps            = std::clamp<int32_t>((clusterColor * L + 31) / 32, 4, kClusterMaxWarps);
             for (int2 const r : hostPartRange)
                 for (int32_t s = r.x; s < r.y; s += 32 / L)

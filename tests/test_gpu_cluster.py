@@ -174,3 +174,18 @@ def test_the_cluster_hook_rejects_out_of_range_limits():
     L = _capi.lib()
     for ns, tile in ((10, -1), (5_000_000_000, -1), (1_000_000, -2)):
         assert L.pbgb_debug_cluster_wait(I.handle, ns, tile) == 1
+
+
+@pytest.mark.parametrize("shape", [(4, 3, 3), (20, 20, 20)])
+def test_damping_switched_on_and_off(shape):
+    """The step's shared memory holds more with damping: a launch made without is not used with it."""
+    d = data_of(*shape, rho=0.85)
+    A, B = pbat.gpu.vbd.Integrator(d), pbat.gpu.vbd.Integrator(d)
+    set_persistent(B, False)
+    for kD in (0.0, 1e-3, 0.0, 1e-2):
+        for I in (A, B):
+            I.kD = kD
+            I.step(1 / 60, 5, 1)
+        np.testing.assert_array_equal(A.x, B.x)
+        np.testing.assert_array_equal(A.v, B.v)
+    assert A.launches_per_step(5, 1) == 1
