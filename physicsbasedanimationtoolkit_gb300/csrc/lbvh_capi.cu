@@ -11,6 +11,7 @@
 #include <exception>
 #include <new>
 #include <stdexcept>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -84,6 +85,7 @@ struct pbgb_bvh
     cudaStream_t stream       = nullptr;
     unsigned char* work = nullptr; // inputs of the *_columns calls, grown to the largest one
     size_t workBytes    = 0;
+    std::mutex workMutex; // held by such a call: several threads may query one hierarchy
     std::string error;
 
     ~pbgb_bvh()
@@ -124,7 +126,8 @@ struct pbgb_bvh
         ck(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     }
 
-    // At least `bytes` of device memory that only the calling entry point uses until it returns.
+    // At least `bytes` of device memory that only the calling entry point, which holds workMutex, uses until
+    // it returns.
     unsigned char* workspace(size_t bytes)
     {
         if (workBytes < bytes)
@@ -266,6 +269,7 @@ PBGB_API int pbgb_bvh_build_columns(pbgb_bvh* b, int32_t n, const float* lower, 
     if (n < 1 || n > b->capacity || !lower || !upper || !wmin || !wmax)
         return bvh_fail(b, PBGB_ERR_INVALID_ARGUMENT, "pbgb_bvh_build_columns: expected 1 <= n <= capacity and non-null boxes");
     return bvh_guard(b, [&] {
+        std::lock_guard<std::mutex> const lock(b->workMutex);
         size_t const bytes = sizeof(float) * 3 * size_t(n);
         Pieces at;
         size_t const l = at.add(bytes), u = at.add(bytes);
@@ -503,6 +507,7 @@ PBGB_API int pbgb_bvh_nearest_simplices_columns(
         return bvh_fail(b, PBGB_ERR_INVALID_ARGUMENT,
                         "pbgb_bvh_nearest_simplices_columns: expected the built BVH's simplices (nS = boxes), k = 3 or 4");
     return bvh_guard(b, [&] {
+        std::lock_guard<std::mutex> const lock(b->workMutex);
         size_t const xBytes = sizeof(float) * 3 * size_t(nq), pBytes = sizeof(float) * 3 * size_t(nP);
         size_t const sBytes = size_t(index_bytes) * size_t(nS) * size_t(k);
         Pieces at;

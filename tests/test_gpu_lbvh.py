@@ -3,6 +3,7 @@ overlap pair sets equal to brute force."""
 
 import json
 import pathlib
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import pytest
@@ -491,3 +492,28 @@ def test_wide_indices_are_checked_before_they_are_narrowed(itype, order, bad):
             call()
         assert err.value.code == 1 and "out of range" in str(err.value)
     np.testing.assert_array_equal(bvh.point_triangle_nearest_neighbours(boxes, P, P, F), nn)
+
+
+def test_threads_query_one_hierarchy():
+    """Queries of different sizes from several threads at once, each against its own points: every thread gets
+    what it gets alone."""
+    rng = np.random.default_rng(5)
+    n = 2000
+    P = (rng.uniform(-1, 1, (n, 1, 3)) + rng.uniform(-0.05, 0.05, (n, 3, 3))).reshape(-1, 3).astype(np.float32)
+    F = np.arange(3 * n).reshape(n, 3)
+    boxes, bvh = boxes_and_tree(P, F)
+    V, S = np.ascontiguousarray(P.T), np.ascontiguousarray(F.T)
+    queries = [rng.uniform(-1, 1, (3, m)).astype(np.float32) for m in (1, 700, 5000, 60, 20000, 333, 9000, 2500)]
+    # A hierarchy each for the answers; the one that is shared has no workspace yet and grows it while others query.
+    expected = []
+    for q in queries:
+        _, own = boxes_and_tree(P, F)
+        expected.append(own.point_triangle_nearest_neighbours(boxes, q, V, S))
+
+    def work(k):
+        return [bvh.point_triangle_nearest_neighbours(boxes, queries[k], V, S) for _ in range(20)]
+
+    with ThreadPoolExecutor(len(queries)) as pool:
+        for k, out in enumerate(pool.map(work, range(len(queries)))):
+            for nn in out:
+                np.testing.assert_array_equal(nn, expected[k])
