@@ -1773,6 +1773,8 @@ class VbdSystem
         std::copy(mu, mu + nT, hostMu.begin());
         std::copy(lambda, lambda + nT, hostLambda.begin());
         uploadMaterial();
+        // The uploads read hostMu and hostLambda, which the next call writes.
+        check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     }
 
     void adjointReserve(int32_t slots, int32_t iterations)

@@ -3,6 +3,7 @@
 Tolerance: positions within 1e-4 of the bounding-box diagonal after the configured steps (FP32
 device arithmetic against the FP64 oracle on the same mesh, colouring and iteration count)."""
 
+import ctypes as C
 import json
 import pathlib
 
@@ -324,3 +325,20 @@ def test_staged_sweep_batched_and_recorded():
         C.step(1 / 60, 9, 1)
         D.step_record(1 / 60, 9, 1, 0)
     np.testing.assert_array_equal(C.x, D.x)
+
+
+def test_set_material_returns_with_its_uploads_done():
+    """The header says that the call synchronizes: the handle keeps the coefficients on the host, and a second
+    call writes them, so an upload must not be under way when the first returns."""
+    torch = pytest.importorskip("torch")
+    X, T = meshgen.hex_grid(40, 30, 30, hi=(4.0, 3.0, 3.0))
+    mu, lam = meshgen.lame(np.full(T.shape[0], 1e6), np.full(T.shape[0], 0.45))
+    d = (pbat.sim.vbd.Data().with_volume_mesh(X.T, T.T).with_material(np.full(T.shape[0], 1000.0), mu, lam)
+         .with_dirichlet_vertices(meshgen.face_vertices(X, 0, 0.0)).construct())
+    I = pbat.gpu.vbd.Integrator(d)
+    s = C.c_void_p()
+    _capi.check(_capi.lib().pbgb_vbd_stream(I.handle, C.byref(s)), I.handle)
+    stream = torch.cuda.ExternalStream(s.value)
+    for k in range(5):
+        I.set_material(mu * (1 + k), lam * (1 + k))
+        assert stream.query()
