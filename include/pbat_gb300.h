@@ -518,6 +518,11 @@ PBGB_API int pbgb_debug_batched_wait(pbgb_vbd* h, int64_t wait_ns, int32_t poiso
  * none). */
 PBGB_API int pbgb_debug_cluster_wait(pbgb_vbd* h, int64_t wait_ns, int32_t poison_tile);
 
+/* Test hook of the handles' memory limits: the allocation of device memory that a call of this thread on
+ * an integrator makes after `after` others fails on the host, as if there were no room (-1: none; one
+ * failure at most).  left (may be NULL): what was left of the last setting, -1 once it failed. */
+PBGB_API int pbgb_debug_fail_allocation(int64_t after, int64_t* left);
+
 /* Host self-check of the closed-form vertex block (FP64): accumulates n incident tets and
  * applies damping, inertia and the Newton step exactly like the device sweep.  Arguments as the
  * oracle's per-vertex solve: xe n x 12 (3x4 column-major per tet), GPs n x 12 (row-major 4x3). */

@@ -54,6 +54,9 @@ inline void check(cudaError_t e, char const* what)
         throw CudaFailure{e, what};
 }
 
+// pbgb_debug_fail_allocation: allocations of this thread until one fails, -1: none does.
+thread_local int64_t gAllocationsLeft = -1;
+
 template <class T>
 class DeviceArray
 {
@@ -65,9 +68,14 @@ class DeviceArray
     void allocate(size_t n)
     {
         release();
-        n_ = n;
         if (n > 0)
-            check(cudaMalloc(reinterpret_cast<void**>(&p_), n * sizeof(T)), "cudaMalloc");
+        {
+            bool const fails = gAllocationsLeft == 0;
+            if (gAllocationsLeft >= 0)
+                --gAllocationsLeft;
+            check(fails ? cudaErrorMemoryAllocation : cudaMalloc(reinterpret_cast<void**>(&p_), n * sizeof(T)), "cudaMalloc");
+        }
+        n_ = n;
     }
     void upload(T const* h, size_t n, cudaStream_t s)
     {
@@ -487,7 +495,7 @@ class VbdSystem
     DeviceArray<double> adjMu, adjLa;
 
     // Reversed substeps of small meshes (AdjointChain): the lists, made at the first
-    // pbgb_vbd_adjoint_reserve (chainEdges = -1: not yet, 0: none), and the workspace of chainSpan iterations.
+    // pbgb_vbd_adjoint_reserve (chainEdges = -1: not yet or no room, 0: none), and the workspace of chainSpan iterations.
     int32_t chainEdges = -1, chainSpan = 0, chainGroups = 0;
     size_t chainSmem = 0;
     DeviceArray<int32_t> chainEdgePtr, chainPlace, chainTetPtr, chainGatherPtr, chainGatherMid, chainGather, chainEntry, chainColor, chainFixed, chainGatherAt;
@@ -1786,6 +1794,8 @@ class VbdSystem
             return;
         check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
         dropSlotGraphs();
+        // No slots until every array is there: one that does not fit leaves a tape that refuses every step.
+        tapeSlots = tapeIters = 0;
         adjX.allocate(size_t(nV) * 3);
         adjV.allocate(size_t(nV) * 3);
         adjP.allocate(size_t(nV) * 3);
@@ -1828,6 +1838,14 @@ class VbdSystem
         chainOmega.release();
     }
 
+    // Passes over an allocation that found no room, and over nothing else.
+    static void noRoom(CudaFailure const& e)
+    {
+        if (e.err != cudaErrorMemoryAllocation)
+            throw e;
+        cudaGetLastError();
+    }
+
     void reserveAdjointChain(int32_t iterations)
     {
         releaseAdjointChain();
@@ -1835,7 +1853,7 @@ class VbdSystem
             return;
         if (chainEdges < 0)
             buildAdjointChain();
-        if (chainEdges == 0)
+        if (chainEdges <= 0)
             return;
         size_t const perIteration = size_t(chainEdges) * 36 + size_t(nFree) * 48;
         int32_t const span        = int32_t(std::clamp<size_t>(kAdjointChainBytes / perIteration, 1, size_t(std::min(iterations, 65535))));
@@ -1848,11 +1866,10 @@ class VbdSystem
             chainW.allocate(size_t(iterations) * size_t(nFree));
             chainOmega.allocate(size_t(iterations));
         }
-        catch (std::exception const&)
+        catch (CudaFailure const& e)
         {
-            // No room: the sweeps with atomics need none.
-            cudaGetLastError();
             releaseAdjointChain();
+            noRoom(e); // the sweeps with atomics need none
             return;
         }
         std::vector<float> om(static_cast<size_t>(iterations));
@@ -1983,12 +2000,13 @@ class VbdSystem
             put(chainColor, colorPtr);
             put(chainFixed, fixed);
         }
-        catch (std::exception const&)
+        catch (CudaFailure const& e)
         {
-            cudaGetLastError();
             for (auto* a : {&chainEdgePtr, &chainPlace, &chainTetPtr, &chainGatherPtr, &chainGatherMid, &chainGather, &chainEntry, &chainColor, &chainFixed, &chainGatherAt})
                 a->release();
             chainCode.release();
+            noRoom(e);
+            chainEdges = -1; // the next reservation tries again
             return;
         }
         chainEdges = int32_t(to.size());
@@ -3867,6 +3885,16 @@ PBGB_API int pbgb_debug_cluster_wait(pbgb_vbd* h, int64_t wait_ns, int32_t poiso
     h->sys.clusterWaitNs = wait_ns;
     h->sys.clusterPoison = poison_tile;
     h->sys.invalidate();
+    return kOk;
+}
+
+PBGB_API int pbgb_debug_fail_allocation(int64_t after, int64_t* left)
+{
+    if (after < -1)
+        return fail(nullptr, kInvalid, "pbgb_debug_fail_allocation: expected after >= -1");
+    if (left)
+        *left = pbgb::gAllocationsLeft;
+    pbgb::gAllocationsLeft = after;
     return kOk;
 }
 

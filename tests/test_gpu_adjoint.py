@@ -5,6 +5,8 @@ differentiation beam (40 x 10 x 10 hexes, 30 steps of 20 iterations, dt = 1/60, 
 directions, eps = 1e-5), with KineticEnergyMinimum and with the reference Data's default initial
 guess, AdaptivePbat."""
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -280,3 +282,47 @@ def test_rollouts_recorded_on_one_integrator_before_their_backward(every, iterat
     loss.backward()
     for a, b in zip(gradients(leaves), alone[0]):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("rho", [None, 0.85])
+def test_a_reservation_without_room(rho):
+    """Every allocation of a reservation fails in turn.  The tape's: the call says so, recording is refused and a
+    second reservation works.  The reversed chain's: the call succeeds, and the sweeps that need no workspace
+    give the same gradients."""
+    w = meshgen.adjoint_beam_workload(nx=5, ny=2, nz=2)
+    extra = dict() if rho is None else dict(rho_chebyshev=rho)
+    mu, lam = meshgen.lame(np.exp(w["logE"]), np.full(w["T"].shape[0], w["nu"]))
+    L = _capi.lib()
+
+    def gradients(I):
+        leaves = [torch.tensor(mu, requires_grad=True), torch.tensor(lam, requires_grad=True),
+                  torch.tensor(w["X"], dtype=torch.float32, device="cuda", requires_grad=True),
+                  torch.ones(w["X"].shape, dtype=torch.float32, device="cuda", requires_grad=True)]
+        x, v = pbat.gpu.vbd.rollout(I, *leaves, dt=1 / 60, iterations=4, steps=2)
+        ((x ** 2).sum() + (v ** 2).sum()).backward()
+        return [a.grad.cpu().numpy() for a in leaves]
+
+    expected = gradients(gpu_integrator(w, **extra))
+    tape = 12 if rho is None else 15  # arrays of the tape and the adjoints; the chain's follow
+    left, k = C.c_int64(), 0
+    while True:
+        I = gpu_integrator(w, **extra)
+        _capi.check(L.pbgb_debug_fail_allocation(k, None))
+        rc = L.pbgb_vbd_adjoint_reserve(I.handle, 2, 4)
+        _capi.check(L.pbgb_debug_fail_allocation(-1, C.byref(left)))
+        if left.value >= 0:
+            assert rc == 0  # nothing was left to fail
+            break
+        if k < tape:
+            assert rc != 0
+            with pytest.raises(_capi.PbgbError):
+                I.step_record(1 / 60, 4, 1, 0)
+            with pytest.raises(_capi.PbgbError):
+                I.step_record(1 / 60, 0, 1, 0)
+            I.adjoint_reserve(2, 4)
+        else:
+            assert rc == 0
+        for a, b in zip(gradients(I), expected):
+            assert rel(a, b) <= 1e-4
+        k += 1
+    assert k > tape + 10
