@@ -108,7 +108,7 @@ int ccd_flags(pbgb_ccd* c)
     cc(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
     if (f)
     {
-        cc(cudaMemset(c->S.flags, 0, sizeof(int32_t)), "cudaMemset");
+        cc(cudaMemsetAsync(c->S.flags, 0, sizeof(int32_t), c->stream), "cudaMemsetAsync");
         return ccd_fail(c, PBGB_ERR_INTERNAL, "BVH traversal stack overflow or tree deeper than 64 levels");
     }
     return PBGB_OK;
@@ -175,6 +175,8 @@ PBGB_API int pbgb_ccd_create(int32_t nV, int32_t nSurfV, const int32_t* V, int32
         cc(cudaMemset(S.nActive, 0, sizeof(int32_t)), "cudaMemset");
         cc(cudaMemset(S.nn, 0xFF, sizeof(int32_t) * size_t(nSurfV > 0 ? nSurfV : 1) * pbgb::kMaxContacts), "cudaMemset");
         cc(cudaMemset(S.fc, 0xFF, sizeof(int32_t) * size_t(nV) * pbgb::kMaxContacts), "cudaMemset");
+        // The default stream's copies and fills end before this (non-blocking) stream's kernels read them.
+        cc(cudaStreamSynchronize(cudaStreamLegacy), "cudaStreamSynchronize");
         c->M = pbgb::ContactMesh{nV, nSurfV, nF, c->V, c->F, c->B};
         return int(PBGB_OK);
     });

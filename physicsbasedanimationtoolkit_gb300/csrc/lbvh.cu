@@ -928,6 +928,8 @@ cudaError_t bvh_allocate(BvhBuffers& B, int32_t capacity)
     get(B.flags, 1);
     if (e == cudaSuccess)
         e = cudaMemset(B.flags, 0, sizeof(int32_t));
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(cudaStreamLegacy); // ordered before no other stream
     return e;
 }
 

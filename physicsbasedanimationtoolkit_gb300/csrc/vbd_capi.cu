@@ -1066,10 +1066,6 @@ class VbdSystem
             hVertex.insert(hVertex.end(), local[size_t(q)].begin(), local[size_t(q)].end());
             hPtr[q + 1] = int32_t(hVertex.size());
         }
-        auto put = [&](auto& array, auto const& host) {
-            array.allocate(host.size());
-            array.upload(host.data(), host.size(), stream);
-        };
         put(partPtr, hPtr);
         put(partOwned, owned);
         put(partVertex, hVertex);
@@ -1078,7 +1074,6 @@ class VbdSystem
         put(clusterTile, hTile);
         put(tileData, hData);
         put(tileAt, hAt);
-        check(cudaStreamSynchronize(stream), "cudaStreamSynchronize"); // the uploads read local arrays
         return true;
     }
 
@@ -1150,6 +1145,29 @@ class VbdSystem
                (acceleration == PBGB_ACCEL_TRUST_REGION && trCurved);
     }
 
+    // Chebyshev weights of the first iterations (at least one entry).
+    std::vector<float> chebyshevWeights(int32_t iterations) const
+    {
+        std::vector<float> om(size_t(std::max(iterations, 1)), 1.f);
+        double omega = 0.0;
+        for (int32_t k = 0; k < iterations; ++k)
+        {
+            omega         = chebyshev_omega<double>(k, rho * rho, omega, chebFormula);
+            om[size_t(k)] = float(omega);
+        }
+        return om;
+    }
+
+    // The array with the host's contents, on the handle's stream: a copy on the default stream may still be
+    // under way when it returns, and nothing would order it before this (non-blocking) stream's kernels.
+    template <class T>
+    void put(DeviceArray<T>& array, std::vector<T> const& host)
+    {
+        array.allocate(host.size());
+        array.upload(host.data(), host.size(), stream);
+        check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+    }
+
     // The same, with the Chebyshev weights of at least `iterations` on the device.
     bool prepareCluster(int32_t iterations, bool record)
     {
@@ -1158,16 +1176,9 @@ class VbdSystem
         if (acceleration == PBGB_ACCEL_CHEBYSHEV && omegaIterations < iterations)
         {
             check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-            std::vector<float> om(size_t(std::max(iterations, 1)), 1.f);
-            double omega = 0.0;
-            for (int32_t k = 0; k < iterations; ++k)
-            {
-                omega         = chebyshev_omega<double>(k, rho * rho, omega, chebFormula);
-                om[size_t(k)] = float(omega);
-            }
             invalidate(); // captured graphs hold the array's address
-            stepOmega.allocate(om.size());
-            check(cudaMemcpy(stepOmega.get(), om.data(), sizeof(float) * om.size(), cudaMemcpyHostToDevice), "H2D");
+            omegaIterations = -1; // none, should the allocation fail
+            put(stepOmega, chebyshevWeights(iterations));
             omegaIterations = iterations;
         }
         return true;
@@ -1694,7 +1705,7 @@ class VbdSystem
             cRec.allocate(size_t(nV) * kMaxContacts);
             cPen.allocate(size_t(nV) * kMaxContacts);
             cCount.allocate(size_t(nV));
-            check(cudaMemset(cCount.get(), 0, sizeof(int32_t) * size_t(nV)), "cudaMemset");
+            check(cudaMemsetAsync(cCount.get(), 0, sizeof(int32_t) * size_t(nV), stream), "cudaMemsetAsync");
             check(bvh_allocate(cstate.bvh, nF), "cudaMalloc");
             cV.upload(hV.data(), nS, stream);
             cF.upload(hF.data(), nF, stream);
@@ -1864,7 +1875,7 @@ class VbdSystem
             chainBlock2.allocate(size_t(span) * size_t(chainEdges));
             chainOwn.allocate(size_t(span) * size_t(nFree) * 3);
             chainW.allocate(size_t(iterations) * size_t(nFree));
-            chainOmega.allocate(size_t(iterations));
+            put(chainOmega, chebyshevWeights(iterations));
         }
         catch (CudaFailure const& e)
         {
@@ -1872,14 +1883,6 @@ class VbdSystem
             noRoom(e); // the sweeps with atomics need none
             return;
         }
-        std::vector<float> om(static_cast<size_t>(iterations));
-        double omega = 0.0;
-        for (int32_t k = 0; k < iterations; ++k)
-        {
-            omega         = chebyshev_omega<double>(k, rho * rho, omega, chebFormula);
-            om[size_t(k)] = float(omega);
-        }
-        check(cudaMemcpy(chainOmega.get(), om.data(), sizeof(float) * om.size(), cudaMemcpyHostToDevice), "H2D");
         chainSpan = span;
     }
 
@@ -1981,11 +1984,6 @@ class VbdSystem
                 gather[place[n]]   = s;
                 gatherAt[place[n]] = held[s];
             }
-        auto put = [&](auto& array, auto const& host) {
-            array.allocate(host.size());
-            if (!host.empty())
-                check(cudaMemcpy(array.get(), host.data(), sizeof(host[0]) * host.size(), cudaMemcpyHostToDevice), "H2D");
-        };
         try
         {
             put(chainEdgePtr, edgePtr);
@@ -2256,15 +2254,7 @@ class VbdSystem
         int const L     = launchLanes();
         bool const cheb = acceleration == PBGB_ACCEL_CHEBYSHEV;
         // Chebyshev weights of the iterations, as the forward formed them.
-        std::vector<float> om(size_t(std::max(tapeIters, 1)), 1.f);
-        {
-            double omega = 0.0;
-            for (int32_t k = 0; k < tapeIters; ++k)
-            {
-                omega         = chebyshev_omega<double>(k, rho * rho, omega, chebFormula);
-                om[size_t(k)] = float(omega);
-            }
-        }
+        std::vector<float> const om = chebyshevWeights(tapeIters);
         for (int32_t s = substeps - 1; s >= 0; --s)
         {
             int32_t const slot = slot0 + s;
@@ -2444,20 +2434,9 @@ class VbdSystem
             items[i].b.z = before[b] + iterations * perIteration[b] + count[b];
         }
         check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-        batchItems.allocate(std::max<size_t>(items.size(), 1));
-        if (!items.empty())
-            check(cudaMemcpy(batchItems.get(), items.data(), sizeof(BatchItemWords) * items.size(), cudaMemcpyHostToDevice),
-                  "H2D");
+        put(batchItems, items);
         batchCounters.allocate((2 + size_t(nMeshes)) * kBatchWordStride);
-        std::vector<float> om(size_t(std::max(iterations, 1)), 1.f);
-        double omega = 0.0;
-        for (int32_t k = 0; k < iterations; ++k)
-        {
-            omega          = chebyshev_omega<double>(k, rho * rho, omega, chebFormula);
-            om[size_t(k)] = float(omega);
-        }
-        batchOmega.allocate(om.size());
-        check(cudaMemcpy(batchOmega.get(), om.data(), sizeof(float) * om.size(), cudaMemcpyHostToDevice), "H2D");
+        put(batchOmega, chebyshevWeights(iterations));
         plan.nBegin = int32_t(nBegin);
         plan.nSweep = int32_t(nSweep);
         plan.nEnd   = int32_t(nEnd);

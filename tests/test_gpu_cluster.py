@@ -189,3 +189,33 @@ def test_damping_switched_on_and_off(shape):
         np.testing.assert_array_equal(A.x, B.x)
         np.testing.assert_array_equal(A.v, B.v)
     assert A.launches_per_step(5, 1) == 1
+
+
+def test_chebyshev_weights_of_many_iterations():
+    """The weights of a longer step are on the device before its kernel reads them (80 KB: more than a copy from
+    pageable memory stages at once): the first such step equals a later one."""
+    d = data_of(2, 2, 2, rho=0.9, strategy=2)
+    I = pbat.gpu.vbd.Integrator(d)
+    x0, v0 = I.x, I.v
+    out = []
+    for _ in range(2):
+        I.x, I.v = x0, v0
+        I.step(1 / 60, 20000, 1)
+        out.append((I.x, I.v))
+    np.testing.assert_array_equal(out[0], out[1])
+
+
+def test_a_step_whose_weights_find_no_room():
+    """The call says so; the next one makes the weights again, also a shorter step that the lost ones covered."""
+    d = data_of(3, 3, 3, rho=0.9, strategy=2)
+    A, B = pbat.gpu.vbd.Integrator(d), pbat.gpu.vbd.Integrator(d)
+    L = _capi.lib()
+    for I in (A, B):
+        I.step(1 / 60, 10, 1)
+    _capi.check(L.pbgb_debug_fail_allocation(0, None))
+    with pytest.raises(_capi.PbgbError):
+        A.step(1 / 60, 20, 1)
+    for n in (5, 30):
+        for I in (A, B):
+            I.step(1 / 60, n, 1)
+        np.testing.assert_array_equal(A.x, B.x)
