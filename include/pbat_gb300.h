@@ -231,9 +231,11 @@ PBGB_API int pbgb_vbd_set_block_size(pbgb_vbd* h, int32_t block_size);
 /* Lanes cooperating on one vertex: 1, 2, 4, 8, 16 or 32 (0 = by size, or autotuned). */
 PBGB_API int pbgb_vbd_set_lanes_per_vertex(pbgb_vbd* h, int32_t lanes);
 /* Autotuner: times one step of (dt, iterations, substeps) for every lanes-per-vertex in
- * {1,2,4,8,16,32} x block size in {64,128,256}, keeps the fastest for this handle and caches it per
- * size bucket (vertex and tet counts rounded up to powers of two, colours, iterations).  The
- * handle's positions and velocities are restored after each trial.  Outputs may be NULL. */
+ * {1,2,4,8,16,32} x block size in {64,96,128,160,192,224,256}, keeps the fastest for this handle and caches it
+ * per size bucket (vertex and tet counts rounded up to powers of two, colours, iterations) and path.  A step
+ * that runs in thread-block clusters has only lanes to choose: they are kept for such steps, and the handle's
+ * block size (returned) and its reversed sweeps stay as they were.  The handle's positions and velocities are
+ * restored after each trial.  Outputs may be NULL. */
 PBGB_API int pbgb_vbd_autotune(
     pbgb_vbd* h,
     float dt,

@@ -550,6 +550,7 @@ class VbdSystem
     } clusterLaunch;
     long long clusterWaitNs = kBatchWaitNs; // pbgb_debug_cluster_wait
     int32_t clusterPoison   = -1;
+    int32_t clusterLanes    = 0;     // autotuned lanes of the cluster step; 0: by `lanes`
     bool stepInCluster      = false; // the last step ran (or is being captured) as a cluster launch
     int32_t omegaIterations = -1; // iterations stepOmega holds the Chebyshev weights of
     DeviceArray<float> stepOmega;
@@ -690,6 +691,8 @@ class VbdSystem
     // for bit.
     int lanesToUse() const
     {
+        if (clusterLanes > 0)
+            return clusterLanes;
         if (lanes > 0)
             return lanes;
         return clusterBlocks > 0 ? clusterDefaultLanes() : launchLanes();
@@ -1096,11 +1099,17 @@ class VbdSystem
         return p;
     }
 
+    // Whether steps of colour sweeps alone run in clusters where the launch for the current lanes fits.
+    bool clusterWanted() const
+    {
+        return clusterBlocks > 0 && stagedOk && staged && persistent && !profiling && !(nMeshes > 1 && batchPoison >= 0);
+    }
+
     // Makes the cluster step's launch for the current lanes (outside any stream capture).  False: the
     // system takes the other paths.
     bool prepareClusterLaunch(bool record)
     {
-        if (clusterBlocks < 1 || !stagedOk || !staged || !persistent || profiling || (nMeshes > 1 && batchPoison >= 0))
+        if (!clusterWanted())
             return false;
         bool const cheb = acceleration == PBGB_ACCEL_CHEBYSHEV;
         int const L     = lanesToUse();
@@ -3064,25 +3073,42 @@ class VbdSystem
 
     // Project-written autotuner: times one replayed step per candidate (lanes per vertex x block
     // size) with CUDA events on the handle's stream, restoring the state after each candidate, and
-    // keeps the fastest.  Results are cached per (vertices, tets, colours) bucket.
+    // keeps the fastest.  Results are cached per (vertices, tets, colours) bucket and path: what is fastest
+    // in clusters says nothing of launches per colour, and meshes of one bucket lie on both sides of the line
+    // between them.
     struct TuneKey
     {
         int64_t nV, nT, nC, iters, sub;
         int32_t accel;
         bool contact;
-        bool persistent;
+        int32_t path; // 0: launches per colour, -1: the persistent batch, else clusters of so many blocks
         bool operator==(TuneKey const& o) const
         {
             return nV == o.nV && nT == o.nT && nC == o.nC && iters == o.iters && sub == o.sub && accel == o.accel &&
-                   contact == o.contact && persistent == o.persistent;
+                   contact == o.contact && path == o.path;
         }
     };
     struct TuneEntry
     {
         TuneKey key;
-        int32_t lanes, block;
+        int32_t lanes, block; // block 0: clusters, which size their own
         float ms;
     };
+    // The lanes of a step in clusters are kept apart from those of the launches, which the reversed sweeps of
+    // the same handle take with the block size it had.
+    void useTuned(TuneEntry const& e, int32_t* bestLanes, int32_t* bestBlock, float* bestMs)
+    {
+        clusterLanes = e.block > 0 ? 0 : e.lanes;
+        if (e.block > 0)
+        {
+            lanes = e.lanes;
+            block = e.block;
+        }
+        invalidate();
+        *bestLanes = e.lanes;
+        *bestBlock = block;
+        *bestMs    = e.ms;
+    }
     static std::vector<TuneEntry>& tuneCache()
     {
         static std::vector<TuneEntry> cache;
@@ -3099,18 +3125,17 @@ class VbdSystem
                 b <<= 1;
             return b;
         };
-        TuneKey const key{bucket(nV), bucket(nT), nColors, iterations, substeps, acceleration, contact, persistentActive()};
+        bool const savedProfiling = profiling;
+        profiling                 = false; // the candidates are timed without
+        TuneKey const key{bucket(nV), bucket(nT), nColors, iterations, substeps, acceleration, contact,
+                          plainForm(iterations) && clusterWanted() ? clusterBlocks : (persistentActive() ? -1 : 0)};
+        profiling = savedProfiling;
         {
             std::lock_guard<std::mutex> lock(cacheMutex);
             for (auto const& e : tuneCache())
                 if (e.key == key)
                 {
-                    lanes = e.lanes;
-                    block = e.block;
-                    invalidate();
-                    *bestLanes = e.lanes;
-                    *bestBlock = e.block;
-                    *bestMs    = e.ms;
+                    useTuned(e, bestLanes, bestBlock, bestMs);
                     return;
                 }
         }
@@ -3137,11 +3162,16 @@ class VbdSystem
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         check(cudaEventCreate(&e0), "cudaEventCreate");
         check(cudaEventCreate(&e1), "cudaEventCreate");
-        int32_t const savedLanes = lanes, savedBlock = block;
-        bool const savedProfiling = profiling;
-        profiling = false;
-        float best = -1.f;
-        int32_t bl = lanesToUse(), bb = block;
+        int32_t const savedLanes = lanes, savedBlock = block, savedCluster = clusterLanes;
+        profiling    = false;
+        clusterLanes = 0; // the candidates' lanes
+        TuneEntry best{key, 0, 0, -1.f};
+        auto const reset = [&] {
+            lanes        = savedLanes;
+            block        = savedBlock;
+            clusterLanes = savedCluster;
+            profiling    = savedProfiling;
+        };
         try
         {
             int32_t const laneSet[]  = {1, 2, 4, 8, 16, 32};
@@ -3152,10 +3182,10 @@ class VbdSystem
                 for (int32_t B : blockSet)
                 {
                     lanes = L;
-                    // The cluster step sizes its own blocks.
-                    if (plainForm(iterations) && prepareClusterLaunch(false) && B != 256)
-                        continue;
                     block = B;
+                    bool const cluster = plainForm(iterations) && prepareClusterLaunch(false);
+                    if (cluster && B != blockSet[0])
+                        continue;
                     invalidate();
                     step(dt, iterations, substeps); // capture + warm-up
                     restore();
@@ -3173,19 +3203,13 @@ class VbdSystem
                         check(cudaEventElapsedTime(&t, e0, e1), "cudaEventElapsedTime");
                         ms = ms < 0.f || t < ms ? t : ms;
                     }
-                    if (best < 0.f || ms < best)
-                    {
-                        best = ms;
-                        bl   = L;
-                        bb   = B;
-                    }
+                    if (best.ms < 0.f || ms < best.ms)
+                        best = TuneEntry{key, L, cluster ? 0 : B, ms};
                 }
         }
         catch (...)
         {
-            lanes     = savedLanes;
-            block     = savedBlock;
-            profiling = savedProfiling;
+            reset();
             invalidate();
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
@@ -3196,17 +3220,12 @@ class VbdSystem
         cudaEventDestroy(e1);
         check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
         check(cudaMemsetAsync(flags.get(), 0, sizeof(int32_t), stream), "cudaMemsetAsync");
-        lanes     = bl;
-        block     = bb;
-        profiling = savedProfiling;
-        invalidate();
+        reset();
         {
             std::lock_guard<std::mutex> lock(cacheMutex);
-            tuneCache().push_back(TuneEntry{key, bl, bb, best});
+            tuneCache().push_back(best);
         }
-        *bestLanes = bl;
-        *bestBlock = bb;
-        *bestMs    = best;
+        useTuned(best, bestLanes, bestBlock, bestMs);
     }
 
     int synchronize()
@@ -3754,7 +3773,8 @@ PBGB_API int pbgb_vbd_set_lanes_per_vertex(pbgb_vbd* h, int32_t lanes)
         return fail(nullptr, kInvalid, "null handle");
     if (lanes != 0 && lanes != 1 && lanes != 2 && lanes != 4 && lanes != 8 && lanes != 16 && lanes != 32)
         return fail(h, kInvalid, "lanes per vertex must be 0, 1, 2, 4, 8, 16 or 32");
-    h->sys.lanes = lanes;
+    h->sys.lanes        = lanes;
+    h->sys.clusterLanes = 0;
     h->sys.invalidate();
     return kOk;
 }

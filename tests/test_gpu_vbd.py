@@ -342,3 +342,41 @@ def test_set_material_returns_with_its_uploads_done():
     for k in range(5):
         I.set_material(mu * (1 + k), lam * (1 + k))
         assert stream.query()
+
+
+def grid_integrator(nx, ny, nz):
+    X, T = meshgen.hex_grid(nx, ny, nz, hi=(nx / nz, ny / nz, 1.0))
+    mu, lam = meshgen.lame(np.full(T.shape[0], 1e6), np.full(T.shape[0], 0.45))
+    d = (pbat.sim.vbd.Data().with_volume_mesh(X.T, T.T).with_material(np.full(T.shape[0], 1000.0), mu, lam)
+         .with_dirichlet_vertices(meshgen.face_vertices(X, 0, 0.0)).construct())
+    return pbat.gpu.vbd.Integrator(d)
+
+
+def test_autotuned_launches_are_those_of_the_path_that_was_timed():
+    """Two meshes of one size bucket, one stepping in a cluster and one in launches per colour, and one mesh with
+    the cluster step switched off: the paths are timed by themselves, and a step in a cluster leaves the
+    handle's block size alone."""
+    args = (1 / 60, 7, 1)
+    A, B, A2 = grid_integrator(21, 19, 19), grid_integrator(24, 20, 20), grid_integrator(21, 19, 19)
+    _capi.check(_capi.lib().pbgb_vbd_set_persistent(A2.handle, 0), A2.handle)
+    for I, J in ((A, B), (A, A2)):
+        assert int(np.ceil(np.log2(I.n_vertices))) == int(np.ceil(np.log2(J.n_vertices)))
+    out = {k: I.autotune(*args) for k, I in (("A", A), ("B", B), ("A2", A2))}
+    assert A.launches_per_step(7, 1) == 1 and B.launches_per_step(7, 1) > 1 and A2.launches_per_step(7, 1) > 1
+    # Both launch per colour and share the bucket; the cluster's entry is neither's.
+    assert out["A2"] == out["B"] and out["A"][2] != out["B"][2]
+    assert out["A"][1] == 128  # the default of one mesh
+    for k, I in (("A", A), ("B", B), ("A2", A2)):
+        assert I.autotune(*args) == out[k]
+    # The same positions on either path with the same lanes, tuned or set.
+    U = grid_integrator(21, 19, 19)
+    U.lanes_per_vertex = out["A"][0]
+    _capi.check(_capi.lib().pbgb_vbd_set_persistent(U.handle, 0), U.handle)
+    for I in (A, U):
+        I.step(1 / 60, 7, 1)
+    np.testing.assert_array_equal(A.x, U.x)
+    # Lanes set by hand replace the tuned ones.
+    for I in (A, U):
+        I.lanes_per_vertex = 2
+        I.step(1 / 60, 7, 1)
+    np.testing.assert_array_equal(A.x, U.x)
