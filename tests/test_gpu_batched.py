@@ -142,3 +142,21 @@ def test_ticket_kernel_equals_colour_launches(rho, lanes, block, tile, iteration
     assert P.launches_per_step(iterations, substeps) == 1
     np.testing.assert_array_equal(P.x, U.x)
     np.testing.assert_array_equal(P.v, U.v)
+
+
+@pytest.mark.parametrize("rho", [None, 0.9])
+def test_ticket_kernel_matches_oracle_per_mesh(rho):
+    """Batches of this size step in clusters; the hook (no item has that number) leaves them the ticket kernel."""
+    meshes = meshgen.batch_workload(n_meshes=12, nmin=3, nmax=10, seed=21)
+    B = pbat.gpu.vbd.BatchedIntegrator(make_datas(meshes, rho))
+    _capi.check(_capi.lib().pbgb_debug_batched_wait(B.handle, 2_000_000_000, 2**30), B.handle)
+    for _ in range(5):
+        B.step(1 / 60, 20, 1)
+    assert B.launches_per_step(20, 1) == 1
+    x, off = B.x, B.vertex_offsets
+    for b, m in enumerate(meshes):
+        R = O.OracleVbd(m["X"], m["T"], m["rho"], m["mu"], m["lam"], m["dbc"], v=m["v"], strategy=4, semantics=1,
+                        rho_chebyshev=rho)
+        R.step(1 / 60, 20, 1, 5)
+        diag = np.linalg.norm(m["X"].max(0) - m["X"].min(0))
+        assert np.abs(x[:, off[b]: off[b + 1]].T.astype(np.float64) - R.x).max() / diag <= TOL
