@@ -1524,9 +1524,10 @@ class VbdSystem
         stagedOk = true;
         {
             int32_t const ranges = std::clamp<int32_t>(nFree / 300, 1, std::clamp<int32_t>(int32_t(std::thread::hardware_concurrency()), 1, 8));
+            // (Deferred: run here, where no further thread can be had.)
             std::vector<std::future<Range>> rest;
             for (int32_t k = 1; k < ranges; ++k)
-                rest.push_back(std::async(std::launch::async, lists, int32_t(int64_t(nFree) * k / ranges), int32_t(int64_t(nFree) * (k + 1) / ranges)));
+                rest.push_back(std::async(std::launch::async | std::launch::deferred, lists, int32_t(int64_t(nFree) * k / ranges), int32_t(int64_t(nFree) * (k + 1) / ranges)));
             auto join = [&](Range const& r) {
                 int32_t const p0 = int32_t(pairs.inc.size()), n0 = int32_t(hNbr.size());
                 for (int32_t p : r.pairs.ptr)
@@ -1774,7 +1775,6 @@ class VbdSystem
         p.mu       = dMu.get();
         p.lambda   = dLambda.get();
         p.tets     = tets.get();
-        p.solve    = solve.get();
         p.incPtr   = incPtr.get();
         p.inc      = inc.get();
         p.nbrPtr   = nbrPtr.get();
@@ -3957,8 +3957,10 @@ PBGB_API int pbgb_vbd_launches_per_step(pbgb_vbd* h, int32_t iterations, int32_t
 {
     if (!h || !launches)
         return fail(h, kInvalid, "null argument");
-    *launches = h->sys.launchesPerStep(iterations, substeps);
-    return kOk;
+    return guarded(h, [&] {
+        *launches = h->sys.launchesPerStep(iterations, substeps);
+        return int(kOk);
+    });
 }
 
 PBGB_API int pbgb_vbd_step_graph_kernels(pbgb_vbd* h, int64_t* kernels)

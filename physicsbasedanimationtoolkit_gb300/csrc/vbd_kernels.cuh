@@ -143,7 +143,6 @@ struct StiffnessParams
     double const* __restrict__ mu;
     double const* __restrict__ lambda;
     TetRecord* __restrict__ tets; // mat written
-    int32_t const* __restrict__ solve;
     int32_t const* __restrict__ incPtr;
     uint32_t const* __restrict__ inc;
     int32_t const* __restrict__ nbrPtr;
