@@ -111,8 +111,16 @@ __device__ __forceinline__ bool barrier_wait(uint64_t* bar, uint32_t parity, int
 // When a wait gives up, the tile that did not arrive is never read and a barrier whose phase did not end is
 // not arrived on again; the warps run down the step's block and cluster barriers.  The positions are then
 // not valid, which the host reports.
+//
+// Registers: two blocks share an SM at 80 and often do not at 88, and clusters of 16 blocks find room in few
+// places: 9 meshes of 4^3 to 12^3 take 65 us a step at 80 and 94 at 87 (two rounds of clusters).  None of the
+// limits spills.  Streamed tiles and two-buffer sums lose more than that gains below 96 (a 5,040-vertex
+// Chebyshev step 124 us at 96, 127 at 88, 129 at 80), so those lanes that large parts take keep 96.
 template <int L, bool CHEB, bool REC, bool CLUSTER>
-__global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_kernel(ClusterStepParams p)
+constexpr int kClusterRegisters = REC ? 96 : (!CLUSTER || (!CHEB && (L == 1 || L >= 8)) ? 80 : (CHEB && (L == 1 || L == 32) ? 88 : 96));
+
+template <int L, bool CHEB, bool REC, bool CLUSTER>
+__global__ void __maxnreg__((kClusterRegisters<L, CHEB, REC, CLUSTER>)) cluster_step_kernel(ClusterStepParams p)
 {
     // Neighbours a lane has in flight at once: a block holds few warps, so a lane's own independent
     // loads hide the latency of shared memory.
@@ -439,9 +447,11 @@ __global__ void __launch_bounds__(32 * (kClusterMaxWarps + 1), 1) cluster_step_k
                     stage0 -= p.stages;
                     ++round0;
                 }
-                asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
-                if (CLUSTER && expects)
+                // One warp, the one with the least to solve, waits for the block: its acquire empties the SM's L1,
+                // and the block's barrier passes on what it makes visible.
+                if (CLUSTER && expects && warp == warps - 1)
                     barrier_wait<true>(halo + c, phase, gaveUp, flags, ns);
+                asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
             }
         }
 

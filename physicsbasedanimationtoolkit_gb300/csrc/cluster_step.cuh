@@ -22,11 +22,11 @@
 //
 // What a block reads from global memory inside a substep goes to L2 (the acquire of other blocks' positions
 // empties L1), so the positions damping needs are in shared memory too: a 5,040-vertex Chebyshev step of
-// 2 x 15 damped iterations takes 126 us with them, 137 us without.
+// 2 x 15 damped iterations took 126 us with them, 137 us without.
 //
-// Every wait has a time limit.  Asking for a tile as a warp costs a vote per group where tiles are streamed, 4
-// to 5 us of that step; steps whose tiles stay are as fast as without the limit (1331 vertices 58.5 us, 27
-// vertices 23.6, among others).
+// Every wait has a time limit.  Asking for a tile as a warp costs a vote per group where tiles are streamed (4
+// to 5 us of that step); with one warp waiting for the halo, and before the block's barrier, the steps take
+// 124 us (that one), 58.7 (1331 vertices) and 24.0 (27 vertices) among others.
 //
 // What bounds it: with a few solves per part and colour, the chain of one vertex solve (about 300
 // instructions of one warp, 0.8 us) times the colours; with many, shared memory (with three 16-byte reads per
