@@ -63,12 +63,30 @@ def make_data(pbat, w, rho=0.95):
     )
 
 
+_NEIGHBOURS = {}
+
+
+def neighbour_count(data):
+    """Sum over the free vertices of their distinct neighbours (vertices that share a tetrahedron).  Grids of
+    one size share it: kept by the counts of vertices, tets and free vertices."""
+    key = (data.X.shape[1], data.E.shape[1], data.Padj.size)
+    if key not in _NEIGHBOURS:
+        nV, T = data.X.shape[1], np.asarray(data.E).T
+        e = np.sort(np.concatenate([T[:, [a, b]] for a in range(4) for b in range(a + 1, 4)]), axis=1)
+        e = np.unique(e[:, 0] * nV + e[:, 1])
+        free = np.zeros(nV, bool)
+        free[data.Padj] = True
+        _NEIGHBOURS[key] = int(free[e // nV].sum() + free[e % nV].sum())
+    return _NEIGHBOURS[key]
+
+
 def algorithmic_bytes(data):
-    """Sum over free vertices of (60 + 120 deg(i)) bytes: one vertex-update's FP32/int32 inputs and
-    output (CSR pair 8, mass 4, xt 12, xtilde 12, x read 12 and written 12; per incident tet:
-    (e, ilocal) 8, 4 indices 16, GP 48, (mu, lambda) 8, wg 4, three other positions 36)."""
+    """Bytes a sweep over the free vertices asks of memory (L2 or DRAM) in the solver's layout, each input once
+    per vertex-update: per vertex 80 (solve entry, two list offsets and the block's constant 16; start position
+    with the mass, inertial target, own position read and written 64), per distinct neighbour 24 (index and K 8,
+    position 16), per pair of incidences 20 (two kappa, sigma 16, slots 4), at least deg / 2 of them."""
     deg = np.diff(data.GVGp)[data.Padj]
-    return int(60 * deg.size + 120 * int(deg.sum()))
+    return int(80 * deg.size + 24 * neighbour_count(data) + 20 * int(((deg + 1) // 2).sum()))
 
 
 class ClockSampler:
@@ -292,9 +310,8 @@ def batch_workload(args, pbat):
 
 
 def batch_algorithmic_bytes(datas, iterations):
-    """Algorithmic bytes of one batched step: per iteration the sum over every mesh's free vertices
-    of (60 + 120 deg(i)) bytes (the vertex-update formula of the sweep), plus per substep the
-    inertial target and initial guess (48 B read, 64 B written per vertex) and the velocity update
+    """Algorithmic bytes of one batched step: per iteration the vertex-update formula of the sweep over
+    every mesh's free vertices, plus per substep the inertial target and initial guess (48 B read, 64 B written per vertex) and the velocity update
     (48 B read, 32 B written per vertex)."""
     per_iter = sum(algorithmic_bytes(d) for d in datas)
     nV = sum(int(d.X.shape[1]) for d in datas)

@@ -278,7 +278,9 @@ PBGB_API int pbgb_vbd_sweep_timing(pbgb_vbd* h, double* milliseconds, int64_t* s
  * colour is done (per-mesh completion counters, bounded waits: a wait that gives up makes the next
  * synchronizing call return PBGB_ERR_TIMEOUT).  Used for plain VBD and Chebyshev without contact
  * when every colour's neighbours fit in shared memory; otherwise, or when disabled, a batch steps
- * with one launch per colour.  pbgb_vbd_persistent reports whether the next step uses it.
+ * with one launch per colour.  Waits of the cluster step are bounded in the same way.
+ * pbgb_vbd_persistent reports for a batch whether its next step is one launch (of either kind), and 0 for a
+ * single mesh, also where its step is one cluster launch: pbgb_vbd_launches_per_step tells that.
  * pbgb_vbd_set_batch_tile: sweep work items of subtiles x (block / lanes) vertices (default 1). */
 PBGB_API int pbgb_vbd_set_persistent(pbgb_vbd* h, int32_t enable);
 PBGB_API int pbgb_vbd_persistent(pbgb_vbd* h, int32_t* active);
@@ -510,7 +512,8 @@ PBGB_API int pbgb_debug_adjoint_tet(
     double* dlogmu,
     double* dloglambda);
 
-/* Test hook of the persistent batched step's bounded waits: the time limit of one wait (1 us ..
+/* Test hook of the persistent batched step's bounded waits (any item number, reached or not, keeps a batch out
+ * of the cluster step): the time limit of one wait (1 us ..
  * 2 s; default 2 s) and one work item whose requirement is never met (-1: none), for the steps that
  * follow.  With a poisoned item the step's wait gives up after wait_ns, the step ends with invalid
  * positions and the next synchronizing call returns PBGB_ERR_TIMEOUT; the context stays usable. */
@@ -525,8 +528,8 @@ PBGB_API int pbgb_debug_cluster_wait(pbgb_vbd* h, int64_t wait_ns, int32_t poiso
  * failure at most).  left (may be NULL): what was left of the last setting, -1 once it failed. */
 PBGB_API int pbgb_debug_fail_allocation(int64_t after, int64_t* left);
 
-/* Host self-check of the closed-form vertex block (FP64): accumulates n incident tets and
- * applies damping, inertia and the Newton step exactly like the device sweep.  Arguments as the
+/* Host self-check of the closed-form vertex block (FP64): accumulates n incident tets one by one (the device
+ * sweep adds the same terms two tets at a time) and applies damping, inertia and the Newton step like it.  Arguments as the
  * oracle's per-vertex solve: xe n x 12 (3x4 column-major per tet), GPs n x 12 (row-major 4x3). */
 PBGB_API int pbgb_debug_vertex_block(
     int32_t n,

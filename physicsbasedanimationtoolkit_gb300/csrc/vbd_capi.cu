@@ -701,7 +701,9 @@ class VbdSystem
     // The same for kernels launched per colour only (the reversed sweeps, the other accelerations,
     // contact, meshes past the cluster step).  One mesh, by the solves n of a colour: below 1,000 a
     // vertex's chain is what counts (32 lanes), then blocks that leave room for the next colour's while
-    // the GPU fills (8), at last work per vertex (4).  With blocks of 128 (the default for one mesh), us
+    // the GPU fills (8), at last work per vertex (4).  Where a step alone and steps in turn disagree (n = 8,400 and
+    // 18,260 below), those in turn decide: the other choice gains 6 to 11 % alone and loses 24 to 48 % there.
+    // A program with one integrator that wants the rest autotunes, which times a step alone.  With blocks of 128 (the default for one mesh), us
     // per 20-iteration step alone / in turn with two others: n = 578: 32 lanes 281, 8 lanes 285, 4 lanes
     // 327 (alone); n = 2,369: 32 lanes 450 / 179, 8 lanes 300 / 137, 4 lanes 329 / 137; n = 8,400: 8 lanes
     // 472 / 205, 4 lanes 421 / 255; n = 18,260: 8 lanes 641 / 456, 4 lanes 681 / 308; n = 33,600
