@@ -745,10 +745,12 @@ __global__ void simplex_shape_kernel(BvhView V, float4 const* __restrict__ P, in
     }
     if ((threadIdx.x & 31) == 0)
     {
-        // Non-negative floats order as their bits do.
-        atomicMax(shape, __float_as_int(h));
-        atomicMax(shape + 1, __float_as_int(face));
-        atomicMax(shape + 2, __float_as_int(slack));
+        // Non-negative floats order as their bits do.  Few warps hold more than what is there already.
+        int32_t const mine[3] = {__float_as_int(h), __float_as_int(face), __float_as_int(slack)};
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (mine[k] > *reinterpret_cast<int32_t const volatile*>(shape + k))
+                atomicMax(shape + k, mine[k]);
     }
 }
 

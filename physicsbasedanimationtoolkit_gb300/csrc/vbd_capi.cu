@@ -4,7 +4,7 @@
 // Reference counterpart: pbat::gpu::impl::vbd::Integrator (gpu/impl/vbd/Integrator.cu:22-347)
 // and the public pimpl pbat::gpu::vbd::Integrator (gpu/vbd/Integrator.cu).  Differences by design:
 // one stream per handle (the reference creates one and never uses it), the whole step replayed
-// from a CUDA graph, tets packed into 64-byte records, the in-place colour sweep (no xb copy-back
+// from a CUDA graph, tets packed into 32-byte records, the in-place colour sweep (no xb copy-back
 // pass), and several meshes concatenated into one system for the batched form.
 #include "adjoint.cuh"
 #include "batched.cuh"
